@@ -318,10 +318,10 @@ __global__ void __launch_bounds__(kMmaThreads + 96, 1)
     // ================= two MMA warps: even steps -> accumulator 0, odd steps -> accumulator 1
     const int which = warp == kMmaWarp ? 0 : 1;
     const uint32_t tmem_d = tmem + (which ? (uint32_t)Cfg::kAcc1 : 0u);
-    for (int s = which; s < nsteps; s += 2) {
-      const int st = s % kStages;
-      ok = tc_wait(ok, &full[st], (uint32_t)((s / kStages) & 1), p.status);
-      if (lane == 0) {
+    if (tc_elect()) {
+      for (int s = which; s < nsteps; s += 2) {
+        const int st = s % kStages;
+        ok = tc_wait(ok, &full[st], (uint32_t)((s / kStages) & 1), p.status);
         tc_after_sync();
         const uint32_t a_t = tmem + Cfg::kA0 + (uint32_t)st * (kStepGroups * kAGroupCols);
         const uint32_t bbase = smem_u32(bstg + (size_t)st * kStepGroups * kBBytes);
@@ -337,9 +337,9 @@ __global__ void __launch_bounds__(kMmaThreads + 96, 1)
           }
         tc_commit(&mma_done[st]);  // arrives once these (and all earlier) MMAs have retired
       }
-      __syncwarp();
+      tc_commit(done);
     }
-    if (lane == 0) tc_commit(done);
+    __syncwarp();
   } else {
     // ================= expander warps ========================================================
     // warp w owns TMEM lanes (= weight rows) 32*(w&3).., and K-half h = w>>2 of every group:

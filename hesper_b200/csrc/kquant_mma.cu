@@ -201,10 +201,10 @@ __global__ void __launch_bounds__(kQmThreads, 1) kq_mma_kernel(const __grid_cons
     // ================= MMA issue: even steps -> accumulator 0, odd steps -> accumulator 1 =====
     const int which = warp == kMmaWarpA ? 0 : 1;
     const uint32_t tmem_d = tmem + (uint32_t)(which * NT);
-    for (int s = which; s < nsteps && which < Cfg::kIssuers; s += Cfg::kIssuers) {
-      const int st = s % kQmStages;
-      ok = tc_wait(ok, &full[st], (uint32_t)((s / kQmStages) & 1), p.status);
-      if (lane == 0) {
+    if (tc_elect()) {
+      for (int s = which; s < nsteps && which < Cfg::kIssuers; s += Cfg::kIssuers) {
+        const int st = s % kQmStages;
+        ok = tc_wait(ok, &full[st], (uint32_t)((s / kQmStages) & 1), p.status);
         tc_after_sync();
         const uint32_t a_t = tmem + kQmA0 + (uint32_t)st * kQmACols;
         const uint32_t bbase = smem_u32(bstg + (size_t)st * kQmBBytes);
@@ -215,9 +215,9 @@ __global__ void __launch_bounds__(kQmThreads, 1) kq_mma_kernel(const __grid_cons
                         p.idesc, (s >= Cfg::kIssuers || j > 0) ? 1u : 0u);
         tc_commit(&mma_done[st]);
       }
-      __syncwarp();
+      tc_commit(done);
     }
-    if (lane == 0) tc_commit(done);
+    __syncwarp();
   } else {
     // ================= dequantise into tensor memory ==========================================
     const int q = warp & 3, h = warp >> 2;       // lane quarter, which 64-weight chunk of the step

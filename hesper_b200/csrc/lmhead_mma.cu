@@ -352,10 +352,10 @@ __global__ void __launch_bounds__(kLmThreads, 2)
     }
   } else if (warp == 1) {
     // ================= MMA issuer ===========================================================
-    for (int ks = 0; ks < nsteps; ++ks) {
-      const int st = ks % S;
-      ok = tc_wait(ok, &full[st], (uint32_t)((ks / S) & 1), p.status);
-      if (lane == 0) {
+    if (tc_elect()) {
+      for (int ks = 0; ks < nsteps; ++ks) {
+        const int st = ks % S;
+        ok = tc_wait(ok, &full[st], (uint32_t)((ks / S) & 1), p.status);
         tc_after_sync();
         const uint32_t abase = smem_u32(stg + (size_t)st * (kLmABytes + kLmBBytes));
         const uint32_t bbase = abase + kLmABytes;
@@ -366,9 +366,9 @@ __global__ void __launch_bounds__(kLmThreads, 2)
                       (ks > 0 || j > 0) ? 1u : 0u);
         tc_commit(&empty[st]);
       }
-      __syncwarp();
+      tc_commit(done);
     }
-    if (lane == 0) tc_commit(done);
+    __syncwarp();
   }
   // ================= epilogue (warps 2..5) ====================================================
   if (warp >= 2) {

@@ -23,6 +23,20 @@ __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t smem_addr, uint32_t lb
   return d;
 }
 
+// One lane of a converged warp, as a predicate ptxas can trace to elect.sync.  MMAs are issued from
+// under it and never from under `lane == 0`: behind a data-dependent branch every tcgen05.mma
+// costs its thread ~132 cycles whatever its shape (the descriptors are moved to uniform
+// registers behind a loop over the active lanes); behind this one M = 128, K = 32 bytes with A in
+// tensor memory issues every 42 / 74 / 138 cycles at N = 64 / 128 / 256, the tensor pipe's own
+// 32 / 64 / 128 plus ten.  Loops over pipeline steps sit inside the branch, not around it.
+__device__ __forceinline__ bool tc_elect() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
 // kind::f16 with the A operand in tensor memory (lane = row, two 16-bit K elements per
 // 32-bit column) and B through a shared-memory descriptor.
 __device__ __forceinline__ void tc_mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
