@@ -228,7 +228,7 @@ int hb_lmhead_mma_run(struct hb200_ctx* ctx, const void* d_table, int dtype, lon
 
 // Layout of the context's device scratch (one stream at a time uses it; regions of ops that
 // never overlap in time may overlap in space):
-constexpr size_t kScratchBytes = (size_t)24 << 20;
+constexpr size_t kScratchBytes = (size_t)56 << 20;
 constexpr size_t kScratchActs = 0;                     // batched ternary: d[64], sumq[64], int8 tiles
 constexpr size_t kScratchGlu = (size_t)2 << 20;       // batched gate/up products before the GLU
 constexpr size_t kScratchLmSplit = (size_t)8 << 20;   // 16-bit products: hi/lo activation tiles
@@ -252,13 +252,9 @@ struct HbKqSeg {
   float* y;
   const float* residual;
   long ldy;
-  int glu;
 };
-int hb_kq_mma_run_multi(struct hb200_ctx* ctx, const HbKqSeg* segs, int nseg, int K, int M,
-                        int NT, cudaStream_t st, int fmt = HB200_FMT_Q4_K);
-int hb_kq_mma_run(struct hb200_ctx* ctx, const uint8_t* d_blocks, int K, long N, int M, int NT,
-                  float* d_y, const float* d_residual, long ldy, int glu, cudaStream_t st,
-                  int fmt = HB200_FMT_Q4_K);
+int hb_kq_mma_run_multi(struct hb200_ctx* ctx, const HbKqSeg* segs, int nseg, int K, int M, int NT,
+                        int glu, cudaStream_t st, int fmt);
 
 struct hb200_ctx {
   int device;

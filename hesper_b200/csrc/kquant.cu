@@ -555,27 +555,24 @@ struct KQPre {
   float* out;
 };
 
-// One product of a batched call: y[M][N] = W x, plus a residual or, with glu set, times
-// gelu_tanh of the gate values in `residual`.
+// One product of a batched call: y[M][N] = W x (+ residual).
 struct KQBatchSeg {
   const uint8_t* blocks;
   long N;
   const float* residual;
   float* y;
-  int glu;
 };
 
-// Q4_K or Q8_0 (K a multiple of 256), any M >= 1, several tensors against the same activations:
-// the dequantiser is fused into the product kernel (kquant_mma.cu; split-K when there are few
-// row tiles).  The activations of a pass are normalised, rounded and laid out once and shared
-// by every tensor.
-static int kq_batched_fused(hb200_ctx* ctx, int fmt, const KQBatchSeg* segs, int nseg, int K,
+// Q4_K or Q8_0 (K a multiple of 256), any M >= 1, several tensors against the same activations
+// in one product launch per pass (kquant_mma.cu); glu: the tensors are gate and up, the result
+// gelu_tanh(gate) * up.  The activations of a pass are normalised, rounded and laid out once.
+static int kq_batched_fused(hb200_ctx* ctx, int fmt, const KQBatchSeg* segs, int nseg, int glu, int K,
                             const float* d_x, int M, const KQPre& pre, const float* gamma,
                             float eps, cudaStream_t st) {
-  ScratchUse use(ctx, st);  // staged activations, row scales, split-K partials, tickets
-  // tokens per pass: the tensor time of a pass does not depend on it, the activation tile
-  // and the accumulator do; K above 8192 keeps the 256-token tiles out of their scratch
-  const int cap = K <= 8192 ? 256 : 128;
+  ScratchUse use(ctx, st);  // staged activations, row scales, partials of cut tiles
+  // tokens per pass: the weights are dequantised once per pass, so as many as there are; 256
+  // while the staged activations fit their scratch
+  const int cap = (size_t)K * 512 <= kScratchRowScale - kScratchLmSplit ? 256 : 128;
   for (int m0 = 0; m0 < M;) {
     const int left = M - m0;
     const int NT = left <= 64 ? 64 : (left <= 128 || cap == 128 ? 128 : 256);
@@ -585,21 +582,14 @@ static int kq_batched_fused(hb200_ctx* ctx, int fmt, const KQBatchSeg* segs, int
                                  pre.gamma ? pre.out + (size_t)m0 * K : nullptr, gamma, eps, NT,
                                  st);
     if (rc != HB200_OK) return rc;
-    // tensors without a GLU epilogue go into one launch, three at a time (their row tiles
-    // add up, so small ones like k and v no longer leave most SMs idle); an up product
-    // whose epilogue reads the gate product's output needs that launch finished first
-    for (int s = 0; s < nseg;) {
-      HbKqSeg run[3];
-      int n = 0;
-      do {
-        const KQBatchSeg& g = segs[s];
-        run[n++] = {g.blocks, g.N, g.y + (size_t)m0 * g.N,
-                    g.residual ? g.residual + (size_t)m0 * g.N : nullptr, g.N, g.glu};
-        ++s;
-      } while (n < 3 && s < nseg && !segs[s].glu && !segs[s - 1].glu);
-      rc = hb_kq_mma_run_multi(ctx, run, n, K, mc, NT, st, fmt);
-      if (rc != HB200_OK) return rc;
+    HbKqSeg run[kKQMaxSeg];
+    for (int s = 0; s < nseg; ++s) {
+      const KQBatchSeg& g = segs[s];
+      run[s] = {g.blocks, g.N, g.y + (size_t)m0 * g.N,
+                g.residual ? g.residual + (size_t)m0 * g.N : nullptr, g.N};
     }
+    rc = hb_kq_mma_run_multi(ctx, run, nseg, K, mc, NT, glu, st, fmt);
+    if (rc != HB200_OK) return rc;
     m0 += mc;
   }
   return HB200_OK;
@@ -735,8 +725,8 @@ static int kq_forward_multi_impl(hb200_ctx* ctx, int fmt, const hb200_kquant_seg
     KQBatchSeg g[kKQMaxSeg];
     for (int s = 0; s < nseg; ++s)
       g[s] = {static_cast<const uint8_t*>(segs[s].d_blocks), segs[s].N, segs[s].d_residual,
-              segs[s].d_y, 0};
-    return kq_batched_fused(ctx, fmt, g, nseg, K, d_x, M, pre, d_rms_gamma, rms_eps, st);
+              segs[s].d_y};
+    return kq_batched_fused(ctx, fmt, g, nseg, 0, K, d_x, M, pre, d_rms_gamma, rms_eps, st);
   }
   HB_REQUIRE(M <= 64, "kquant: M=%d needs the batched path (HB200_NO_MMA is set)", M);
   if (M == 1) {  // one token: integer tensor-core matvec when the rows fit shared memory
@@ -816,12 +806,10 @@ static int kq_gateup_impl(hb200_ctx* ctx, int fmt, const void* d_blocks_gate,
              "kquant gate/up: blocks must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (M >= kKQBatchedFrom && !ctx->no_mma) {
-    // both products on the tensor cores against one staging of the activations: the gate
-    // product writes d_y, the up product's epilogue multiplies gelu_tanh(gate) in place
-    const KQBatchSeg g[2] = {
-        {static_cast<const uint8_t*>(d_blocks_gate), N, nullptr, d_y, 0},
-        {static_cast<const uint8_t*>(d_blocks_up), N, d_y, d_y, 1}};
-    return kq_batched_fused(ctx, fmt, g, 2, K, d_x, M, pre, d_rms_gamma, rms_eps, st);
+    // both products on the tensor cores in one launch, GeGLU in its epilogue
+    const KQBatchSeg g[2] = {{static_cast<const uint8_t*>(d_blocks_gate), N, nullptr, d_y},
+                             {static_cast<const uint8_t*>(d_blocks_up), N, nullptr, d_y}};
+    return kq_batched_fused(ctx, fmt, g, 2, 1, K, d_x, M, pre, d_rms_gamma, rms_eps, st);
   }
   HB_REQUIRE(M <= 64, "kquant gate/up: M=%d needs the batched path", M);
   if (M == 1) {
