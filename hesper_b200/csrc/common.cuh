@@ -236,16 +236,7 @@ constexpr size_t kScratchRowScale = ((size_t)16 << 20) - 4096;  // f16 products:
                                                        // scale per staged activation row
 constexpr size_t kScratchSplitK = (size_t)16 << 20;   // batched paths: split-K partials
 
-// the two halves of it, also used by the batched k-quant path (weights dequantised to f16)
-int hb_gemm16_split(struct hb200_ctx* ctx, int dtype, int K, const float* d_x, int M,
-                    const float* d_rms_gamma, float rms_eps, int single, cudaStream_t st);
-int hb_gemm16_split_pre(struct hb200_ctx* ctx, int dtype, int K, const float* d_x, int M,
-                        const float* d_pre_base, const float* d_pre_gamma, float* d_pre_out,
-                        const float* d_rms_gamma, float rms_eps, int single, cudaStream_t st);
-int hb_gemm16_mma(struct hb200_ctx* ctx, const void* d_table, int dtype, long V, int K, int M,
-                  float* d_y, const float* d_residual, long ldy, unsigned long long* d_keys,
-                  int table_constant, cudaStream_t st);
-// batched Q4_K with the dequantiser fused into the tensor-core kernel, kquant_mma.cu
+// batched k-quants with the dequantiser fused into the tensor-core kernel, kquant_mma.cu
 struct HbKqSeg {
   const uint8_t* blocks;
   long N;
@@ -255,6 +246,10 @@ struct HbKqSeg {
 };
 int hb_kq_mma_run_multi(struct hb200_ctx* ctx, const HbKqSeg* segs, int nseg, int K, int M, int NT,
                         int glu, cudaStream_t st, int fmt);
+int hb_kq_mma_max_tokens(int fmt, int K);
+int hb_kq_stage(struct hb200_ctx* ctx, int fmt, int K, int NT, const float* d_x, int M,
+                const float* d_pre_base, const float* d_pre_gamma, float* d_pre_out,
+                const float* d_rms_gamma, float rms_eps, cudaStream_t st);
 
 struct hb200_ctx {
   int device;

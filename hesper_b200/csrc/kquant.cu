@@ -570,17 +570,16 @@ static int kq_batched_fused(hb200_ctx* ctx, int fmt, const KQBatchSeg* segs, int
                             const float* d_x, int M, const KQPre& pre, const float* gamma,
                             float eps, cudaStream_t st) {
   ScratchUse use(ctx, st);  // staged activations, row scales, partials of cut tiles
-  // tokens per pass: the weights are dequantised once per pass, so as many as there are; 256
-  // while the staged activations fit their scratch
-  const int cap = (size_t)K * 512 <= kScratchRowScale - kScratchLmSplit ? 256 : 128;
+  // tokens per pass: the weights are dequantised once per pass, so as many as there are and as the
+  // staging scratch takes
+  const int cap = hb_kq_mma_max_tokens(fmt, K);
   for (int m0 = 0; m0 < M;) {
     const int left = M - m0;
-    const int NT = left <= 64 ? 64 : (left <= 128 || cap == 128 ? 128 : 256);
+    const int NT = left <= 64 || cap == 64 ? 64 : (left <= 128 || cap == 128 ? 128 : 256);
     const int mc = left < NT ? left : NT;
-    int rc = hb_gemm16_split_pre(ctx, 1, K, d_x + (size_t)m0 * K, mc,
-                                 pre.gamma ? pre.base + (size_t)m0 * K : nullptr, pre.gamma,
-                                 pre.gamma ? pre.out + (size_t)m0 * K : nullptr, gamma, eps, NT,
-                                 st);
+    int rc = hb_kq_stage(ctx, fmt, K, NT, d_x + (size_t)m0 * K, mc,
+                         pre.gamma ? pre.base + (size_t)m0 * K : nullptr, pre.gamma,
+                         pre.gamma ? pre.out + (size_t)m0 * K : nullptr, gamma, eps, st);
     if (rc != HB200_OK) return rc;
     HbKqSeg run[kKQMaxSeg];
     for (int s = 0; s < nseg; ++s) {

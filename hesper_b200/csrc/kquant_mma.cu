@@ -8,24 +8,26 @@
 // Hesper/Layers/Linear.lean:1152-1760,5973-6177).  Weights AND activations are rounded to f16
 // (2^-11 each): measured error ~4e-4 of max|y|, bar 1e-3.
 //
-// What bounds it: at 64 tokens the dequantiser (about 3 instructions per weight) and HBM, at
+// What bounds it: at 64 tokens the dequantiser (about 2 instructions per weight) and HBM, at
 // 256 tokens the tensor pipe (M=128, N=256, K=16 in 138 cycles).  Either way only when every SM
 // works, so the work is dealt in units of (row tile of 128, super-block of 256 weights):
 //   * whole waves of row tiles go one tile to a CTA (W per CTA, results stored directly);
 //   * the R row tiles left over are cut along K into runs of `upc` consecutive units, one run
 //     per CTA.  A run that does not cover its tile leaves an f32 partial in the context's
-//     scratch and a small second kernel adds a tile's partials in K order (deterministic).
+//     scratch and a small second kernel adds a tile's partials in K order (deterministic; adding
+//     them in this kernel by the last part to arrive was slower: the fence in front of the
+//     ticket waits for the CTA's stores, 43 against 28 us at K=10240 N=2560, 256 tokens).
 //     160 tiles of a 10240-row gate/up pair so take 11 super-block times on 148 SMs instead of
 //     20, the 20 tiles of a 2560-row down projection 6 instead of 40.
-// 19 warps with fixed roles:
-//   warps 0-15 dequantise: warps 0-7 the even, 8-15 the odd steps of 128 weights; a thread owns
-//              one row and 64 weights of a step and stores them with one tcgen05.st.  They also
-//              run the epilogue of a finished tile, after they have refilled the A stages for
-//              the next one;
-//   warp 16    weights: 2-D tensor-map TMA boxes of 64 rows x 256 weights, a ring of 2 to 7 tiles;
-//   warp 17    activations: bulk copies of the step's tiles (f16, operand layout written by the
+// Warps with fixed roles:
+//   16 or 24   dequantise, in groups of 8 that take the steps of 128 weights in turn; a thread owns
+//              one row and 64 weights of a step and stores them with tcgen05.st.  The first 16
+//              also run the epilogue of a finished tile, after they have refilled the A stages
+//              for the next one;
+//   one        weights: 2-D tensor-map TMA boxes of 64 rows x 256 weights, a ring of 2 to 7 tiles;
+//   one        activations: bulk copies of the step's tiles (f16, operand layout written by the
 //              staging kernel);
-//   warp 18    one elected thread issues the MMAs (M=128, N=NT tokens, K=16).
+//   one        an elected thread issues the MMAs (M=128, N=NT tokens, K=16).
 // A gate/up pair is one launch: a tile holds 64 gate rows and the 64 up rows of the same outputs,
 // dealt to the tensor-memory lanes so that a gate lane's up value sits 16 lanes further in the
 // same warp (one shuffle per two tokens in the epilogue).
@@ -39,8 +41,6 @@ namespace hb {
 constexpr int kQmRows = 128;          // weight rows per tile = MMA M
 constexpr int kQmStepK = 128;         // weights per pipeline step (half a super-block)
 constexpr int kQmACols = kQmStepK / 2;  // 64 TMEM columns of f16 pairs per stage
-constexpr int kQmExpWarps = 16;
-constexpr int kQmThreads = (kQmExpWarps + 3) * 32;
 constexpr int kQmMaxSeg = 4;          // tensors one launch multiplies by the same activations
 
 // NT tokens per pass = MMA N; a unit is the bytes of 256 weights (one Q4_K super-block, eight
@@ -49,16 +49,33 @@ template <int NT, int FMT>
 struct QmCfg {
   static constexpr int kUnit = FMT == 12 ? 144 : 272;
   static constexpr int kPkBytes = kQmRows * kUnit;          // 18 / 34 KB
+  // kind::f16: D = f32, A and B f16, both K-major, N = NT, M = 128
+  static constexpr uint32_t kIdesc =
+      (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kQmRows >> 4) << 24);
+  static constexpr bool kSums = FMT == 12;                  // sub-block sums as extra K columns
   static constexpr int kAccBufs = NT <= 128 ? 2 : 1;        // accumulators in tensor memory
   static constexpr int kA0 = kAccBufs * NT;                 // first TMEM column of the A stages
-  static constexpr int kAStages = NT == 64 ? 6 : 4;
-  // activation stages: a whole step, or half of one at 256 tokens (64 KB per step)
+  static constexpr int kAStages = NT == 64 ? 5 : 3;
+  static constexpr int kE0 = kA0 + kAStages * kQmACols;     // TMEM columns of the min residues:
+  static constexpr int kESlots = kSums ? 8 : 0;             //   8 per super-block
+  // staged bytes of a super-block: four blocks of [NT rows][64 f16], then [NT rows][16 f16]
+  static constexpr int kSumBytes = kSums ? NT * 32 : 0;
+  static constexpr int kSbBytes = NT * 512 + kSumBytes;
+  // activation stages: a whole step, or half of one at 256 tokens (64 KB per step); the last of a
+  // super-block brings the sums along
   static constexpr int kBPer = NT == 256 ? 2 : 1;
-  static constexpr int kBBytes = NT * kQmStepK * 2 / kBPer;  // 16 / 32 / 32 KB
-  static constexpr int kBStages = NT == 64 ? 6 : 4;
-  static constexpr int kPkStages = FMT == 12 ? (NT == 64 ? 7 : 5) : (NT == 64 ? 3 : 2);
-  static constexpr int kSmem = 1024 + kPkStages * kPkBytes + kBStages * kBBytes;
-  static_assert(kA0 + kAStages * kQmACols <= 512, "tensor memory columns");
+  static constexpr int kBStep = NT * kQmStepK * 2 / kBPer;  // 16 / 32 / 32 KB
+  static constexpr int kBBytes = kBStep + kSumBytes;
+  static constexpr int kBStages = NT == 64 ? 5 : (NT == 128 ? 3 : 4);
+  static constexpr int kPkStages = FMT == 12 ? (NT == 64 ? 7 : (NT == 128 ? 6 : 3)) : (NT == 256 ? 2 : 3);
+  // dequantising warps, in groups of 8 that take the steps in turn: a step is a chain of ~1000
+  // cycles (barrier, shared memory, conversion, store) of which a warp issues 150, so below
+  // 256 tokens, where the dequantiser is the bound, six warps per scheduler beat four
+  static constexpr int kGroups = NT == 256 ? 2 : 3;
+  static constexpr int kExpWarps = 8 * kGroups;
+  static constexpr int kThreads = (kExpWarps + 3) * 32;
+  static constexpr int kSmem = 2048 + kPkStages * kPkBytes + kBStages * kBBytes;
+  static_assert(kE0 + kESlots * 8 <= 512, "tensor memory columns");
   static_assert(kSmem <= 232448, "shared memory budget of one CTA");
 };
 
@@ -84,74 +101,56 @@ struct QmParams {
   int nseg;
   int glu;                // seg 0 = gate, seg 1 = up; y = gelu_tanh(gate) * up into seg 0's y
   QmDeal deal;
-  const uint8_t* xb;      // f16 activations: [K/64][NT rows x 64 f16, operand layout]
+  const uint8_t* xb;      // staged activations: kSbBytes per super-block
   const float* rowscale;  // [NT] power of two each token's row was divided by before rounding
   int M;
-  float* part;            // [cta][2][NT tokens][128 lanes] partial sums of left-over tiles
-  uint32_t idesc;
+  float* part;            // [cta][2][NT / 4][128 lanes][4 tokens] partial sums of left-over tiles
   uint32_t* status;
 };
 
-// 0.5*g*(1+tanh(sqrt(2/pi)*(g+0.044715 g^3))), the gate factor of the GeGLU
-// (Hesper/Layers/FusedFFNSpec.lean:42-45), same expression as the standalone kernel
+// 0.5*g*(1+tanh(t)), t = sqrt(2/pi)*(g+0.044715 g^3), the gate factor of the GeGLU
+// (Hesper/Layers/FusedFFNSpec.lean:42-45), as g * sigmoid(2t): the same function without the
+// cancellation of 1 + tanh at negative t, and a third of tanhf's instructions (the epilogue of a
+// 256-token tile evaluates 16384 of them).  t -> -inf: exp overflows to inf, the result is -0.
 __device__ __forceinline__ float glu_gate(float g) {
-  const float t = 0.7978845608028654f * (g + 0.044715f * g * g * g);
-  return 0.5f * g * (1.0f + tanhf(t));
+  const float t2 = 1.5957691216057308f * (g + 0.044715f * g * g * g);
+  return __fdividef(g, 1.0f + __expf(-t2));
 }
 
-__device__ __forceinline__ uint32_t pack_f16(float a, float b) {
-  const __half2 h = __floats2half2_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-__device__ __forceinline__ float2 h2f(uint32_t h) {
-  return __half22float2(*reinterpret_cast<const __half2*>(&h));
-}
-// {a.x*s + c, a.y*s + c} in one packed instruction
-__device__ __forceinline__ float2 fma2(float2 a, float2 s, float2 c) {
-  float2 r;
-  asm("{\n\t.reg .b64 a, s, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 s, {%4, %5};\n\t"
-      "mov.b64 c, {%6, %7};\n\tfma.rn.f32x2 d, a, s, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(s.x), "f"(s.y), "f"(c.x), "f"(c.y));
-  return r;
-}
+__device__ __forceinline__ __half2 as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
+__device__ __forceinline__ uint32_t as_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 
-// 32 nibble bytes of a chunk (two sub-blocks of 32 weights: low and high nibbles) -> 64 f16 as
-// fma(ds, q, -dm) in f32, rounded once.  A nibble is moved to bits 4-7 of a 16-bit lane and
-// completed to the f16 1024 + 16 q with one LOP3 for two of them; widened exactly, the f32 fma
-// takes scale ds / 16 and addend -dm - 64 ds.  o[0..15]: low, o[16..31]: high nibbles.
-__device__ __forceinline__ void q4k_expand(const uint32_t (&q)[8], float ds0, float dm0, float ds1,
-                                           float dm1, uint32_t (&o)[32]) {
-  const float2 s0 = make_float2(ds0 * 0.0625f, ds0 * 0.0625f);
-  const float2 s1 = make_float2(ds1 * 0.0625f, ds1 * 0.0625f);
-  const float a0 = fmaf(-64.f, ds0, -dm0), a1 = fmaf(-64.f, ds1, -dm1);
-  const float2 c0 = make_float2(a0, a0), c1 = make_float2(a1, a1);
+// 32 nibble bytes of a chunk (two sub-blocks of 32 weights: low and high nibbles) -> 64 f16.
+// Everything stays in packed f16 and only one step rounds: LOP3 completes two nibbles to the
+// f16 1024 + q (low) or 1024 + 16 q (high), one HFMA2 turns them into the integers sc * q (at
+// most 945: exact), one HFMA2 forms d * (sc q) - c with c = dmin * m rounded to f16.  What c lost,
+// e = dmin * m - c, is not dropped: it goes into the product as sixteen further K columns per
+// super-block (e of its 8 sub-blocks against the sub-blocks' activation sums), so the weights
+// carry the one rounding of the f32 formula and nothing else.  Two instructions per two weights
+// and step instead of five through f32 (I2F / FFMA / pack).
+// The pairs come out as bytes {0, 2}, {1, 3} of every word; the activations are staged in the
+// same order.  HI: the high nibbles.
+template <bool HI>
+__device__ __forceinline__ void q4k_expand(const uint32_t (&q)[8], __half2 d, __half2 mul, __half2 add,
+                                           __half2 c, uint32_t (&o)[16]) {
+  constexpr uint32_t kMask = HI ? 0x00F000F0u : 0x000F000Fu;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const uint32_t w = q[i];
-    const float2 lA = h2f(((w << 4) & 0x00F000F0u) | 0x64006400u);  // bytes 0, 2
-    const float2 lB = h2f(((w >> 4) & 0x00F000F0u) | 0x64006400u);  // bytes 1, 3
-    const float2 hA = h2f((w & 0x00F000F0u) | 0x64006400u);
-    const float2 hB = h2f(((w >> 8) & 0x00F000F0u) | 0x64006400u);
-    const float2 l01 = fma2(make_float2(lA.x, lB.x), s0, c0), l23 = fma2(make_float2(lA.y, lB.y), s0, c0);
-    const float2 h01 = fma2(make_float2(hA.x, hB.x), s1, c1), h23 = fma2(make_float2(hA.y, hB.y), s1, c1);
-    o[2 * i] = pack_f16(l01.x, l01.y);
-    o[2 * i + 1] = pack_f16(l23.x, l23.y);
-    o[16 + 2 * i] = pack_f16(h01.x, h01.y);
-    o[16 + 2 * i + 1] = pack_f16(h23.x, h23.y);
+    const uint32_t t0 = (q[i] & kMask) | 0x64006400u, t1 = ((q[i] >> 8) & kMask) | 0x64006400u;
+    o[2 * i] = as_u32(__hfma2(d, __hfma2(as_h2(t0), mul, add), c));
+    o[2 * i + 1] = as_u32(__hfma2(d, __hfma2(as_h2(t1), mul, add), c));
   }
 }
 
 // Four int8 times d, rounded once to f16: bytes biased to 1024 + (q + 128), the bias taken off
 // exactly, then an f16 product (d is an f16, q an integer: the exact product is rounded once).
+// Pairs {0, 2}, {1, 3} as in q4k_expand.
 __device__ __forceinline__ void q80_word(uint32_t w, __half2 d, uint32_t& lo, uint32_t& hi) {
   const uint32_t x = w ^ 0x80808080u;
-  const uint32_t a = __byte_perm(x, 0x64646464u, 0x4140), b = __byte_perm(x, 0x64646464u, 0x4342);
+  const uint32_t a = __byte_perm(x, 0x64646464u, 0x4240), b = __byte_perm(x, 0x64646464u, 0x4341);
   const __half2 bias = __floats2half2_rn(1152.f, 1152.f);
-  const __half2 r0 = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&a), bias), d);
-  const __half2 r1 = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&b), bias), d);
-  lo = *reinterpret_cast<const uint32_t*>(&r0);
-  hi = *reinterpret_cast<const uint32_t*>(&r1);
+  lo = as_u32(__hmul2(__hsub2(as_h2(a), bias), d));
+  hi = as_u32(__hmul2(__hsub2(as_h2(b), bias), d));
 }
 
 // One stretch of work of a CTA: units [b0, b0 + n) of a tile.
@@ -172,15 +171,156 @@ __device__ __forceinline__ QmJob qm_job(const QmDeal& d, int j) {
   return {d.W * (int)gridDim.x + t, lo - t * d.nb, hi - lo, hi - lo == d.nb ? -1 : k};
 }
 
+// ---- staging of the activations -----------------------------------------------------------
+//
+// One CTA per token row: optional x' = base + rmsnorm(x) * pre_gamma (x' also written out), optional
+// RMSNorm * gamma, the row divided by a power of two that brings its largest magnitude into
+// [2^13, 2^14) (f16 has 5 exponent bits: an activation above 65504 would round to infinity, one
+// below 6e-5 lose bits; the product's epilogue multiplies the scale back), rounded to f16 and laid
+// out as the MMA's B operand: per super-block four blocks [row / 8][k / 8][row % 8][8 k] of 64
+// elements and, for Q4_K, [row / 8][2][row % 8][8] with the sums of the 8 sub-blocks / 32 (the
+// second half zero).  The four bytes of a weight word pair up as {0, 2}, {1, 3}: so do the k here.
+// Latency is all there is to it (a row, three block-wide reductions at most), so the row stays
+// in registers from its one read and the norm weights are fetched before the wait.
+struct QmStage {
+  const float *x, *gamma, *pre_base, *pre_gamma;
+  float* pre_out;
+  float eps;
+  int K;
+  uint8_t* xb;
+  size_t sb_bytes;   // bytes of a super-block
+  int sums_off;      // where its sums start, 0: none
+  float* rowscale;
+};
+
+template <int G>
+__global__ void __launch_bounds__(1024) kq_stage_kernel(const __grid_constant__ QmStage p) {
+  __shared__ double red[2][32];
+  __shared__ float redf[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int m = blockIdx.x, n8 = p.K >> 3;
+  float g[G][8], pg[G][8], v[G][8];
+  auto load8 = [&](float (&d)[8], const float* src, int i, bool ro) {
+    if (ro && (reinterpret_cast<uintptr_t>(src) & 15)) {  // norm weights may sit anywhere
+#pragma unroll
+      for (int e = 0; e < 8; ++e) d[e] = __ldg(src + 8 * i + e);
+      return;
+    }
+    const float4* s4 = reinterpret_cast<const float4*>(src) + 2 * i;
+    const float4 a = ro ? __ldg(s4) : __ldcg(s4), b = ro ? __ldg(s4 + 1) : __ldcg(s4 + 1);
+    d[0] = a.x; d[1] = a.y; d[2] = a.z; d[3] = a.w;
+    d[4] = b.x; d[5] = b.y; d[6] = b.z; d[7] = b.w;
+  };
+  pdl_trigger();
+#pragma unroll
+  for (int j = 0; j < G; ++j) {
+    const int i = tid + j * blockDim.x;
+    if (i < n8 && p.gamma) load8(g[j], p.gamma, i, true);
+    if (i < n8 && p.pre_gamma) load8(pg[j], p.pre_gamma, i, true);
+  }
+  pdl_wait();
+#pragma unroll
+  for (int j = 0; j < G; ++j) {
+    const int i = tid + j * blockDim.x;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[j][e] = 0.f;
+    if (i < n8) load8(v[j], p.x + (size_t)m * p.K, i, false);
+  }
+  auto row_rinv = [&](double* scr) {  // 1 / rms of the row held in v (block-wide)
+    double ss = 0.0;
+#pragma unroll
+    for (int j = 0; j < G; ++j)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss += (double)v[j][e] * v[j][e];
+    ss = warp_sum(ss);
+    if (lane == 0) scr[warp] = ss;
+    __syncthreads();
+    ss = warp_sum(lane < nwarps ? scr[lane] : 0.0);
+    return (float)(1.0 / sqrt(ss / (double)p.K + (double)p.eps));
+  };
+  if (p.pre_gamma) {
+    float b[G][8];
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      const int i = tid + j * blockDim.x;
+      if (i < n8) load8(b[j], p.pre_base + (size_t)m * p.K, i, false);
+    }
+    const float r1 = row_rinv(red[0]);
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      const int i = tid + j * blockDim.x;
+      if (i < n8) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          v[j][e] = __fadd_rn(b[j][e], __fmul_rn(__fmul_rn(v[j][e], r1), pg[j][e]));
+        float4* og = reinterpret_cast<float4*>(p.pre_out + (size_t)m * p.K) + 2 * i;
+        og[0] = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
+        og[1] = make_float4(v[j][4], v[j][5], v[j][6], v[j][7]);
+      }
+    }
+  }
+  if (p.gamma) {
+    const float rinv = row_rinv(red[1]);
+#pragma unroll
+    for (int j = 0; j < G; ++j)
+      if (tid + j * (int)blockDim.x < n8) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[j][e] = __fmul_rn(__fmul_rn(v[j][e], rinv), g[j][e]);
+      }
+  }
+  float amax = 0.f;
+#pragma unroll
+  for (int j = 0; j < G; ++j)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[j][e]));  // groups past K hold zeros
+  amax = warp_max(amax);
+  if (lane == 0) redf[warp] = amax;
+  __syncthreads();
+  amax = warp_max(lane < nwarps ? redf[lane] : 0.f);
+  int ex = 13;  // an all-zero (or non-finite) row keeps scale 1
+  if (amax > 0.f && amax <= 3.0e38f) ex = min(max(ilogbf(amax), -100), 120);
+  if (tid == 0) p.rowscale[m] = ldexpf(1.f, ex - 13);
+  const float inv_s = ldexpf(1.f, 13 - ex);
+#pragma unroll
+  for (int j = 0; j < G; ++j) {
+    const int i = tid + j * blockDim.x;
+    float sum = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      v[j][e] *= inv_s;  // exact: a power of two
+      sum += v[j][e];
+    }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (i >= n8) continue;
+    uint8_t* sb = p.xb + (size_t)(i >> 5) * p.sb_bytes;
+    uint4 o;
+    o.x = as_u32(__floats2half2_rn(v[j][0], v[j][2]));
+    o.y = as_u32(__floats2half2_rn(v[j][1], v[j][3]));
+    o.z = as_u32(__floats2half2_rn(v[j][4], v[j][6]));
+    o.w = as_u32(__floats2half2_rn(v[j][5], v[j][7]));
+    // four blocks of NT rows x 128 bytes: sums_off (or sb_bytes) is their total
+    const size_t blk = (p.sums_off ? (size_t)p.sums_off : p.sb_bytes) >> 2;
+    *reinterpret_cast<uint4*>(sb + ((i & 31) >> 3) * blk + (m >> 3) * 1024 + (i & 7) * 128 + (m & 7) * 16) = o;
+    if (p.sums_off) {
+      uint8_t* sd = sb + p.sums_off + (m >> 3) * 256 + (m & 7) * 16;
+      if ((i & 3) == 0)
+        *reinterpret_cast<__half*>(sd + ((i & 31) >> 2) * 2) = __float2half_rn(sum * 0.03125f);
+      if ((i & 31) == 1) *reinterpret_cast<uint4*>(sd + 128) = make_uint4(0, 0, 0, 0);
+    }
+  }
+}
+
 template <int NT, int FMT>
-__global__ void __launch_bounds__(kQmThreads, 1) kq_mma_kernel(const __grid_constant__ QmParams p) {
+__global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(const __grid_constant__ QmParams p) {
   using Cfg = QmCfg<NT, FMT>;
   constexpr int kPkStages = Cfg::kPkStages, kPkBytes = Cfg::kPkBytes, kUnit = Cfg::kUnit;
   constexpr int kAStages = Cfg::kAStages, kBStages = Cfg::kBStages, kBBytes = Cfg::kBBytes;
-  constexpr int kBPer = Cfg::kBPer, kA0 = Cfg::kA0, kAccBufs = Cfg::kAccBufs;
+  constexpr int kBPer = Cfg::kBPer, kA0 = Cfg::kA0, kAccBufs = Cfg::kAccBufs, kGroups = Cfg::kGroups;
   // a box dimension holds at most 256 elements: the 272-byte Q8_0 unit is mapped as 68 words
   constexpr int kBoxX = FMT == 12 ? 144 : 68;
-  constexpr int kPkWarp = kQmExpWarps, kActWarp = kQmExpWarps + 1, kMmaWarp = kQmExpWarps + 2;
+  constexpr int kEpiWarps = 16;
+  constexpr int kPkWarp = Cfg::kExpWarps, kActWarp = kPkWarp + 1, kMmaWarp = kPkWarp + 2;
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -194,16 +334,17 @@ __global__ void __launch_bounds__(kQmThreads, 1) kq_mma_kernel(const __grid_cons
   uint64_t* acc_full = b_free + kBStages;    // [kAccBufs] a tile's products are complete
   uint64_t* acc_free = acc_full + kAccBufs;  // [kAccBufs] the epilogue has read them
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + kAccBufs);
-  uint8_t* pk = smem + 1024;
+  float* rs_s = reinterpret_cast<float*>(smem + 1024);  // [NT] row scales
+  uint8_t* pk = smem + 2048;
   uint8_t* bstg = pk + kPkStages * kPkBytes;
 
   if (tid == 0) {
     for (int i = 0; i < kPkStages; ++i) {
       mbar_init(&pk_full[i], 1);
-      mbar_init(&pk_free[i], kQmExpWarps);
+      mbar_init(&pk_free[i], 16);  // two steps of 8 warps
     }
     for (int i = 0; i < kAStages; ++i) {
-      mbar_init(&a_full[i], kQmExpWarps / 2);
+      mbar_init(&a_full[i], 8);
       mbar_init(&a_free[i], 1);
     }
     for (int i = 0; i < kBStages; ++i) {
@@ -212,7 +353,7 @@ __global__ void __launch_bounds__(kQmThreads, 1) kq_mma_kernel(const __grid_cons
     }
     for (int i = 0; i < kAccBufs; ++i) {
       mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_free[i], kQmExpWarps);
+      mbar_init(&acc_free[i], kEpiWarps);
     }
     fence_mbar_init();
   }
@@ -224,101 +365,114 @@ __global__ void __launch_bounds__(kQmThreads, 1) kq_mma_kernel(const __grid_cons
   tc_before_sync();
   __syncthreads();
   tc_after_sync();
-  const uint32_t tmem = *tmem_slot;
+  // All 512 columns are this CTA's, so the allocation starts at column 0: a constant base keeps
+  // the MMA warp's addresses in the uniform datapath.
+  constexpr uint32_t tmem = 0;
   const int njobs = qm_jobs(p.deal);
   bool ok = true;
   pdl_trigger();
 
   if (warp == kPkWarp) {
     // ================= weights: constant, so no wait on the previous kernel =====================
-    if (tc_elect()) {
-      const uint64_t pol = policy_evict_first();
-      int n = 0;  // units brought so far
-      for (int j = 0; j < njobs && ok; ++j) {
-        const QmJob job = qm_job(p.deal, j);
-        int si = 0;
-        if (!p.glu) {
+    const uint64_t pol = policy_evict_first();
+    TcRing<kPkStages> r;
+    for (int j = 0; j < njobs && ok; ++j) {
+      const QmJob job = qm_job(p.deal, j);
+      int si = 0;
+      if (!p.glu) {
 #pragma unroll
-          for (int i = 1; i < kQmMaxSeg; ++i)
-            if (i < p.nseg && job.tile >= p.seg[i].tile0) si = i;
+        for (int i = 1; i < kQmMaxSeg; ++i)
+          if (i < p.nseg && job.tile >= p.seg[i].tile0) si = i;
+      }
+      const CUtensorMap* tm0 = &p.tmap[si];
+      const CUtensorMap* tm1 = p.glu ? &p.tmap[1] : tm0;
+      const int y0 = p.glu ? job.tile * 64 : (job.tile - p.seg[si].tile0) * kQmRows;
+      const int y1 = p.glu ? y0 : y0 + 64;
+      int x = job.b0 * kBoxX;
+      for (int b = 0; b < job.n; ++b, x += kBoxX, r.advance()) {
+        ok = tc_wait_w(&pk_free[r.i], r.phase ^ 1, p.status);
+        if (!ok) break;
+        if (tc_elect()) {
+          mbar_arrive_expect_tx(&pk_full[r.i], kPkBytes);
+          uint8_t* dst = pk + (size_t)r.i * kPkBytes;
+          tc_tma_box_2d(dst, tm0, x, y0, &pk_full[r.i], pol);
+          tc_tma_box_2d(dst + kPkBytes / 2, tm1, x, y1, &pk_full[r.i], pol);
         }
-        const CUtensorMap* tm0 = &p.tmap[si];
-        const CUtensorMap* tm1 = p.glu ? &p.tmap[1] : tm0;
-        const int y0 = p.glu ? job.tile * 64 : (job.tile - p.seg[si].tile0) * kQmRows;
-        const int y1 = p.glu ? y0 : y0 + 64;
-        for (int b = 0; b < job.n; ++b, ++n) {
-          const int st = n % kPkStages;
-          if (n >= kPkStages)
-            ok = tc_wait(ok, &pk_free[st], (uint32_t)((n / kPkStages - 1) & 1), p.status);
-          if (!ok) break;
-          mbar_arrive_expect_tx(&pk_full[st], kPkBytes);
-          uint8_t* dst = pk + (size_t)st * kPkBytes;
-          tc_tma_box_2d(dst, tm0, (job.b0 + b) * kBoxX, y0, &pk_full[st], pol);
-          tc_tma_box_2d(dst + kPkBytes / 2, tm1, (job.b0 + b) * kBoxX, y1, &pk_full[st], pol);
-        }
+        __syncwarp();
       }
     }
-    __syncwarp();
   } else if (warp == kActWarp) {
     // ================= activations: written by the kernel before this one =======================
     pdl_wait();
-    if (tc_elect()) {
-      int n = 0;
-      for (int j = 0; j < njobs && ok; ++j) {
-        const QmJob job = qm_job(p.deal, j);
-        const uint8_t* src = p.xb + (size_t)job.b0 * 2 * kBPer * kBBytes;
-        for (int s = 0; s < job.n * 2 * kBPer; ++s, ++n) {
-          const int st = n % kBStages;
-          if (n >= kBStages)
-            ok = tc_wait(ok, &b_free[st], (uint32_t)((n / kBStages - 1) & 1), p.status);
+    TcRing<kBStages> r;
+    for (int j = 0; j < njobs && ok; ++j) {
+      const QmJob job = qm_job(p.deal, j);
+      const uint8_t* src = p.xb + (size_t)job.b0 * Cfg::kSbBytes;
+      for (int s = 0; s < job.n && ok; ++s) {
+#pragma unroll
+        for (int h = 0; h < 2 * kBPer; ++h, r.advance()) {
+          const uint32_t bytes = h == 2 * kBPer - 1 ? kBBytes : Cfg::kBStep;
+          ok = tc_wait_w(&b_free[r.i], r.phase ^ 1, p.status);
           if (!ok) break;
-          mbar_arrive_expect_tx(&b_full[st], kBBytes);
-          bulk_g2s(bstg + (size_t)st * kBBytes, src + (size_t)s * kBBytes, kBBytes, &b_full[st]);
+          if (tc_elect()) {
+            mbar_arrive_expect_tx(&b_full[r.i], bytes);
+            bulk_g2s(bstg + (size_t)r.i * kBBytes, src, bytes, &b_full[r.i]);
+          }
+          __syncwarp();
+          src += bytes;
         }
       }
     }
-    __syncwarp();
   } else if (warp == kMmaWarp) {
-    // ================= MMA issue =================================================================
-    if (tc_elect()) {
-      int s = 0, h = 0;  // steps and activation stages so far
-      for (int j = 0; j < njobs && ok; ++j) {
-        const QmJob job = qm_job(p.deal, j);
-        const int buf = j % kAccBufs;
-        const uint32_t tmem_d = tmem + (uint32_t)(buf * NT);
-        if (j >= kAccBufs) {
-          ok = tc_wait(ok, &acc_free[buf], (uint32_t)((j / kAccBufs - 1) & 1), p.status);
-          tc_after_sync();
-        }
-        for (int i = 0; i < 2 * job.n && ok; ++i, ++s) {
-          const int st = s % kAStages;
-          ok = tc_wait(ok, &a_full[st], (uint32_t)((s / kAStages) & 1), p.status);
-          const uint32_t a_t = tmem + kA0 + (uint32_t)st * kQmACols;
+    // ================= MMA issue: the whole warp runs the loop, one lane issues =================
+    TcRing<kAStages> ra;
+    TcRing<kBStages> rb;
+    TcRing<kAccBufs> rd;
+    uint32_t eslot = 0;
+    const uint32_t b0 = tc_desc_lo(smem_u32(bstg), 128);
+    for (int j = 0; j < njobs && ok; ++j, rd.advance()) {
+      const int nu = qm_job(p.deal, j).n;
+      const uint32_t tmem_d = tmem + rd.i * NT;
+      ok = tc_wait_w(&acc_free[rd.i], rd.phase ^ 1, p.status);
+      if (!ok) break;
+      uint32_t accum = 0;
+      for (int u = 0; u < nu && ok; ++u) {
 #pragma unroll
-          for (int hh = 0; hh < kBPer; ++hh, ++h) {
-            const int bs = h % kBStages;
-            ok = tc_wait(ok, &b_full[bs], (uint32_t)((h / kBStages) & 1), p.status);
+        for (int half = 0; half < 2; ++half, ra.advance()) {
+          ok = tc_wait_w(&a_full[ra.i], ra.phase, p.status);
+          if (!ok) break;
+          const uint32_t a_t = tmem + kA0 + ra.i * kQmACols;
+#pragma unroll
+          for (int hh = 0; hh < kBPer; ++hh, rb.advance()) {
+            ok = tc_wait_w(&b_full[rb.i], rb.phase, p.status);
+            if (!ok) break;
             tc_after_sync();
-            const uint32_t bbase = smem_u32(bstg + (size_t)bs * kBBytes);
+            const uint32_t bdesc = b0 + rb.i * (kBBytes >> 4);
             constexpr int kMma = kQmStepK / 16 / kBPer;  // K = 16 per instruction: 8 columns of A
 #pragma unroll
-            for (int m = 0; m < kMma; ++m)
-              tc_mma_f16_ta(tmem_d, a_t + (hh * kMma + m) * 8,
-                            tc_smem_desc(bbase + (m >> 2) * (NT * 128) + (m & 3) * 256, 128, 1024, 0),
-                            p.idesc, (i > 0 || hh > 0 || m > 0) ? 1u : 0u);
-            tc_commit(&b_free[bs]);
+            for (int m = 0; m < kMma; ++m) {
+              tc_mma_f16_ta_w<tc_desc_hi(1024), Cfg::kIdesc>(
+                  tmem_d, a_t + (hh * kMma + m) * 8,
+                  bdesc + (((m >> 2) * (NT * 128) + (m & 3) * 256) >> 4), accum);
+              accum = 1;
+            }
+            if constexpr (Cfg::kSums)
+              if (half == 1 && hh == kBPer - 1) {  // residues of the super-block's mins
+                tc_mma_f16_ta_w<tc_desc_hi(256), Cfg::kIdesc>(tmem_d, tmem + Cfg::kE0 + eslot * 8,
+                                                              bdesc + (Cfg::kBStep >> 4), 1u);
+                eslot = (eslot + 1) % Cfg::kESlots;
+              }
+            tc_commit_w(&b_free[rb.i]);
           }
-          tc_commit(&a_free[st]);
+          tc_commit_w(&a_free[ra.i]);
         }
-        tc_commit(&acc_full[buf]);
       }
+      tc_commit_w(&acc_full[rd.i]);
     }
-    __syncwarp();
   } else {
     // ================= dequantise into tensor memory, epilogue ==================================
-    // lane quarter, 64-weight chunk of the step, which steps (0: even, 1: odd)
-    const int q = warp & 3, c2 = (warp >> 2) & 1, grp = warp >> 3;
-    const int c = 2 * grp + c2;  // chunk of the super-block: sub-blocks 2c, 2c+1
+    const int q = warp & 3, c2 = (warp >> 2) & 1, grp = warp >> 3;  // lane quarter, 64-weight
+                                                                    // chunk of the step, group
     // row of the tile that this tensor-memory lane holds: a gate/up tile has 16 gate rows and the
     // 16 up rows of the same outputs in every lane quarter
     const int erow = p.glu ? (lane & 15) + 16 * q + (lane >> 4) * 64 : q * 32 + lane;
@@ -329,7 +483,7 @@ __global__ void __launch_bounds__(kQmThreads, 1) kq_mma_kernel(const __grid_cons
     auto epilogue = [&](int j) {
       const QmJob job = qm_job(p.deal, j);
       const int buf = j % kAccBufs;
-      ok = tc_wait(ok, &acc_full[buf], (uint32_t)((j / kAccBufs) & 1), p.status);
+      ok = ok && tc_wait_w(&acc_full[buf], (uint32_t)((j / kAccBufs) & 1), p.status);
       tc_after_sync();
       int si = 0;
       if (!p.glu) {
@@ -341,42 +495,52 @@ __global__ void __launch_bounds__(kQmThreads, 1) kq_mma_kernel(const __grid_cons
       const int row = p.glu ? job.tile * 64 + 16 * q + (lane & 15)
                             : (job.tile - sg.tile0) * kQmRows + q * 32 + lane;
       const bool row_ok = ok && row < sg.N;
-#pragma unroll 1
+      // the whole share into registers, then the accumulator is free for the job after next
+      uint32_t va[NT / 64][16];
+#pragma unroll
       for (int g = 0; g < NT / 64; ++g) {  // 16 tokens at a time
-        const int m0 = (warp >> 2) * (NT / 4) + 16 * g;
-        if (m0 >= p.M) break;  // the same for the whole warp
-        uint32_t v[16];
+        uint32_t(&v)[16] = va[g];
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
             "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
               "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
               "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(lane_base + (uint32_t)(buf * NT + m0)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const int mc = min(16, p.M - m0);
-        if (job.slot >= 0) {
-          float* dst = p.part + (((size_t)blockIdx.x * 2 + job.slot) * NT + m0) * kQmRows + q * 32 + lane;
+            : "r"(lane_base + (uint32_t)(buf * NT + (warp >> 2) * (NT / 4) + 16 * g)));
+      }
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      tc_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_free[buf]);
 #pragma unroll
-          for (int t = 0; t < 16; ++t)
-            if (t < mc) dst[(size_t)t * kQmRows] = __uint_as_float(v[t]);
+      for (int g = 0; g < NT / 64; ++g) {
+        const int m0 = (warp >> 2) * (NT / 4) + 16 * g;
+        if (m0 >= p.M) break;  // the same for the whole warp
+        uint32_t(&v)[16] = va[g];
+        if (job.slot >= 0) {
+          // a part of a tile: four tokens of a row per 16-byte store
+          float4* dst = reinterpret_cast<float4*>(p.part) +
+                        (((size_t)blockIdx.x * 2 + job.slot) * (NT / 4) + (m0 >> 2)) * kQmRows + q * 32 + lane;
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            dst[t * kQmRows] = make_float4(__uint_as_float(v[4 * t]), __uint_as_float(v[4 * t + 1]),
+                                           __uint_as_float(v[4 * t + 2]), __uint_as_float(v[4 * t + 3]));
           continue;
         }
-        float rs[16];
-#pragma unroll
-        for (int t = 0; t < 16; t += 4) {
-          const float4 r4 = __ldcg(reinterpret_cast<const float4*>(p.rowscale + m0 + t));
-          rs[t] = r4.x; rs[t + 1] = r4.y; rs[t + 2] = r4.z; rs[t + 3] = r4.w;
-        }
+        const int mc = min(16, p.M - m0);
         if (!p.glu) {
           const size_t o0 = (size_t)m0 * sg.ldy + row;
           if (row_ok) {
+            float res[16];
+            if (sg.residual) {
+#pragma unroll
+              for (int t = 0; t < 16; ++t) res[t] = t < mc ? sg.residual[o0 + (size_t)t * sg.ldy] : 0.f;
+            }
 #pragma unroll
             for (int t = 0; t < 16; ++t)
               if (t < mc) {
-                float r = __uint_as_float(v[t]) * rs[t];
-                if (sg.residual) r = __fadd_rn(r, sg.residual[o0 + (size_t)t * sg.ldy]);
-                sg.y[o0 + (size_t)t * sg.ldy] = r;
+                const float r = __uint_as_float(v[t]) * rs_s[m0 + t];
+                sg.y[o0 + (size_t)t * sg.ldy] = sg.residual ? __fadd_rn(r, res[t]) : r;
               }
           }
         } else {
@@ -384,7 +548,8 @@ __global__ void __launch_bounds__(kQmThreads, 1) kq_mma_kernel(const __grid_cons
           const bool up = lane >= 16;
 #pragma unroll
           for (int t = 0; t < 16; t += 2) {
-            const float a = __uint_as_float(v[t]) * rs[t], b = __uint_as_float(v[t + 1]) * rs[t + 1];
+            const float a = __uint_as_float(v[t]) * rs_s[m0 + t];
+            const float b = __uint_as_float(v[t + 1]) * rs_s[m0 + t + 1];
             const float got = __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
             const float r = up ? glu_gate(got) * b : glu_gate(a) * got;
             const int tt = up ? t + 1 : t;
@@ -392,138 +557,201 @@ __global__ void __launch_bounds__(kQmThreads, 1) kq_mma_kernel(const __grid_cons
           }
         }
       }
-      tc_before_sync();
-      __syncwarp();
-      if (lane == 0)
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_free[buf]))
-                     : "memory");
     };
 
-    int n = 0;            // units so far
-    int s = grp;          // this warp's steps: grp, grp + 2, ...
-    int pending = -1;     // job whose epilogue is due
-    bool waited = false;  // the epilogue reads what the previous kernel wrote (row scales, residual)
+    bool waited = false;
+    // the epilogue reads what the previous kernel wrote (row scales, residual)
+    auto wait_previous = [&]() {
+      if (waited) return;
+      waited = true;
+      pdl_wait();
+      // this warp's tokens (the four warps that share them write the same values)
+      for (int t = lane; t < NT / 4; t += 32) {
+        const int m = (warp >> 2) * (NT / 4) + t;
+        rs_s[m] = m < p.M ? __ldcg(p.rowscale + m) : 0.f;
+      }
+      __syncwarp();
+    };
+    if constexpr (Cfg::kSums) {  // the upper half of every residue slot meets zero columns: keep it finite
+      if (warp < 4) {
+#pragma unroll
+        for (int e = 0; e < Cfg::kESlots; ++e)
+          asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%1,%1,%1};" ::"r"(
+                           lane_base + (uint32_t)(Cfg::kE0 + 8 * e + 4)), "r"(0)
+                       : "memory");
+      }
+    }
+    const bool epi = warp < kEpiWarps;
+    int s = grp;       // this warp's steps: grp, grp + kGroups, ...
+    int end = 0;       // first step of the next job
+    int pending = -1;  // job whose epilogue is due
+    TcRing<kPkStages> rp;
+    TcRing<kAStages> ra;
+    rp.advance(grp >> 1);
+    ra.advance(grp);
     for (int j = 0; j < njobs; ++j) {
-      const int nu = qm_job(p.deal, j).n;
-      for (int b = 0; b < nu; ++b, ++n, s += 2) {
-        const int ps = n % kPkStages, st = s % kAStages;
-        ok = tc_wait(ok, &pk_full[ps], (uint32_t)((n / kPkStages) & 1), p.status);
-        uint32_t o[32];
-        const uint8_t* blk = pk + (size_t)ps * kPkBytes + (size_t)erow * kUnit;
-        if (FMT == 12) {
+      end += 2 * qm_job(p.deal, j).n;
+      int since = 0;
+      for (; s < end; s += kGroups) {
+        const int c = 2 * (s & 1) + c2;  // sub-blocks 2c, 2c+1 of unit s / 2
+        ok = ok && tc_wait_w(&pk_full[rp.i], rp.phase, p.status);
+        const uint8_t* blk = pk + (size_t)rp.i * kPkBytes + (size_t)erow * kUnit;
+        const uint32_t a_t = a_base + ra.i * kQmACols;
+        auto stage_free = [&]() {
+          ok = ok && tc_wait_w(&a_free[ra.i], ra.phase ^ 1, p.status);
+          tc_after_sync();
+        };
+        auto store16 = [&](uint32_t col, const uint32_t (&o)[16]) {
+          asm volatile(
+              "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+              "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(a_t + col),
+              "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]),
+              "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]),
+              "r"(o[15])
+              : "memory");
+        };
+        if constexpr (FMT == 12) {
           // super-block of this row: f16 d, f16 dmin, 12 bytes of 6-bit scales and mins, 128 bytes
           // of nibbles (Hesper/Quantization/Q4_K_M.lean:13-52,120-144)
           const uint4 hdr = *reinterpret_cast<const uint4*>(blk);
           const uint4 qa = *reinterpret_cast<const uint4*>(blk + 16 + 32 * c);
           const uint4 qb = *reinterpret_cast<const uint4*>(blk + 32 + 32 * c);
-          const float2 dd = h2f(hdr.x);
           // scale / min bytes j and j+1 (j = 2c) out of the 12 packed bytes hdr.y, hdr.z, hdr.w
           uint32_t sc2, m2;  // two 6-bit values each, in bytes 0 and 1
           const int sh = 16 * c2;
-          if (grp == 0) {
+          if (!(s & 1)) {
             sc2 = (hdr.y >> sh) & 0x3F3Fu;
             m2 = (hdr.z >> sh) & 0x3F3Fu;
           } else {
             sc2 = ((hdr.w >> sh) & 0x0F0Fu) | ((hdr.y >> (sh + 2)) & 0x3030u);
             m2 = ((hdr.w >> (sh + 4)) & 0x0F0Fu) | ((hdr.z >> (sh + 2)) & 0x3030u);
           }
+          // {scale 2c, scale 2c+1} as f16, then multiplier and addend of the two nibble positions
+          const __half2 sc = __hsub2(as_h2(__byte_perm(sc2, 0x64646464u, 0x4140)), __floats2half2_rn(1024.f, 1024.f));
+          const __half2 mn = __hsub2(as_h2(__byte_perm(m2, 0x64646464u, 0x4140)), __floats2half2_rn(1024.f, 1024.f));
+          const __half2 mul = __hmul2(sc, __floats2half2_rn(1.f, 0.0625f));
+          const __half2 add = __hmul2(sc, __floats2half2_rn(-1024.f, -64.f));
+          // c = -dmin * m rounded to f16, and 32 times what that lost (an f16 fma forms dmin * m + c
+          // exactly up to its own rounding)
+          const __half2 dm = __high2half2(as_h2(hdr.x));
+          const __half2 cc = __hneg2(__hmul2(dm, mn));
+          const __half2 lost = __hmul2(__hneg2(__hfma2(dm, mn, cc)), __floats2half2_rn(32.f, 32.f));
           const uint32_t qq[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-          q4k_expand(qq, dd.x * (float)(sc2 & 0xFF), dd.y * (float)(m2 & 0xFF),
-                     dd.x * (float)(sc2 >> 8), dd.y * (float)(m2 >> 8), o);
+          const __half2 d = __low2half2(as_h2(hdr.x));
+          uint32_t o[16];
+          q4k_expand<false>(qq, d, __low2half2(mul), __low2half2(add), __low2half2(cc), o);
+          stage_free();
+          store16(0, o);
+          asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(
+                           lane_base + (uint32_t)(Cfg::kE0 + 8 * ((s >> 1) % Cfg::kESlots) + c)),
+                       "r"(as_u32(lost))
+                       : "memory");
+          q4k_expand<true>(qq, d, __high2half2(mul), __high2half2(add), __high2half2(cc), o);
+          store16(16, o);
         } else {
           // Q8_0 (Hesper/Layers/Linear.lean:6207-6223): blocks 2c and 2c+1 of the row's eight, 34
           // bytes each -- f16 d, then 32 int8.  The chunk starts on a word; block 2c's quants sit
           // two bytes into it (funnel shifts), block 2c+1's are word aligned.
           const uint32_t* wq = reinterpret_cast<const uint32_t*>(blk + 68 * c);
-          uint32_t w[17];
+          uint32_t w[9], o[16];
 #pragma unroll
-          for (int i = 0; i < 17; ++i) w[i] = wq[i];
+          for (int i = 0; i < 9; ++i) w[i] = wq[i];
           const __half2 d0 = __half2half2(__ushort_as_half((unsigned short)(w[0] & 0xFFFFu)));
           const __half2 d1 = __half2half2(__ushort_as_half((unsigned short)(w[8] >> 16)));
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
+          for (int i = 0; i < 8; ++i)
             q80_word(__funnelshift_r(w[i], w[i + 1], 16), d0, o[2 * i], o[2 * i + 1]);
-            q80_word(w[9 + i], d1, o[16 + 2 * i], o[16 + 2 * i + 1]);
-          }
+          stage_free();
+          store16(0, o);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) q80_word(wq[9 + i], d1, o[2 * i], o[2 * i + 1]);
+          store16(16, o);
         }
-        if (s >= kAStages) {
-          ok = tc_wait(ok, &a_free[st], (uint32_t)((s / kAStages - 1) & 1), p.status);
-          tc_after_sync();
-        }
-        HB_TMEM_ST32(a_base + (uint32_t)st * kQmACols, o);
         __syncwarp();
-        if (lane == 0)
-          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&pk_free[ps]))
-                       : "memory");
+        if (lane == 0) mbar_arrive(&pk_free[rp.i]);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_before_sync();
         __syncwarp();
-        if (lane == 0)
-          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&a_full[st]))
-                       : "memory");
+        if (lane == 0) mbar_arrive(&a_full[ra.i]);
+        ra.advance(kGroups);
+        rp.advance(((s & 1) + kGroups) >> 1);
         // the A stages are refilled for this job: now the previous job's accumulator
-        if (pending >= 0 && b == kAStages / 2 - 1) {
-          if (!waited) pdl_wait();
-          waited = true;
+        if (pending >= 0 && ++since == kAStages / kGroups) {
+          wait_previous();
           epilogue(pending);
           pending = -1;
         }
       }
       if (pending >= 0) {
-        if (!waited) pdl_wait();
-        waited = true;
+        wait_previous();
         epilogue(pending);
       }
-      pending = j;
+      pending = epi ? j : -1;
     }
-    if (!waited) pdl_wait();
+    wait_previous();
     if (pending >= 0) epilogue(pending);
   }
   tc_before_sync();
   __syncthreads();
   if (warp == kMmaWarp)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(*tmem_slot));
 }
 
-// Adds the partials of the left-over tiles in K order and runs the epilogue on the sums.  One
-// warp per (tile, token): 128 lanes' values as a float4 per lane.
-__global__ void __launch_bounds__(256) kq_combine_kernel(const __grid_constant__ QmParams p, int NT,
+// Adds the partials of the left-over tiles in K order and runs the epilogue on the sums: a thread
+// per tensor-memory lane and four tokens.
+__global__ void __launch_bounds__(128) kq_combine_kernel(const __grid_constant__ QmParams p, int NT,
                                                          int grid) {
   pdl_trigger();
   pdl_wait();
-  const int lane = threadIdx.x & 31, m = blockIdx.y * 8 + (threadIdx.x >> 5);
+  const int l = threadIdx.x, m0 = blockIdx.y * 4;
   const int t = blockIdx.x, nb = p.deal.nb, upc = p.deal.upc;
   const int c0 = t * nb / upc, c1 = ((t + 1) * nb - 1) / upc;
-  if (m >= p.M || c0 == c1) return;  // one CTA did the whole tile and has stored it
+  if (c0 == c1) return;  // one CTA did the whole tile and has stored it
+  const float4* part = reinterpret_cast<const float4*>(p.part) + (size_t)(m0 >> 2) * kQmRows + l;
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int cta = c0; cta <= c1; ++cta) {
-    const int slot = t - cta * upc / nb;
-    const float4 v = __ldcg(reinterpret_cast<const float4*>(
-        p.part + (((size_t)cta * 2 + slot) * NT + m) * kQmRows + 4 * lane));
-    a.x = __fadd_rn(a.x, v.x); a.y = __fadd_rn(a.y, v.y);
-    a.z = __fadd_rn(a.z, v.z); a.w = __fadd_rn(a.w, v.w);
+  for (int cb = c0; cb <= c1; cb += 8) {  // eight partials in flight
+    float4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int cta = cb + i, slot = t - cta * upc / nb;
+      v[i] = cta <= c1 ? __ldcg(part + ((size_t)cta * 2 + slot) * (NT / 4) * kQmRows)
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      a.x = __fadd_rn(a.x, v[i].x); a.y = __fadd_rn(a.y, v[i].y);
+      a.z = __fadd_rn(a.z, v[i].z); a.w = __fadd_rn(a.w, v[i].w);
+    }
   }
-  const float rs = __ldcg(p.rowscale + m);
-  float r[4] = {a.x * rs, a.y * rs, a.z * rs, a.w * rs};
-  const int tile = p.deal.W * grid + t;
+  const float4 rs = __ldcg(reinterpret_cast<const float4*>(p.rowscale + m0));
+  const float r[4] = {a.x * rs.x, a.y * rs.y, a.z * rs.z, a.w * rs.w};
+  const int tile = p.deal.W * grid + t, mc = min(4, p.M - m0);
   if (!p.glu) {
     int si = 0;
 #pragma unroll
     for (int i = 1; i < kQmMaxSeg; ++i)
       if (i < p.nseg && tile >= p.seg[i].tile0) si = i;
     const QmSeg& sg = p.seg[si];
-    const int row = (tile - sg.tile0) * kQmRows + 4 * lane;
-    const size_t o = (size_t)m * sg.ldy + row;
+    const int row = (tile - sg.tile0) * kQmRows + l;
+    const size_t o = (size_t)m0 * sg.ldy + row;
+    if (row < sg.N) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (row + e < sg.N) sg.y[o + e] = sg.residual ? __fadd_rn(r[e], sg.residual[o + e]) : r[e];
-  } else {  // lanes 8q..8q+3 hold gate rows 16q.., lanes 8q+4..8q+7 their up rows
+      for (int e = 0; e < 4; ++e)
+        if (e < mc) {
+          const size_t i = o + (size_t)e * sg.ldy;
+          sg.y[i] = sg.residual ? __fadd_rn(r[e], sg.residual[i]) : r[e];
+        }
+    }
+  } else {  // lanes 32q..32q+15 hold gate rows, lanes 32q+16..32q+31 their up rows
     const QmSeg& sg = p.seg[0];
-    const int row = tile * 64 + 16 * (lane >> 3) + 4 * (lane & 3);
+    const bool up = l & 16;
+    const int row = tile * 64 + 16 * (l >> 5) + (l & 15);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float up = __shfl_down_sync(0xffffffffu, r[e], 4);
-      if (!(lane & 4) && row + e < sg.N) sg.y[(size_t)m * sg.ldy + row + e] = glu_gate(r[e]) * up;
+    for (int e = 0; e < 4; e += 2) {  // gate lanes finish the even tokens, up lanes the odd ones
+      const float got = __shfl_xor_sync(0xffffffffu, up ? r[e] : r[e + 1], 16);
+      const float y = up ? glu_gate(got) * r[e + 1] : glu_gate(r[e]) * got;
+      const int ee = up ? e + 1 : e;
+      if (row < sg.N && ee < mc) sg.y[(size_t)(m0 + ee) * sg.ldy + row] = y;
     }
   }
 }
@@ -535,13 +763,13 @@ using namespace hb;
 // Dealing `tiles` row tiles of `nb` super-blocks to the SMs: whole waves, then the rest cut into
 // equal runs of units.  The rest stays whole (upc = nb) when cutting it saves less than the
 // partials cost: a unit takes a CTA about max(800, 16 * (NT / 2 + 10)) cycles, partials and the
-// second kernel about 3000 + 12 NT.
+// second kernel about 4000 + 12 NT.
 static QmDeal qm_deal(int tiles, int nb, int NT, int sms, int* grid) {
   QmDeal d = {tiles / sms, tiles % sms, nb, nb};
   if (d.R) {
     const int upc = (d.R * nb + sms - 1) / sms;
     const int unit = 16 * (NT / 2 + 10) > 800 ? 16 * (NT / 2 + 10) : 800;
-    if ((long)(nb - upc) * unit > 3000 + 12 * NT) d.upc = upc;
+    if ((long)(nb - upc) * unit > 4000 + 12 * NT) d.upc = upc;
   }
   *grid = d.W ? sms : (d.R * nb + d.upc - 1) / d.upc;
   return d;
@@ -550,8 +778,6 @@ static QmDeal qm_deal(int tiles, int nb, int NT, int sms, int* grid) {
 template <int NT, int FMT>
 static int kq_mma_launch(hb200_ctx* ctx, QmParams& p, int tiles, int nb, cudaStream_t st) {
   using Cfg = QmCfg<NT, FMT>;
-  // kind::f16: D = f32, A and B f16, both K-major, N = NT, M = 128
-  p.idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kQmRows >> 4) << 24);
   int grid = 0;
   p.deal = qm_deal(tiles, nb, NT, ctx->sm_count, &grid);
   if (p.deal.upc < nb &&
@@ -562,17 +788,17 @@ static int kq_mma_launch(hb200_ctx* ctx, QmParams& p, int tiles, int nb, cudaStr
   const int rc = hb_func_smem(ctx, reinterpret_cast<const void*>(kq_mma_kernel<NT, FMT>),
                               (size_t)Cfg::kSmem);
   if (rc != HB200_OK) return rc;
-  HB_CUDA(launch_pdl(kq_mma_kernel<NT, FMT>, dim3((unsigned)grid), dim3(kQmThreads),
+  HB_CUDA(launch_pdl(kq_mma_kernel<NT, FMT>, dim3((unsigned)grid), dim3(Cfg::kThreads),
                      (size_t)Cfg::kSmem, st, ctx->pdl, p));
   if (p.deal.R && p.deal.upc < nb)
-    HB_CUDA(launch_pdl(kq_combine_kernel, dim3((unsigned)p.deal.R, (unsigned)((p.M + 7) / 8)), dim3(256),
+    HB_CUDA(launch_pdl(kq_combine_kernel, dim3((unsigned)p.deal.R, (unsigned)((p.M + 3) / 4)), dim3(128),
                        0, st, ctx->pdl, p, NT, grid));
   return HB200_OK;
 }
 
 // For each of nseg tensors: y[m*ldy + n] = sum_k dequant(W)[n,k] x[m,k] (+ residual) for the
-// M <= NT tokens staged by hb_gemm16_split (dtype f16, single term, NT token rows per block;
-// NT = 64, 128 or 256), all in ONE product launch.  glu != 0: two tensors of equal shape, gate and
+// M <= NT tokens staged by hb_kq_stage for the same NT (64, 128 or 256) and format, all in ONE
+// product launch.  glu != 0: two tensors of equal shape, gate and
 // up, and segs[0].y = gelu_tanh(gate) * up.  Q4_K or Q8_0 (fmt: the GGUF type id); K a multiple
 // of 256.
 int hb_kq_mma_run_multi(hb200_ctx* ctx, const HbKqSeg* segs, int nseg, int K, int M, int NT, int glu,
@@ -629,4 +855,45 @@ int hb_kq_mma_run_multi(hb200_ctx* ctx, const HbKqSeg* segs, int nseg, int K, in
     case 128: return kq_mma_launch<128, 8>(ctx, p, tiles, nb, st);
     default: return kq_mma_launch<256, 8>(ctx, p, tiles, nb, st);
   }
+}
+
+// Bytes of staged activations per super-block of 256 weights.
+static size_t qm_sb_bytes(int fmt, int NT) { return (size_t)NT * (fmt == HB200_FMT_Q4_K ? 544 : 512); }
+
+// Most tokens (64, 128 or 256) one pass can stage at this K.
+int hb_kq_mma_max_tokens(int fmt, int K) {
+  for (int NT = 256; NT > 64; NT >>= 1)
+    if (qm_sb_bytes(fmt, NT) * (size_t)(K / 256) <= kScratchRowScale - kScratchLmSplit) return NT;
+  return 64;
+}
+
+// x[M][K] (M <= NT) -> f16 operand layout and row scales in the context scratch; optional pre-step
+// x' = d_pre_base + rmsnorm(d_x) * d_pre_gamma (written to d_pre_out), optional RMSNorm.
+int hb_kq_stage(hb200_ctx* ctx, int fmt, int K, int NT, const float* d_x, int M,
+                const float* d_pre_base, const float* d_pre_gamma, float* d_pre_out,
+                const float* d_rms_gamma, float rms_eps, cudaStream_t st) {
+  QmStage p = {};
+  p.sb_bytes = qm_sb_bytes(fmt, NT);
+  p.sums_off = fmt == HB200_FMT_Q4_K ? NT * 512 : 0;
+  HB_REQUIRE(p.sb_bytes * (size_t)(K / 256) <= kScratchRowScale - kScratchLmSplit && K <= 65536,
+             "kquant (fused batched): K=%d does not fit the activation scratch", K);
+  p.x = d_x;
+  p.gamma = d_rms_gamma;
+  p.pre_base = d_pre_base;
+  p.pre_gamma = d_pre_gamma;
+  p.pre_out = d_pre_out;
+  p.eps = rms_eps;
+  p.K = K;
+  p.xb = static_cast<uint8_t*>(ctx->d_scratch) + kScratchLmSplit;
+  p.rowscale = reinterpret_cast<float*>(static_cast<uint8_t*>(ctx->d_scratch) + kScratchRowScale);
+  const int n8 = K / 8;  // groups of 8 elements; one or two per thread, eight for a huge row
+  const int G = n8 <= 640 ? 1 : (n8 <= 2048 ? 2 : 8);
+  const int threads = ((n8 + G - 1) / G + 31) & ~31;
+  if (G == 1)
+    HB_CUDA(launch_pdl(kq_stage_kernel<1>, dim3(M), dim3(threads), 0, st, ctx->pdl, p));
+  else if (G == 2)
+    HB_CUDA(launch_pdl(kq_stage_kernel<2>, dim3(M), dim3(threads), 0, st, ctx->pdl, p));
+  else
+    HB_CUDA(launch_pdl(kq_stage_kernel<8>, dim3(M), dim3(threads), 0, st, ctx->pdl, p));
+  return HB200_OK;
 }

@@ -444,6 +444,9 @@ __global__ void __launch_bounds__(kLmThreads, 2)
 
 using namespace hb;
 
+int hb_gemm16_split_pre(hb200_ctx* ctx, int dtype, int K, const float* d_x, int M,
+                        const float* d_pre_base, const float* d_pre_gamma, float* d_pre_out,
+                        const float* d_rms_gamma, float rms_eps, int single, cudaStream_t st);
 // x[M][K] (M <= 64) -> hi/lo 16-bit operand blocks in the context scratch, optional RMSNorm.
 // single = 64, 128 or 256: only the rounded value (no lo term), that many token rows per
 // 64-wide K block (M <= single).

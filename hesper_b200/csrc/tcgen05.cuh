@@ -23,12 +23,12 @@ __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t smem_addr, uint32_t lb
   return d;
 }
 
-// One lane of a converged warp, as a predicate ptxas can trace to elect.sync.  MMAs are issued from
-// under it and never from under `lane == 0`: behind a data-dependent branch every tcgen05.mma
-// costs its thread ~132 cycles whatever its shape (the descriptors are moved to uniform
-// registers behind a loop over the active lanes); behind this one M = 128, K = 32 bytes with A in
-// tensor memory issues every 42 / 74 / 138 cycles at N = 64 / 128 / 256, the tensor pipe's own
-// 32 / 64 / 128 plus ten.  Loops over pipeline steps sit inside the branch, not around it.
+// One lane of a converged warp, as a predicate ptxas can trace to elect.sync.  How an MMA loop is
+// written decides what it costs (measured, M = 128, A in tensor memory, N = 64 / 128, cycles per
+// MMA): behind `lane == 0` 132 whatever N; behind this predicate 42 / 74; with the whole warp
+// converged and only the instruction itself predicated (tc_mma_f16_ta_w, tc_commit_w) 32 / 64, the
+// tensor pipe's own rate -- descriptors are then computed in the uniform datapath.  A completed
+// mbarrier costs 21 cycles through tc_wait_w and ~185 through the bounded loop of tc_wait.
 __device__ __forceinline__ bool tc_elect() {
   uint32_t p;
   asm volatile(
@@ -59,6 +59,35 @@ __device__ __forceinline__ void tc_before_sync() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
 
+// The same two for a converged warp: every lane calls, one issues.  The MMA warp shares its
+// scheduler with compute warps, so what an MMA costs is its instruction count: the descriptor's
+// high word (no swizzle, LBO, SBO) and the instruction descriptor are immediates, and the low
+// word -- smem address / 16 with LBO above it, tc_desc_lo -- is one addition per MMA.
+__host__ __device__ constexpr uint32_t tc_desc_hi(uint32_t sbo) { return ((sbo >> 4) & 0x3FFF) | (1u << 14); }
+__device__ __forceinline__ uint32_t tc_desc_lo(uint32_t smem_addr, uint32_t lbo) {
+  return ((smem_addr & 0x3FFFF) >> 4) | ((lbo >> 4) << 16);
+}
+template <uint32_t kDescHi, uint32_t kIdesc>
+__device__ __forceinline__ void tc_mma_f16_ta_w(uint32_t tmem_d, uint32_t tmem_a, uint32_t bdesc_lo,
+                                                uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 bd;\n\tmov.b64 bd, {%2, %3};\n\t"
+      "elect.sync _|e, 0xffffffff;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(bdesc_lo), "n"(kDescHi), "n"(kIdesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_w(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+          smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // One box of a 2-D tensor map into shared memory; completion is counted in bytes on `bar`.
 // x in elements of the innermost dimension (x * element size must be a multiple of 16).
 __device__ __forceinline__ void tc_tma_box_2d(void* dst, const CUtensorMap* tm, int x, int y,
@@ -81,6 +110,45 @@ __device__ __forceinline__ bool tc_wait(bool ok, uint64_t* bar, uint32_t parity,
   atomicOr(status, kStatusMbarTimeout);
   return false;
 }
+
+// The slow path of tc_wait_w: the barrier was not complete at the first look.
+static __device__ __noinline__ bool tc_wait_slow(uint32_t bar, uint32_t parity, uint32_t* status) {
+#pragma unroll 1
+  for (uint32_t it = 0; it < (1u << 17); ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  atomicOr(status, kStatusMbarTimeout);
+  return false;
+}
+// Bounded wait for the inner loops: one inline try, the loop out of line.  False when the bound
+// ran out (the caller leaves its loop; what it would have produced never arrives, so the others'
+// waits run out as well and the kernel ends).
+__device__ __forceinline__ bool tc_wait_w(uint64_t* bar, uint32_t parity, uint32_t* status) {
+  if (mbar_try_wait(bar, parity)) return true;
+  return tc_wait_slow(smem_u32(bar), parity, status);
+}
+
+// Position in a ring of N stages and the parity of its current lap.  A consumer waits for parity
+// `phase`; a producer waits for the stage to be free with parity `phase ^ 1`, which a fresh barrier
+// passes at once.
+template <int N>
+struct TcRing {
+  uint32_t i = 0, phase = 0;
+  __device__ __forceinline__ void advance(int by = 1) {  // by <= N
+    i += by;
+    if (i >= N) {
+      i -= N;
+      phase ^= 1;
+    }
+  }
+};
 
 #define HB_TMEM_LD32(v, addr)                                                                  \
   asm volatile(                                                                                \
