@@ -154,6 +154,25 @@ def load() -> C.CDLL:
     return _lib
 
 
+_bind = None
+
+
+def binding():
+    """The C++ side of the layer API (csrc/py_binding.cpp); raises if it was not built."""
+    global _bind
+    if _bind is None:
+        load()  # the library first: _binding.so links against it
+        import torch  # noqa: F401  (its symbols must be loaded)
+        try:
+            from . import _binding
+        except ImportError as e:
+            raise HesperB200Error(-2, f"hesper_b200/_binding.so does not load ({e}): run "
+                                      "`python -m hesper_b200.build`") from e
+        _binding.set_error_type(HesperB200Error)
+        _bind = _binding
+    return _bind
+
+
 def check(code: int) -> None:
     if code != HB200_OK:
         raise HesperB200Error(code, load().hb200_last_error().decode("utf-8", "replace"))

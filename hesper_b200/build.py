@@ -1,4 +1,5 @@
-"""Builds libhesper_b200.so (CUDA kernels + C ABI) in-tree with nvcc for sm_100a.
+"""Builds libhesper_b200.so (CUDA kernels + C ABI) in-tree with nvcc for sm_100a, and
+_binding.so (the layer API's calls as C++ over torch and the C ABI) with g++.
 
 Run as ``python -m hesper_b200.build``.  nvcc cross-compiles without a GPU.  The
 shared object carries a static CUDA runtime, so it needs only the driver.
@@ -6,6 +7,7 @@ shared object carries a static CUDA runtime, so it needs only the driver.
 from __future__ import annotations
 
 import os
+import shutil
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -14,6 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libhesper_b200.so")
+BINDING = os.path.join(HERE, "_binding.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -31,6 +34,31 @@ def _stale(target: str, deps) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def build_binding(force: bool = False) -> str:
+    """_binding.so, linked against the library beside it and the torch that is installed."""
+    src = os.path.join(CSRC, "py_binding.cpp")
+    header = os.path.join(HERE, "..", "include", "hesper_b200.h")
+    if not (force or _stale(BINDING, [src, header])):
+        return BINDING
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    tdir = os.path.dirname(torch.__file__)
+    nvcc = shutil.which(os.environ.get("HB200_NVCC", "nvcc"))
+    cuda = cpp_extension.CUDA_HOME or (os.path.dirname(os.path.dirname(nvcc)) if nvcc else "/usr/local/cuda")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wno-deprecated-declarations",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(cuda, "include")]
+    cmd += ["-I" + p for p in cpp_extension.include_paths()]
+    cmd += [src, "-o", BINDING, "-L" + HERE, "-l:libhesper_b200.so", "-Wl,-rpath,$ORIGIN",
+            "-L" + os.path.join(tdir, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed: " + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+    return BINDING
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -64,6 +92,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         link = [nvcc, "-shared", "-o", LIB] + objs + ["-cudart", "static", "-ldl",
                 "-gencode", "arch=compute_100a,code=sm_100a"]
         run(link)
+    build_binding(force)
     return LIB
 
 

@@ -6,8 +6,9 @@ reference's own:
   * ``LinearLayer``    -- Hesper/Layers/Linear.lean:5636-5669, 7115-7942
   * ``execute_flash_attention_v11`` -- Hesper/WGSL/FlashAttentionExperiments.lean:572
 torch is used for device memory and streams only; every computation goes
-through the C ABI (``include/hesper_b200.h``).  There is no CPU path: without
-the CUDA library or a GPU these calls raise.
+through the C ABI (``include/hesper_b200.h``), called from C++
+(``csrc/py_binding.cpp``: checks, output allocation and call in one step).
+There is no CPU path: without the CUDA library or a GPU these calls raise.
 """
 from __future__ import annotations
 
@@ -19,11 +20,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import BitLinearSeg, KQuantSeg, check
-
-
-def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else C.c_void_p(t.data_ptr())
+from ._lib import check
 
 
 def _stream_handle(stream) -> C.c_void_p:
@@ -57,6 +54,8 @@ class Context:
         else:
             check(self._lib.hb200_ctx_create(self.device, C.byref(h)))
         self._h = h
+        self._b = _lib.binding()
+        self._addr = h.value
 
     @property
     def handle(self) -> C.c_void_p:
@@ -83,6 +82,7 @@ class Context:
         if getattr(self, "_h", None) is not None and self._h.value:
             self._lib.hb200_ctx_destroy(self._h)
             self._h = C.c_void_p()
+            self._addr = 0
 
     def __del__(self):
         try:
@@ -117,12 +117,6 @@ class BitLinear:
         s = torch.tensor([scale], dtype=torch.float32, device=dev)
         return cls(ctx, p, s, in_dim, out_dim)
 
-    def _x(self, x: torch.Tensor):
-        x = _need(x, torch.float32, "input")
-        if x.numel() % self.in_dim:
-            raise ValueError("input size is not a multiple of in_dim")
-        return x, x.numel() // self.in_dim
-
     def forward(self, x: torch.Tensor, *, residual: Optional[torch.Tensor] = None,
                 rms_gamma: Optional[torch.Tensor] = None, eps: float = 1e-5,
                 return_acc: bool = False, out: Optional[torch.Tensor] = None, stream=None):
@@ -131,22 +125,9 @@ class BitLinear:
 
         Returns y [M, out_dim] f32, or (y, acc int32 [M, out_dim], d f32 [M]) with return_acc.
         """
-        x, M = self._x(x)
-        y = out if out is not None else torch.empty((M, self.out_dim), dtype=torch.float32,
-                                                    device=x.device)
-        acc = d = None
-        if return_acc:
-            acc = torch.empty((M, self.out_dim), dtype=torch.int32, device=x.device)
-            d = torch.empty((M,), dtype=torch.float32, device=x.device)
-        if residual is not None:
-            _need(residual, torch.float32, "residual")
-        if rms_gamma is not None:
-            _need(rms_gamma, torch.float32, "rms_gamma")
-        check(self.ctx._lib.hb200_bitlinear_forward(
-            self.ctx.handle, _ptr(self.packed), _ptr(self.scale), self.in_dim, self.out_dim,
-            _ptr(x), M, _ptr(rms_gamma), C.c_float(eps), _ptr(residual), _ptr(acc), _ptr(d),
-            _ptr(y), _stream_handle(stream)))
-        return (y, acc, d) if return_acc else y
+        c = self.ctx
+        return c._b.bitlinear_forward(c._addr, self.packed, self.scale, self.in_dim, self.out_dim, x,
+                                      rms_gamma, eps, residual, return_acc, out, stream)
 
     def forward_with_residual(self, x, residual, **kw):
         return self.forward(x, residual=residual, **kw)
@@ -161,38 +142,21 @@ class BitLinear:
         """BitLinear.forwardFusedGateUpReluSqrMul (Hesper/Layers/BitLinear.lean:1419)."""
         if (gate.in_dim, gate.out_dim) != (up.in_dim, up.out_dim):
             raise ValueError("gate and up must have the same shape")
-        x, M = gate._x(x)
-        y = out if out is not None else torch.empty((M, gate.out_dim), dtype=torch.float32,
-                                                    device=x.device)
-        check(gate.ctx._lib.hb200_bitlinear_gateup_relu2(
-            gate.ctx.handle, _ptr(gate.packed), _ptr(gate.scale), _ptr(up.packed), _ptr(up.scale),
-            gate.in_dim, gate.out_dim, _ptr(x), M, _ptr(rms_gamma), C.c_float(eps), _ptr(y),
-            _stream_handle(stream)))
-        return y
+        c = gate.ctx
+        return c._b.bitlinear_gateup(c._addr, gate.packed, gate.scale, up.packed, up.scale, gate.in_dim,
+                                     gate.out_dim, x, rms_gamma, eps, out, stream)
 
     @staticmethod
     def forward_multi(layers: Sequence["BitLinear"], x: torch.Tensor, *, rms_gamma=None,
                       eps: float = 1e-5, residuals=None, return_acc: bool = False, stream=None):
         """Several BitLinear layers over the same input in one launch (fused q/k/v)."""
         l0 = layers[0]
-        x, M = l0._x(x)
-        segs = (BitLinearSeg * len(layers))()
-        ys, accs = [], []
-        for i, l in enumerate(layers):
+        for l in layers:
             if l.in_dim != l0.in_dim:
                 raise ValueError("all layers must share in_dim")
-            y = torch.empty((M, l.out_dim), dtype=torch.float32, device=x.device)
-            a = torch.empty((M, l.out_dim), dtype=torch.int32, device=x.device) if return_acc else None
-            r = residuals[i] if residuals is not None else None
-            ys.append(y)
-            accs.append(a)
-            segs[i] = BitLinearSeg(l.packed.data_ptr(), l.scale.data_ptr(),
-                                   r.data_ptr() if r is not None else None, y.data_ptr(),
-                                   a.data_ptr() if a is not None else None, l.out_dim)
-        check(l0.ctx._lib.hb200_bitlinear_forward_multi(
-            l0.ctx.handle, segs, len(layers), l0.in_dim, _ptr(x), M, _ptr(rms_gamma),
-            C.c_float(eps), None, _stream_handle(stream)))
-        return (ys, accs) if return_acc else ys
+        c = l0.ctx
+        return c._b.bitlinear_multi(c._addr, [(l.packed, l.scale, l.out_dim) for l in layers], l0.in_dim, x,
+                                    rms_gamma, eps, residuals, return_acc, stream)
 
 
 class QuantFormat(enum.IntEnum):
@@ -225,22 +189,12 @@ class LinearLayer:
         b = torch.from_numpy(np.ascontiguousarray(block_bytes, dtype=np.uint8).reshape(-1)).to(dev)
         return cls(ctx, b, QuantFormat(fmt), in_dim, out_dim)
 
-    def _x(self, x):
-        x = _need(x, torch.float32, "input")
-        if x.numel() % self.in_dim:
-            raise ValueError("input size is not a multiple of in_dim")
-        return x, x.numel() // self.in_dim
-
     def forward(self, x: torch.Tensor, *, residual=None, rms_gamma=None, eps: float = 1e-6,
                 out=None, stream=None) -> torch.Tensor:
         """LinearLayer.forward (:7115); with rms_gamma forwardFusedRMSNormLinear."""
-        x, M = self._x(x)
-        y = out if out is not None else torch.empty((M, self.out_dim), dtype=torch.float32,
-                                                    device=x.device)
-        check(self.ctx._lib.hb200_kquant_forward(
-            self.ctx.handle, int(self.fmt), _ptr(self.blocks), self.in_dim, self.out_dim, _ptr(x),
-            M, _ptr(rms_gamma), C.c_float(eps), _ptr(residual), _ptr(y), _stream_handle(stream)))
-        return y
+        c = self.ctx
+        return c._b.kquant_forward(c._addr, self.fmt, self.blocks, self.in_dim, self.out_dim, x, rms_gamma,
+                                   eps, residual, out, stream)
 
     @staticmethod
     def forward_fused_gate_up(gate: "LinearLayer", up: "LinearLayer", x, *, rms_gamma=None,
@@ -249,22 +203,10 @@ class LinearLayer:
 
         pre=(base, gamma): the layer input becomes x' = base + rmsnorm(x) * gamma first
         (a post-norm with its residual add); returns (y, x') in that case."""
-        x, M = gate._x(x)
-        y = out if out is not None else torch.empty((M, gate.out_dim), dtype=torch.float32,
-                                                    device=x.device)
-        if pre is not None:
-            base, pg = pre
-            xo = torch.empty_like(x)
-            check(gate.ctx._lib.hb200_kquant_gateup_gelu_pre(
-                gate.ctx.handle, int(gate.fmt), _ptr(gate.blocks), _ptr(up.blocks), gate.in_dim,
-                gate.out_dim, _ptr(x), M, _ptr(base), _ptr(pg), _ptr(xo), _ptr(rms_gamma),
-                C.c_float(eps), _ptr(y), _stream_handle(stream)))
-            return y, xo
-        check(gate.ctx._lib.hb200_kquant_gateup_gelu(
-            gate.ctx.handle, int(gate.fmt), _ptr(gate.blocks), _ptr(up.blocks), gate.in_dim,
-            gate.out_dim, _ptr(x), M, _ptr(rms_gamma), C.c_float(eps), _ptr(y),
-            _stream_handle(stream)))
-        return y
+        base, pg = pre if pre is not None else (None, None)
+        c = gate.ctx
+        return c._b.kquant_gateup(c._addr, gate.fmt, gate.blocks, up.blocks, gate.in_dim, gate.out_dim, x,
+                                  rms_gamma, eps, base, pg, out, stream)
 
     @staticmethod
     def forward_multi(layers: Sequence["LinearLayer"], x, *, rms_gamma=None, eps: float = 1e-6,
@@ -273,27 +215,11 @@ class LinearLayer:
 
         pre=(base, gamma): the layers' input becomes x' = base + rmsnorm(x) * gamma first;
         returns (ys, x') in that case."""
+        base, pg = pre if pre is not None else (None, None)
         l0 = layers[0]
-        x, M = l0._x(x)
-        segs = (KQuantSeg * len(layers))()
-        ys = []
-        for i, l in enumerate(layers):
-            y = torch.empty((M, l.out_dim), dtype=torch.float32, device=x.device)
-            r = residuals[i] if residuals is not None else None
-            ys.append(y)
-            segs[i] = KQuantSeg(l.blocks.data_ptr(), r.data_ptr() if r is not None else None,
-                                y.data_ptr(), l.out_dim)
-        if pre is not None:
-            base, pg = pre
-            xo = torch.empty_like(x)
-            check(l0.ctx._lib.hb200_kquant_forward_multi_pre(
-                l0.ctx.handle, int(l0.fmt), segs, len(layers), l0.in_dim, _ptr(x), M, _ptr(base),
-                _ptr(pg), _ptr(xo), _ptr(rms_gamma), C.c_float(eps), _stream_handle(stream)))
-            return ys, xo
-        check(l0.ctx._lib.hb200_kquant_forward_multi(
-            l0.ctx.handle, int(l0.fmt), segs, len(layers), l0.in_dim, _ptr(x), M, _ptr(rms_gamma),
-            C.c_float(eps), _stream_handle(stream)))
-        return ys
+        c = l0.ctx
+        return c._b.kquant_multi(c._addr, l0.fmt, [(l.blocks, l.out_dim) for l in layers], l0.in_dim, x,
+                                 rms_gamma, eps, residuals, base, pg, stream)
 
 
 def flash_attention_workspace(ctx: Context, B: int, H: int, Hkv: int, D: int, max_seq: int,
@@ -312,20 +238,8 @@ def flash_attention_prefill(ctx: Context, q: torch.Tensor, k_cache: torch.Tensor
     q [B, T, H, D] f32 or f16: T new tokens per sequence whose K/V already sit at positions
     seqlens[b]-T .. seqlens[b]-1 of the f16 caches [B, Hkv, max_seq_len, D]; returns [B, T, H, D].
     """
-    _need(q, q.dtype, "q")
-    _need(k_cache, torch.float16, "k_cache")
-    _need(v_cache, torch.float16, "v_cache")
-    _need(seqlens, torch.int32, "seqlens")
-    B, T = int(q.shape[0]), int(q.shape[1])
-    n = ctx._lib.hb200_attn_prefill_workspace_bytes(ctx.handle, B, T, num_heads, num_kv_heads,
-                                                    head_dim, max_seq_len)
-    ws = torch.empty((max(int(n), 16),), dtype=torch.uint8, device=q.device)
-    o = torch.empty((B, T, num_heads, head_dim), dtype=torch.float32, device=q.device)
-    check(ctx._lib.hb200_attn_prefill(
-        ctx.handle, _ptr(q), int(q.dtype == torch.float16), _ptr(k_cache), _ptr(v_cache),
-        _ptr(seqlens), B, T, num_heads, num_kv_heads, head_dim, max_seq_len, int(window),
-        C.c_float(scale), _ptr(ws), C.c_size_t(ws.numel()), _ptr(o), _stream_handle(stream)))
-    return o
+    return ctx._b.attn_prefill(ctx._addr, q, k_cache, v_cache, seqlens, num_heads, num_kv_heads, head_dim,
+                               max_seq_len, scale, window, stream)
 
 
 def execute_flash_attention_v11(ctx: Context, q: torch.Tensor, k_cache: torch.Tensor,
@@ -338,21 +252,5 @@ def execute_flash_attention_v11(ctx: Context, q: torch.Tensor, k_cache: torch.Te
     q [B, H, D] f32 or f16; k_cache / v_cache [B, Hkv, max_seq_len, D] f16;
     seqlens [B] int32 (the reference's params[1] = cacheLen, one per sequence).
     """
-    if q.dtype not in (torch.float32, torch.float16):
-        raise TypeError("q must be f32 or f16")
-    _need(q, q.dtype, "q")
-    _need(k_cache, torch.float16, "k_cache")
-    _need(v_cache, torch.float16, "v_cache")
-    _need(seqlens, torch.int32, "seqlens")
-    B = seqlens.numel()
-    if workspace is None:
-        workspace = flash_attention_workspace(ctx, B, num_heads, num_kv_heads, head_dim,
-                                              max_seq_len, q.device)
-    o = out if out is not None else torch.empty((B, num_heads, head_dim), dtype=torch.float32,
-                                                device=q.device)
-    check(ctx._lib.hb200_attn_decode(
-        ctx.handle, _ptr(q), int(q.dtype == torch.float16), _ptr(k_cache), _ptr(v_cache),
-        _ptr(seqlens), B, num_heads, num_kv_heads, head_dim, max_seq_len, int(window),
-        C.c_float(scale), _ptr(workspace), C.c_size_t(workspace.numel()), _ptr(o),
-        _stream_handle(stream)))
-    return o
+    return ctx._b.attn_decode(ctx._addr, q, k_cache, v_cache, seqlens, num_heads, num_kv_heads, head_dim,
+                              max_seq_len, scale, window, workspace, out, stream)
