@@ -1,90 +1,103 @@
-// attention_prefill.cu -- causal GQA attention of a prompt chunk, tiled over queries.
+// attention_prefill.cu -- causal GQA attention of a prompt chunk on the 5th-generation tensor cores.
 //
 // T new query tokens per sequence against the f16 KV cache that already holds them (the role
 // of the reference's batched prefill kernels, flashAttentionBatchKernelF16 and its SWA variant,
-// Hesper/WGSL/FlashAttention.lean:601,1621-1624; math of flashAttentionSpec, :60-90).  The
-// decode kernel can serve a chunk by treating every token as a query of its own, but then every
-// token streams its whole visible cache; here a CTA owns 64 query rows -- 64 / G consecutive
-// tokens times the G query heads of one KV head -- and walks the positions those tokens see in
-// tiles of 64 (32 at head_dim 256), so a K/V tile is read once per 64 / G tokens:
-//   * Q (pre-multiplied by scale * log2 e, f16) stays in shared memory for the whole CTA;
-//   * K/V tiles arrive by 16-byte cp.async into a two-stage ring (XOR-swizzled 16-byte units,
-//     conflict-free ldmatrix); ring caches map position p to slot p % slots;
-//   * S = Q K^T and O += P V on mma.sync.m16n8k16 (f16 in, f32 accumulate), one warp per 16 rows;
-//     the softmax is the online form in the exp2 domain, P is rounded to f16 for the second
-//     product (same rounding as the decode kernel's FAST mode: bar 2e-3 against an f64 evaluation);
+// Hesper/WGSL/FlashAttention.lean:601,1621-1624; math of flashAttentionSpec, :60-90).  A CTA owns
+// 128 query rows -- 128 / G consecutive tokens times the G query heads of one KV head -- and walks
+// the positions those tokens see in tiles of 64, so a K/V tile is read once per 128 / G tokens.
+//
+//   * warp 4: K and V tiles by 2-D tensor-map TMA (boxes of 64 positions x 64 dims, 128-byte
+//     swizzle) into one ring of shared-memory slots, K(j), V(j) alternating.  A tile of a ring
+//     cache never spans the wrap: the positions are walked as at most two runs of slots.
+//   * warp 5: tcgen05.mma kind::f16.  S(j) = Q K^T with Q in TENSOR MEMORY (pre-multiplied by
+//     scale * log2 e, f16) and K as the K-major operand; O += P V with P in tensor memory (it
+//     replaces the S it came from) and V, as it lies in the cache, as the MN-major operand.
+//     S has two buffers: S(j+1) runs while the softmax works on S(j).
+//   * warps 0-3: one thread per row.  Online softmax in the exp2 domain with P rounded to f16
+//     (same rounding as the decode kernel's FAST mode: bar 2e-3 against an f64 evaluation).  The
+//     reference maximum of a row moves only when a tile exceeds it by more than 2^8 (P then stays
+//     below 2^8, far inside f16): O is rescaled in tensor memory a few times per row instead
+//     of once per tile, and the quotient O / l is the same.
 //   * a row's visible positions are [max(0, pos - window + 1), pos] with pos the token's own
 //     position: causal inside the chunk, sliding window if asked.
+//
+// Tensor memory at D = 256: O 256 columns, Q 128, S 2 x 64 = all 512.  What bounds it: a tile is
+// 16 MMAs of N=64 plus 4 of N=256, 1024 cycles of the tensor pipe, against ~700 of softmax (64
+// exponentials per row are 512 cycles of the special-function unit) that overlap all but the part
+// between S(j) and P(j); K and V come from L2 at 64 KB per tile.  When the query tiles leave SMs
+// idle the positions are dealt to several CTAs and a second kernel merges their partials.
 #include <math_constants.h>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace hb {
 
-constexpr int kPfWarps = 4;
-constexpr int kPfThreads = kPfWarps * 32;
-constexpr int kPfRows = 64;   // query rows per CTA
-// positions per K/V tile: 64, and 32 at head_dim 256, where the 128 output accumulators per
-// lane leave no registers for a 64-wide score tile
-template <int D>
-struct PfTile {
-  static constexpr int value = D >= 256 ? 32 : 64;
-};
+constexpr int kPfRows = 128;   // query rows per CTA = MMA M
+constexpr int kPfTile = 64;    // positions per K/V tile
+constexpr int kPfThreads = 192;
+constexpr int kPfMaxSplits = 16;
 
 struct PfParams {
-  const void* q;        // [nseq][T][H][D] f32 or f16
-  const __half* k;      // [nseq][Hkv][slots][D]
-  const __half* v;
+  CUtensorMap tmk, tmv;    // caches as [nseq * Hkv * slots][D], boxes of 64 rows x 64 dims
+  const void* q;           // [nseq][T][H][D] f32 or f16
   const int32_t* seqlens;  // [nseq] lengths after the T tokens
-  float* out;           // [nseq][T][H][D]
+  float* out;              // [nseq][T][H][D]
   int q_is_f16;
   int nseq, T, H, Hkv, G, slots, window, ring;
   float scale_log2;
-  // nsplit > 1: the K/V tiles of a query tile are dealt to nsplit CTAs (a long context at a small
-  // batch would otherwise fill a fraction of the SMs); each writes its unnormalised partial and
-  // its (max, sum), attn_prefill_merge_kernel combines them
+  // nsplit > 1: the K/V tiles of a query tile are dealt to nsplit CTAs; each writes its
+  // unnormalised partial and its (max, sum), attn_prefill_merge_kernel combines them
   int nsplit;
   float* part_o;   // [nseq][T][H][nsplit][D]
   float* part_ml;  // [nseq][T][H][nsplit][2]  (max in the exp2 domain, sum)
+  uint32_t* status;
 };
 
 template <int D>
 struct PfCfg {
-  static constexpr int kQStride = D + 8;                      // halves per Q row (bank spread)
-  static constexpr int kQBytes = kPfRows * kQStride * 2;
-  static constexpr int kRowBytes = D * 2;
-  static constexpr int kTile = PfTile<D>::value;
-  static constexpr int kTileBytes = kTile * kRowBytes;        // one of K or V
-  static constexpr int kSmem = kQBytes + 2 * 2 * kTileBytes;  // Q + two stages of (K, V)
+  static constexpr int kO0 = 0, kQ0 = D, kS0 = D + D / 2;   // tensor-memory columns
+  static constexpr int kCols = D == 256 ? 512 : (D == 128 ? 512 : 256);
+  static constexpr int kSlotBytes = kPfTile * D * 2;        // one K or V tile: 32 / 16 / 8 KB
+  static constexpr int kBoxBytes = kPfTile * 128;
+  static constexpr int kSlots = 6;
+  static constexpr int kOutStride = D * 4 + 16;             // padded f32 row of the epilogue
+  static constexpr int kRing = kSlots * kSlotBytes;
+  static constexpr int kData = kRing > kPfRows * kOutStride ? kRing : kPfRows * kOutStride;
+  static constexpr int kSmem = 1024 + kData;
+  static constexpr uint32_t kIdescS = (1u << 4) | ((uint32_t)(kPfTile >> 3) << 17) | ((uint32_t)(kPfRows >> 4) << 24);
+  // B (= V) is MN-major
+  static constexpr uint32_t kIdescO =
+      (1u << 4) | (1u << 16) | ((uint32_t)(D >> 3) << 17) | ((uint32_t)(kPfRows >> 4) << 24);
+  static_assert(kS0 + 2 * kPfTile <= kCols, "tensor memory columns");
+  static_assert(kSmem <= 232448, "shared memory");
 };
 
-__device__ __forceinline__ void pf_cp16(void* dst, const void* src, bool valid) {
-  const uint32_t n = valid ? 16u : 0u;  // src-size 0: the 16 bytes are zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n)
-               : "memory");
-}
-__device__ __forceinline__ void pf_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void pf_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ void pf_ldsm(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(p)));
-}
-__device__ __forceinline__ void pf_ldsm_t(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(p)));
-}
-__device__ __forceinline__ void pf_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
-                                       uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+// One tile of the walk: first position, its slot, and how many of the 64 are real.
+struct PfTileAt {
+  int pos, slot, n;
+};
+// The positions [lo, hi] as at most two runs of slots (a ring wraps once at most, window + T - 1
+// <= slots), each cut into tiles from its own start.
+struct PfWalk {
+  int lo, hi, slot0, run0, tiles0, tiles;
+  __device__ __forceinline__ PfWalk(int lo_, int hi_, int slots, int ring) : lo(lo_), hi(hi_) {
+    const int n = hi >= lo ? hi - lo + 1 : 0;
+    slot0 = ring ? lo % slots : lo;
+    run0 = ring ? min(n, slots - slot0) : n;
+    tiles0 = (run0 + kPfTile - 1) / kPfTile;
+    tiles = tiles0 + (n - run0 + kPfTile - 1) / kPfTile;
+  }
+  __device__ __forceinline__ PfTileAt at(int j) const {
+    if (j < tiles0) return {lo + j * kPfTile, slot0 + j * kPfTile, min(kPfTile, run0 - j * kPfTile)};
+    const int k = j - tiles0, p = lo + run0 + k * kPfTile;
+    return {p, k * kPfTile, min(kPfTile, hi - p + 1)};
+  }
+};
+
+__device__ __forceinline__ float pf_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 __device__ __forceinline__ uint32_t pf_pack(float a, float b) {
   __half2 h = __floats2half2_rn(a, b);
@@ -92,23 +105,49 @@ __device__ __forceinline__ uint32_t pf_pack(float a, float b) {
 }
 
 template <int D>
-__global__ void __launch_bounds__(kPfThreads, D >= 256 ? 1 : 2)
+__global__ void __launch_bounds__(kPfThreads, 1)
     attn_prefill_tiled_kernel(const __grid_constant__ PfParams p) {
   using Cfg = PfCfg<D>;
-  constexpr int KS = D / 16;  // k-steps of the first product
-  constexpr int NO = D / 8;   // n-tiles of the output
-  constexpr int CPR = D / 8;  // 16-byte units per cache row
-  constexpr int TILE = Cfg::kTile, NS = TILE / 8;  // positions and score n-tiles per K/V tile
-  extern __shared__ __align__(128) uint8_t smem[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t4 = lane & 3;
+  constexpr int kSlots = Cfg::kSlots;
+  constexpr int kCopyWarp = 4, kMmaWarp = 5;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  uint64_t* kv_full = reinterpret_cast<uint64_t*>(smem);  // [kSlots] tile landed
+  uint64_t* kv_free = kv_full + kSlots;  // [kSlots] the MMAs that read it have retired
+  uint64_t* s_full = kv_free + kSlots;   // [2] S(j) complete
+  uint64_t* p_full = s_full + 2;         // [2] P(j) written by the four softmax warps
+  uint64_t* q_full = p_full + 2;         // [1] Q in tensor memory
+  uint64_t* o_done = q_full + 1;         // [1] one phase per P V product
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
+  uint8_t* ring = smem + 1024;
+
   const int G = p.G, TQ = kPfRows / G;
   const int qt = blockIdx.x / p.nsplit, split = blockIdx.x % p.nsplit;
   const int kvh = blockIdx.y, b = blockIdx.z;
 
-  __half* qs = reinterpret_cast<__half*>(smem);
-  uint8_t* stage0 = smem + Cfg::kQBytes;
-
+  if (tid == 0) {
+    for (int i = 0; i < kSlots; ++i) {
+      mbar_init(&kv_full[i], 1);
+      mbar_init(&kv_free[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s_full[i], 1);
+      mbar_init(&p_full[i], 4);
+    }
+    mbar_init(q_full, 4);
+    mbar_init(o_done, 1);
+    fence_mbar_init();
+  }
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_slot)), "n"(Cfg::kCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_before_sync();
+  __syncthreads();
+  tc_after_sync();
+  const uint32_t tmem = *tmem_slot;
   pdl_trigger();
   pdl_wait();  // q, the cache rows of this chunk and seqlens come from earlier kernels
 
@@ -118,258 +157,312 @@ __global__ void __launch_bounds__(kPfThreads, D >= 256 ? 1 : 2)
   const int t1 = min(t0 + TQ, p.T) - 1;  // last one
   // positions of the chunk's tokens: token t sits at len - T + t
   const int pos_first = len - p.T + t0, pos_last = len - p.T + t1;
-  int kv_lo = 0;
-  if (p.window > 0) kv_lo = max(0, pos_first - p.window + 1);
-  const int kv_hi = pos_last;  // inclusive
-  const int ntiles_all = kv_hi >= kv_lo ? (kv_hi - kv_lo) / TILE + 1 : 0;
+  const int kv_lo = p.window > 0 ? max(0, pos_first - p.window + 1) : 0;
+  const PfWalk walk(kv_lo, pos_last, p.slots, p.ring);
   // this CTA's share of the tiles
-  const int tps = (ntiles_all + p.nsplit - 1) / p.nsplit;
+  const int tps = (walk.tiles + p.nsplit - 1) / p.nsplit;
   const int j0 = split * tps;
-  const int ntiles = max(0, min(ntiles_all, j0 + tps) - j0);
+  const int ntiles = max(0, min(walk.tiles, j0 + tps) - j0);
+  bool ok = true;
 
-  const __half* kbase = p.k + ((size_t)b * p.Hkv + kvh) * (size_t)p.slots * D;
-  const __half* vbase = p.v + ((size_t)b * p.Hkv + kvh) * (size_t)p.slots * D;
-  auto issue = [&](int j, int st) {
-    uint8_t* ks = stage0 + (size_t)st * 2 * Cfg::kTileBytes;
-    uint8_t* vs = ks + Cfg::kTileBytes;
-    const int p0 = kv_lo + (j0 + j) * TILE;
+  if (warp == kCopyWarp) {
+    // ================= K and V tiles ============================================================
+    const int row0 = (b * p.Hkv + kvh) * p.slots;
+    TcRing<kSlots> r;
+    for (int i = 0; i < 2 * ntiles && ok; ++i, r.advance()) {
+      ok = tc_wait_w(&kv_free[r.i], r.phase ^ 1, p.status);
+      if (!ok) break;
+      if (tc_elect()) {
+        const CUtensorMap* tm = i & 1 ? &p.tmv : &p.tmk;
+        const PfTileAt t = walk.at(j0 + (i >> 1));
+        uint8_t* dst = ring + (size_t)r.i * Cfg::kSlotBytes;
+        mbar_arrive_expect_tx(&kv_full[r.i], Cfg::kSlotBytes);
 #pragma unroll
-    for (int i = 0; i < TILE * CPR / kPfThreads; ++i) {
-      const int u = tid + i * kPfThreads;
-      const int row = u / CPR, cc = u % CPR;
-      const int pos = p0 + row;
-      const bool ok = pos <= kv_hi && pos >= 0;
-      int slot = ok ? pos : 0;
-      if (p.ring) slot %= p.slots;
-      const size_t goff = (size_t)slot * D + cc * 8;
-      const int soff = row * Cfg::kRowBytes + ((cc ^ (row & 7)) << 4);
-      pf_cp16(ks + soff, kbase + goff, ok);
-      pf_cp16(vs + soff, vbase + goff, ok);
+        for (int c = 0; c < D / 64; ++c)
+          asm volatile(
+              "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+              " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst + c * Cfg::kBoxBytes)),
+              "l"(reinterpret_cast<uint64_t>(tm)), "r"(c * 64), "r"(row0 + t.slot), "r"(smem_u32(&kv_full[r.i]))
+              : "memory");
+      }
+      __syncwarp();
     }
-  };
-  if (ntiles > 0) issue(0, 0);
-  pf_commit();
+  } else if (warp == kMmaWarp) {
+    // ================= MMA issue: the whole warp runs the loop, one lane issues =================
+    TcRing<kSlots> r;  // slot of K(j + 1), then of V(j)
+    const uint32_t kdesc0 = tc_desc_lo(smem_u32(ring), 16), vdesc0 = tc_desc_lo(smem_u32(ring), Cfg::kBoxBytes);
+    constexpr uint32_t kSw = 2u << 29;  // 128-byte swizzle
+    auto scores = [&](int j) {
+      ok = ok && tc_wait_w(&kv_full[r.i], r.phase, p.status);
+      if (!ok) return;
+      tc_after_sync();
+      const uint32_t kd = kdesc0 + r.i * (Cfg::kSlotBytes >> 4);
+#pragma unroll
+      for (int m = 0; m < D / 16; ++m)
+        tc_mma_f16_ta_w<tc_desc_hi(1024) | kSw, Cfg::kIdescS>(
+            tmem + Cfg::kS0 + (j & 1) * kPfTile, tmem + Cfg::kQ0 + m * 8,
+            kd + (((m >> 2) * Cfg::kBoxBytes + (m & 3) * 32) >> 4), m > 0 ? 1u : 0u);
+      tc_commit_w(&s_full[j & 1]);
+      tc_commit_w(&kv_free[r.i]);
+    };
+    ok = tc_wait_w(q_full, 0, p.status);
+    // slots go K(0), V(0), K(1), V(1), ...: the score product of tile j + 1 skips over V(j)
+    if (ntiles > 0) scores(0);
+    uint32_t vi = 1, vphase = 0;  // slot of V(j)
+    for (int j = 0; j < ntiles && ok; ++j) {
+      if (j + 1 < ntiles) {
+        r.advance(2);
+        scores(j + 1);
+      }
+      ok = ok && tc_wait_w(&p_full[j & 1], (uint32_t)((j >> 1) & 1), p.status);
+      ok = ok && tc_wait_w(&kv_full[vi], vphase, p.status);
+      if (!ok) break;
+      tc_after_sync();
+      const uint32_t vd = vdesc0 + vi * (Cfg::kSlotBytes >> 4);
+#pragma unroll
+      for (int m = 0; m < kPfTile / 16; ++m)
+        tc_mma_f16_ta_w<tc_desc_hi(1024) | kSw, Cfg::kIdescO>(
+            tmem + Cfg::kO0, tmem + Cfg::kS0 + (j & 1) * kPfTile + m * 8, vd + ((m * 2048) >> 4),
+            (j > 0 || m > 0) ? 1u : 0u);
+      tc_commit_w(&kv_free[vi]);
+      tc_commit_w(o_done);
+      vi += 2;
+      if (vi >= kSlots) {
+        vi -= kSlots;
+        vphase ^= 1;
+      }
+    }
+  } else {
+    // ================= softmax: one thread per row ================================================
+    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
+    const int row = tid;  // 0..127
+    const int t = t0 + row / G, h = kvh * G + row % G;
+    const bool live = t < p.T;
+    const int pos = len - p.T + t;
+    const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+    // ---- Q row, scaled, f16, into tensor memory (rows past T are zero) ---------------------------
+    {
+      const size_t qi = (((size_t)b * p.T + (live ? t : 0)) * p.H + h) * D;
+#pragma unroll 1
+      for (int c = 0; c < D; c += 64) {
+        uint32_t w[32];
+        if (p.q_is_f16) {
+          const __half2* q2 = reinterpret_cast<const __half2*>(static_cast<const __half*>(p.q) + qi + c);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float2 v = __half22float2(q2[i]);
+            w[i] = live ? pf_pack(v.x * p.scale_log2, v.y * p.scale_log2) : 0u;
+          }
+        } else {
+          const float4* q4 = reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + qi + c);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float4 v = q4[i];
+            w[2 * i] = live ? pf_pack(v.x * p.scale_log2, v.y * p.scale_log2) : 0u;
+            w[2 * i + 1] = live ? pf_pack(v.z * p.scale_log2, v.w * p.scale_log2) : 0u;
+          }
+        }
+        HB_TMEM_ST32(lane_base + (uint32_t)(Cfg::kQ0 + c / 2), w);
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(q_full);
+    }
 
-  // Q rows: row r = (token t0 + r / G, head kvh * G + r % G), scaled, f16; rows past T are zero
-  for (int i = tid; i < kPfRows * (D / 4); i += kPfThreads) {
-    const int r = i / (D / 4), d4 = i % (D / 4);
-    const int t = t0 + r / G, h = kvh * G + r % G;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t < p.T) {
-      const size_t qi = (((size_t)b * p.T + t) * p.H + h) * D + 4 * d4;
-      if (p.q_is_f16) {
-        const __half2* hq = reinterpret_cast<const __half2*>(reinterpret_cast<const __half*>(p.q) + qi);
-        const float2 a = __half22float2(hq[0]), c = __half22float2(hq[1]);
-        v = make_float4(a.x, a.y, c.x, c.y);
+    float m = -CUDART_INF_F, l = 0.f;  // reference maximum and sum of the row
+    for (int j = 0; j < ntiles; ++j) {
+      const PfTileAt at = walk.at(j0 + j);
+      if (at.n < kPfTile) {
+        // Rows of V past the run's end are whatever the cache holds there, NaN included, and P = 0
+        // does not silence that: zero them before P(j) releases the product (at most two tiles of
+        // a walk).
+        const int slot = (2 * j + 1) % kSlots;
+        ok = ok && tc_wait_w(&kv_full[slot], (uint32_t)(((2 * j + 1) / kSlots) & 1), p.status);
+        for (int i = tid; i < (kPfTile - at.n) * (D / 8); i += 128) {
+          const int rr = at.n + i / (D / 8), u = i % (D / 8);
+          *reinterpret_cast<uint4*>(ring + (size_t)slot * Cfg::kSlotBytes + (u >> 3) * Cfg::kBoxBytes + rr * 128 +
+                                    ((u & 7) << 4)) = make_uint4(0, 0, 0, 0);
+        }
+        fence_proxy_async();
+      }
+      ok = ok && tc_wait_w(&s_full[j & 1], (uint32_t)((j >> 1) & 1), p.status);
+      tc_after_sync();
+      const uint32_t s_addr = lane_base + (uint32_t)(Cfg::kS0 + (j & 1) * kPfTile);
+      uint32_t v0[32], v1[32];
+      HB_TMEM_LD32(v0, s_addr);
+      HB_TMEM_LD32(v1, s_addr + 32);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      // positions of this tile that the row sees: [a, e)
+      const int a = max(lo - at.pos, 0), e = live ? min(pos - at.pos + 1, at.n) : 0;
+      if (a > 0 || e < kPfTile) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          if (i < a || i >= e) v0[i] = 0xff800000u;  // -inf
+          if (i + 32 < a || i + 32 >= e) v1[i] = 0xff800000u;
+        }
+      }
+      float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+      for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], fmaxf(__uint_as_float(v0[i]), __uint_as_float(v1[i])));
+      const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      const bool grow = mt > m + 8.f;  // also the first visible tile: m = -inf
+      if (j > 0 && __any_sync(0xffffffffu, grow)) {
+        // rescale O once P V(j - 1) has retired; P V(j - 2) has, S(j) was issued behind it
+        ok = ok && tc_wait_w(o_done, (uint32_t)((j - 1) & 1), p.status);
+        tc_after_sync();
+        const float alpha = grow ? pf_exp2(m - mt) : 1.f;  // m = -inf: 0
+#pragma unroll 1
+        for (int c = 0; c < D; c += 32) {
+          uint32_t o[32];
+          HB_TMEM_LD32(o, lane_base + (uint32_t)(Cfg::kO0 + c));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          HB_TMEM_ST32(lane_base + (uint32_t)(Cfg::kO0 + c), o);
+        }
+        l *= alpha;
+      }
+      if (grow) m = mt;
+      const float base = m == -CUDART_INF_F ? 0.f : m;  // nothing visible yet: avoid inf - inf
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t pk[32];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float e0 = pf_exp2(__uint_as_float(v0[2 * i]) - base), e1 = pf_exp2(__uint_as_float(v0[2 * i + 1]) - base);
+        const float e2 = pf_exp2(__uint_as_float(v1[2 * i]) - base), e3 = pf_exp2(__uint_as_float(v1[2 * i + 1]) - base);
+        sum[0] += e0;
+        sum[1] += e1;
+        sum[2] += e2;
+        sum[3] += e3;
+        pk[i] = pf_pack(e0, e1);
+        pk[16 + i] = pf_pack(e2, e3);
+      }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      HB_TMEM_ST32(s_addr, pk);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[j & 1]);
+    }
+
+    // ---- O out of tensor memory, normalised or as a partial; whole rows by bulk copies -----------
+    // the last two products may both be in flight: one phase after the other, a parity alone
+    // does not tell phase n - 1 from n - 3
+    for (int i = max(0, ntiles - 2); i < ntiles; ++i) ok = ok && tc_wait_w(o_done, (uint32_t)(i & 1), p.status);
+    tc_after_sync();
+    const float f = p.nsplit > 1 ? 1.f : (l > 0.f ? 1.f / l : 0.f);
+    // the K/V ring is idle now: every product has retired
+    float* orow = reinterpret_cast<float*>(ring + (size_t)row * Cfg::kOutStride);
+#pragma unroll 1
+    for (int c = 0; c < D; c += 32) {
+      uint32_t o[32];
+      if (ntiles > 0) {
+        HB_TMEM_LD32(o, lane_base + (uint32_t)(Cfg::kO0 + c));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       } else {
-        v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.q) + qi);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = 0u;
       }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<float4*>(orow + c + 4 * i) =
+            make_float4(__uint_as_float(o[4 * i]) * f, __uint_as_float(o[4 * i + 1]) * f,
+                        __uint_as_float(o[4 * i + 2]) * f, __uint_as_float(o[4 * i + 3]) * f);
     }
-    uint2 w;
-    w.x = pf_pack(v.x * p.scale_log2, v.y * p.scale_log2);
-    w.y = pf_pack(v.z * p.scale_log2, v.w * p.scale_log2);
-    *reinterpret_cast<uint2*>(qs + r * Cfg::kQStride + 4 * d4) = w;
+    fence_proxy_async();
+    if (live) {
+      const size_t ri = ((size_t)b * p.T + t) * p.H + h;
+      float* dst = p.nsplit > 1 ? p.part_o + (ri * p.nsplit + split) * D : p.out + ri * D;
+      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(orow)),
+                   "n"(D * 4)
+                   : "memory");
+      if (p.nsplit > 1)
+        *reinterpret_cast<float2*>(p.part_ml + (ri * p.nsplit + split) * 2) = make_float2(m, l);
+    }
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
+  tc_before_sync();
   __syncthreads();
-
-  // this lane's two rows (g and g + 8 of the warp's 16) and what they may see
-  const int rA = 16 * warp + g, rB = rA + 8;
-  const int tA = t0 + rA / G, tB = t0 + rB / G;
-  const int posA = len - p.T + tA, posB = len - p.T + tB;
-  const int loA = p.window > 0 ? max(0, posA - p.window + 1) : 0;
-  const int loB = p.window > 0 ? max(0, posB - p.window + 1) : 0;
-  const bool liveA = tA < p.T, liveB = tB < p.T;
-
-  float mA = -CUDART_INF_F, mB = -CUDART_INF_F, lA = 0.f, lB = 0.f;
-  float o[NO][4];
-#pragma unroll
-  for (int n = 0; n < NO; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-
-  for (int j = 0; j < ntiles; ++j) {
-    if (j + 1 < ntiles) issue(j + 1, (j + 1) & 1);
-    pf_commit();
-    pf_wait<1>();
-    __syncthreads();  // tile j is in shared memory for every warp
-    const uint8_t* ks = stage0 + (size_t)(j & 1) * 2 * Cfg::kTileBytes;
-    const uint8_t* vs = ks + Cfg::kTileBytes;
-    const int p0 = kv_lo + (j0 + j) * TILE;
-
-    // ---- S = Q K^T: 16 rows x TILE positions per warp -------------------------------------
-    float s[NS][4];
-#pragma unroll
-    for (int n = 0; n < NS; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
-#pragma unroll
-    for (int kk = 0; kk < KS; ++kk) {
-      uint32_t a[4];
-      {
-        // A fragment of Q: matrices (rows 0-7 | 8-15) x (k 0-7 | 8-15) of this warp's 16 rows
-        const int row = 16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8;
-        const int col = 16 * kk + (lane >> 4) * 8;
-        pf_ldsm(a, qs + row * Cfg::kQStride + col);
-      }
-#pragma unroll
-      for (int np = 0; np < NS / 2; ++np) {  // two n-tiles (16 positions) per ldmatrix
-        uint32_t kb[4];
-        // matrices: (pos 0-7, d 0-7), (pos 0-7, d 8-15), (pos 8-15, d 0-7), (pos 8-15, d 8-15)
-        const int row = 16 * np + (lane & 7) + (lane >> 4) * 8;
-        const int cc = 2 * kk + ((lane >> 3) & 1);
-        pf_ldsm(kb, ks + row * Cfg::kRowBytes + ((cc ^ (row & 7)) << 4));
-        pf_mma(s[2 * np], a, kb[0], kb[1]);
-        pf_mma(s[2 * np + 1], a, kb[2], kb[3]);
-      }
-    }
-
-    // ---- mask, online softmax (exp2 domain) ----------------------------------------------
-    float mxA = -CUDART_INF_F, mxB = -CUDART_INF_F;
-#pragma unroll
-    for (int n = 0; n < NS; ++n) {
-      const int pc = p0 + 8 * n + 2 * t4;
-      const bool a0 = liveA && pc >= loA && pc <= posA, a1 = liveA && pc + 1 >= loA && pc + 1 <= posA;
-      const bool b0 = liveB && pc >= loB && pc <= posB, b1 = liveB && pc + 1 >= loB && pc + 1 <= posB;
-      s[n][0] = a0 ? s[n][0] : -CUDART_INF_F;
-      s[n][1] = a1 ? s[n][1] : -CUDART_INF_F;
-      s[n][2] = b0 ? s[n][2] : -CUDART_INF_F;
-      s[n][3] = b1 ? s[n][3] : -CUDART_INF_F;
-      mxA = fmaxf(mxA, fmaxf(s[n][0], s[n][1]));
-      mxB = fmaxf(mxB, fmaxf(s[n][2], s[n][3]));
-    }
-    mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 1));
-    mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 2));
-    mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 1));
-    mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 2));
-    const float mnA = fmaxf(mA, mxA), mnB = fmaxf(mB, mxB);
-    const float baseA = mnA == -CUDART_INF_F ? 0.f : mnA;  // nothing visible yet: avoid inf - inf
-    const float baseB = mnB == -CUDART_INF_F ? 0.f : mnB;
-    const float alA = exp2f(mA - baseA), alB = exp2f(mB - baseB);
-    float sumA = 0.f, sumB = 0.f;
-    uint32_t pa[NS / 2][4];  // P as A fragments of the second product: k-steps of 16 positions
-#pragma unroll
-    for (int n = 0; n < NS; ++n) {
-      const float e0 = exp2f(s[n][0] - baseA), e1 = exp2f(s[n][1] - baseA);
-      const float e2 = exp2f(s[n][2] - baseB), e3 = exp2f(s[n][3] - baseB);
-      sumA += e0 + e1;
-      sumB += e2 + e3;
-      pa[n >> 1][(n & 1) * 2] = pf_pack(e0, e1);      // rows g
-      pa[n >> 1][(n & 1) * 2 + 1] = pf_pack(e2, e3);  // rows g + 8
-    }
-    sumA += __shfl_xor_sync(0xffffffffu, sumA, 1);
-    sumA += __shfl_xor_sync(0xffffffffu, sumA, 2);
-    sumB += __shfl_xor_sync(0xffffffffu, sumB, 1);
-    sumB += __shfl_xor_sync(0xffffffffu, sumB, 2);
-    lA = lA * alA + sumA;
-    lB = lB * alB + sumB;
-    mA = mnA;
-    mB = mnB;
-#pragma unroll
-    for (int n = 0; n < NO; ++n) {
-      o[n][0] *= alA;
-      o[n][1] *= alA;
-      o[n][2] *= alB;
-      o[n][3] *= alB;
-    }
-
-    // ---- O += P V ---------------------------------------------------------------------------
-#pragma unroll
-    for (int kk = 0; kk < NS / 2; ++kk) {  // 16 positions per step
-#pragma unroll
-      for (int np = 0; np < NO / 2; ++np) {  // two n-tiles (16 dims) per ldmatrix
-        uint32_t vb[4];
-        // transposed matrices: (pos 0-7 | 8-15) x (d 0-7 | 8-15) of this step
-        const int row = 16 * kk + (lane & 7) + ((lane >> 3) & 1) * 8;
-        const int cc = 2 * np + (lane >> 4);
-        pf_ldsm_t(vb, vs + row * Cfg::kRowBytes + ((cc ^ (row & 7)) << 4));
-        pf_mma(o[2 * np], pa[kk], vb[0], vb[1]);
-        pf_mma(o[2 * np + 1], pa[kk], vb[2], vb[3]);
-      }
-    }
-    __syncthreads();  // every warp is done with stage j & 1 before it is refilled
-  }
-
-  // ---- normalise and store, or hand the partial to the merge kernel ------------------------
-  if (p.nsplit == 1) {
-    const float invA = lA > 0.f ? 1.f / lA : 0.f, invB = lB > 0.f ? 1.f / lB : 0.f;
-    if (liveA) {
-      float* dst = p.out + (((size_t)b * p.T + tA) * p.H + kvh * G + rA % G) * D;
-#pragma unroll
-      for (int n = 0; n < NO; ++n)
-        *reinterpret_cast<float2*>(dst + 8 * n + 2 * t4) = make_float2(o[n][0] * invA, o[n][1] * invA);
-    }
-    if (liveB) {
-      float* dst = p.out + (((size_t)b * p.T + tB) * p.H + kvh * G + rB % G) * D;
-#pragma unroll
-      for (int n = 0; n < NO; ++n)
-        *reinterpret_cast<float2*>(dst + 8 * n + 2 * t4) = make_float2(o[n][2] * invB, o[n][3] * invB);
-    }
-    return;
-  }
-  if (liveA) {
-    const size_t pi = ((((size_t)b * p.T + tA) * p.H + kvh * G + rA % G) * p.nsplit + split);
-    float* dst = p.part_o + pi * D;
-#pragma unroll
-    for (int n = 0; n < NO; ++n)
-      *reinterpret_cast<float2*>(dst + 8 * n + 2 * t4) = make_float2(o[n][0], o[n][1]);
-    if (t4 == 0) *reinterpret_cast<float2*>(p.part_ml + pi * 2) = make_float2(mA, lA);
-  }
-  if (liveB) {
-    const size_t pi = ((((size_t)b * p.T + tB) * p.H + kvh * G + rB % G) * p.nsplit + split);
-    float* dst = p.part_o + pi * D;
-#pragma unroll
-    for (int n = 0; n < NO; ++n)
-      *reinterpret_cast<float2*>(dst + 8 * n + 2 * t4) = make_float2(o[n][2], o[n][3]);
-    if (t4 == 0) *reinterpret_cast<float2*>(p.part_ml + pi * 2) = make_float2(mB, lB);
-  }
+  if (warp == kMmaWarp)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(Cfg::kCols));
 }
 
-// out = sum_s 2^(m_s - m*) O_s / sum_s 2^(m_s - m*) l_s over the splits of one (token, head).
-__global__ void __launch_bounds__(128) attn_prefill_merge_kernel(const float* part_o,
-                                                                 const float* part_ml, int nsplit,
-                                                                 int D, float* out) {
+// out = sum_s 2^(m_s - m*) O_s / sum_s 2^(m_s - m*) l_s over the splits of one (token, head): a
+// warp per row, lane s holding split s's weight.
+template <int D>
+__global__ void __launch_bounds__(256) attn_prefill_merge_kernel(const float* part_o, const float* part_ml,
+                                                                 int nsplit, long rows, float* out) {
   pdl_trigger();
   pdl_wait();
-  const size_t row = blockIdx.x;  // (sequence, token, head)
-  const float* ml = part_ml + row * nsplit * 2;
-  float mstar = -CUDART_INF_F;
-  for (int s2 = 0; s2 < nsplit; ++s2) mstar = fmaxf(mstar, __ldcg(ml + 2 * s2));
-  float lsum = 0.f;
-  if (mstar != -CUDART_INF_F)
-    for (int s2 = 0; s2 < nsplit; ++s2) lsum += exp2f(__ldcg(ml + 2 * s2) - mstar) * __ldcg(ml + 2 * s2 + 1);
+  constexpr int V = D / 32;  // floats per lane
+  const int lane = threadIdx.x & 31;
+  const long row = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  float2 ml = make_float2(-CUDART_INF_F, 0.f);
+  if (lane < nsplit) ml = __ldcg(reinterpret_cast<const float2*>(part_ml + row * nsplit * 2) + lane);
+  const float mstar = warp_max(ml.x);
+  const float w = ml.x == -CUDART_INF_F ? 0.f : exp2f(ml.x - mstar);
+  const float lsum = warp_sum(w * ml.y);
   const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float acc = 0.f;
-    if (mstar != -CUDART_INF_F)
-      for (int s2 = 0; s2 < nsplit; ++s2)
-        acc += exp2f(__ldcg(ml + 2 * s2) - mstar) * __ldcg(part_o + (row * nsplit + s2) * D + d);
-    out[row * D + d] = acc * inv;
+  float acc[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) acc[i] = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < nsplit; ++s) {
+    const float ws = __shfl_sync(0xffffffffu, w, s);
+    const float2* src = reinterpret_cast<const float2*>(part_o + (row * nsplit + s) * D) + lane;
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) {
+      const float2 x = __ldcg(src + 32 * i);
+      acc[2 * i] += ws * x.x;
+      acc[2 * i + 1] += ws * x.y;
+    }
   }
+  float2* dst = reinterpret_cast<float2*>(out + row * D) + lane;
+#pragma unroll
+  for (int i = 0; i < V / 2; ++i) dst[32 * i] = make_float2(acc[2 * i] * inv, acc[2 * i + 1] * inv);
 }
 
 }  // namespace hb
 
 using namespace hb;
 
-// How many CTAs share the K/V range of a query tile: 1 when the query tiles alone fill the SMs,
-// else enough to, but no split shorter than 4 tiles of the longest range a tile can see and
-// at most 8.  A function of the shapes only (the workspace is sized with it).
-static int pf_pick_splits(const hb200_ctx* ctx, int nseq, int T, int H, int Hkv, int D, int slots,
-                          int window) {
+// How many CTAs share the K/V range of a query tile: as many as there are SMs for in one wave,
+// but no split shorter than 4 tiles of the longest range a tile can see.  A function of the
+// shapes only (the workspace is sized with it).
+static int pf_pick_splits(const hb200_ctx* ctx, int nseq, int T, int H, int Hkv, int slots, int window) {
   const int G = H / Hkv, TQ = kPfRows / G;
   const long ctas = (long)((T + TQ - 1) / TQ) * Hkv * nseq;
-  if (ctas >= ctx->sm_count) return 1;
-  const int tile = D >= 256 ? 32 : 64;
   long span = slots;
   if (window > 0 && (long)window + T < span) span = (long)window + T;
-  const int tiles_max = (int)((span + tile - 1) / tile);
-  int ns = (int)((ctx->sm_count + ctas - 1) / ctas);
-  if (ns > 8) ns = 8;
-  if (ns > tiles_max / 4) ns = tiles_max / 4;
-  return ns < 1 ? 1 : ns;
+  long ns = ctx->sm_count / ctas;
+  const long most = (span + kPfTile - 1) / kPfTile / 4;
+  if (ns > most) ns = most;
+  if (ns > kPfMaxSplits) ns = kPfMaxSplits;
+  return ns < 1 ? 1 : (int)ns;
 }
 
 size_t hb_attn_prefill_tiled_ws(const hb200_ctx* ctx, int nseq, int T, int H, int Hkv, int D,
                                 int slots) {
-  if (H % Hkv) return 0;
-  const int ns = pf_pick_splits(ctx, nseq, T, H, Hkv, D, slots, 0);
+  if (H % Hkv || H / Hkv > 8) return 0;
+  const int ns = pf_pick_splits(ctx, nseq, T, H, Hkv, slots, 0);
   return ns > 1 ? (size_t)nseq * T * H * ns * ((size_t)D + 2) * sizeof(float) + 256 : 0;
+}
+
+template <int D>
+static int pf_launch(hb200_ctx* ctx, const PfParams& p, dim3 grid, cudaStream_t st) {
+  const int rc = hb_func_smem(ctx, reinterpret_cast<const void*>(attn_prefill_tiled_kernel<D>), PfCfg<D>::kSmem);
+  if (rc) return rc;
+  HB_CUDA(launch_pdl(attn_prefill_tiled_kernel<D>, grid, dim3(kPfThreads), (size_t)PfCfg<D>::kSmem, st,
+                     ctx->pdl, p));
+  if (p.nsplit > 1) {
+    const long rows = (long)p.nseq * p.T * p.H;
+    HB_CUDA(launch_pdl(attn_prefill_merge_kernel<D>, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, st,
+                       ctx->pdl, (const float*)p.part_o, (const float*)p.part_ml, p.nsplit, rows, p.out));
+  }
+  return HB200_OK;
 }
 
 // Causal attention of T query tokens per sequence on the tiled kernel.  HB200_OK when the
@@ -382,13 +475,24 @@ int hb_attn_prefill_tiled(hb200_ctx* ctx, const void* d_q, int q_is_f16, const v
   const int G = H / Hkv;
   if (!(G == 1 || G == 2 || G == 4 || G == 8)) return 1;
   if (!(D == 64 || D == 128 || D == 256)) return 1;
-  if (nseq > 65535 || Hkv > 65535) return 1;
+  if (nseq > 65535 || Hkv > 65535 || (long)nseq * Hkv * slots >= (1l << 31)) return 1;
   if (q_is_f16 ? (reinterpret_cast<uintptr_t>(d_q) & 3) : (reinterpret_cast<uintptr_t>(d_q) & 15)) return 1;
-  if (reinterpret_cast<uintptr_t>(d_out) & 7) return 1;
+  if (reinterpret_cast<uintptr_t>(d_out) & 15) return 1;  // rows leave by bulk copies
+  TcEncodeTiledFn encode = tc_tensor_map_encoder();
+  if (encode == nullptr) return 1;
   PfParams p = {};
+  const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)nseq * Hkv * slots};
+  const cuuint64_t strides[1] = {(cuuint64_t)D * 2};
+  const cuuint32_t box[2] = {64, kPfTile};
+  const cuuint32_t estr[2] = {1, 1};
+  for (int i = 0; i < 2; ++i) {
+    const CUresult rc = encode(i ? &p.tmv : &p.tmk, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
+                               const_cast<void*>(i ? d_v : d_k), dims, strides, box, estr,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    HB_REQUIRE(rc == CUDA_SUCCESS, "attn (prefill): cuTensorMapEncodeTiled failed (%d)", (int)rc);
+  }
   p.q = d_q;
-  p.k = static_cast<const __half*>(d_k);
-  p.v = static_cast<const __half*>(d_v);
   p.seqlens = d_seqlens;
   p.out = d_out;
   p.q_is_f16 = q_is_f16;
@@ -401,43 +505,23 @@ int hb_attn_prefill_tiled(hb200_ctx* ctx, const void* d_q, int q_is_f16, const v
   p.window = window;
   p.ring = ring;
   p.scale_log2 = scale * 1.4426950408889634f;
+  p.status = ctx->d_status;
   const int TQ = kPfRows / G;
-  p.nsplit = pf_pick_splits(ctx, nseq, T, H, Hkv, D, slots, window);
+  p.nsplit = pf_pick_splits(ctx, nseq, T, H, Hkv, slots, window);
   if (p.nsplit > 1) {
-    const size_t po = (size_t)nseq * T * H * p.nsplit * (size_t)D * sizeof(float);
-    const size_t need = po + (size_t)nseq * T * H * p.nsplit * 2 * sizeof(float);
-    if (d_ws == nullptr || ws_bytes < need || (reinterpret_cast<uintptr_t>(d_ws) & 15)) {
-      p.nsplit = 1;  // a caller's workspace sized by an older rule: one CTA per query tile
-    } else {
-      p.part_o = static_cast<float*>(d_ws);
-      p.part_ml = reinterpret_cast<float*>(static_cast<uint8_t*>(d_ws) + po);
-    }
+    // never more than the workspace holds (a caller may have sized it for another T)
+    const size_t per = (size_t)nseq * T * H * ((size_t)D + 2) * sizeof(float);
+    if (d_ws == nullptr || (reinterpret_cast<uintptr_t>(d_ws) & 15)) p.nsplit = 1;
+    else if ((size_t)p.nsplit * per > ws_bytes) p.nsplit = ws_bytes / per < 1 ? 1 : (int)(ws_bytes / per);
+  }
+  if (p.nsplit > 1) {
+    p.part_o = static_cast<float*>(d_ws);
+    p.part_ml = p.part_o + (size_t)nseq * T * H * p.nsplit * (size_t)D;
   }
   const dim3 grid((unsigned)((T + TQ - 1) / TQ) * p.nsplit, (unsigned)Hkv, (unsigned)nseq);
-  int rc;
   switch (D) {
-    case 64:
-      rc = hb_func_smem(ctx, reinterpret_cast<const void*>(attn_prefill_tiled_kernel<64>), PfCfg<64>::kSmem);
-      if (rc) return rc;
-      HB_CUDA(launch_pdl(attn_prefill_tiled_kernel<64>, grid, dim3(kPfThreads), (size_t)PfCfg<64>::kSmem,
-                         st, ctx->pdl, p));
-      break;
-    case 128:
-      rc = hb_func_smem(ctx, reinterpret_cast<const void*>(attn_prefill_tiled_kernel<128>), PfCfg<128>::kSmem);
-      if (rc) return rc;
-      HB_CUDA(launch_pdl(attn_prefill_tiled_kernel<128>, grid, dim3(kPfThreads),
-                         (size_t)PfCfg<128>::kSmem, st, ctx->pdl, p));
-      break;
-    default:
-      rc = hb_func_smem(ctx, reinterpret_cast<const void*>(attn_prefill_tiled_kernel<256>), PfCfg<256>::kSmem);
-      if (rc) return rc;
-      HB_CUDA(launch_pdl(attn_prefill_tiled_kernel<256>, grid, dim3(kPfThreads),
-                         (size_t)PfCfg<256>::kSmem, st, ctx->pdl, p));
-      break;
+    case 64: return pf_launch<64>(ctx, p, grid, st);
+    case 128: return pf_launch<128>(ctx, p, grid, st);
+    default: return pf_launch<256>(ctx, p, grid, st);
   }
-  if (p.nsplit > 1)
-    HB_CUDA(launch_pdl(attn_prefill_merge_kernel, dim3((unsigned)((size_t)nseq * T * H)), dim3(128), 0,
-                       st, ctx->pdl, (const float*)p.part_o, (const float*)p.part_ml, p.nsplit, D,
-                       d_out));
-  return HB200_OK;
 }

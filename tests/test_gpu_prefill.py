@@ -114,6 +114,35 @@ def test_ring_cache_prefill_matches_oracle(ctx, oracle, H, Hkv, D, slots, T, len
     assert np.linalg.norm(out - ref) / np.linalg.norm(ref) <= TOL
 
 
+@pytest.mark.parametrize("H,Hkv,D,slots,T,lens", [
+    (8, 1, 64, 200, 19, [193, 64]),    # a last tile of one position; an exactly full tile
+    (8, 2, 128, 333, 65, [333, 66]),   # query tiles of one row; the cache full to its last slot
+    (4, 4, 256, 640, 9, [577, 9]),     # splits, a tile of one position at the end of the last
+])
+def test_prefill_rescales_and_ignores_stale_rows(ctx, oracle, H, Hkv, D, slots, T, lens):
+    """Scores that grow along the sequence (the row maximum moves by far more than the 2^8 below
+    which O is not rescaled) and NaN in every cache row past a sequence's length: TMA brings
+    whole tiles, so stale rows reach shared memory and must not reach the result."""
+    B, scale = len(lens), float(1.0 / np.sqrt(D))
+    rng = np.random.default_rng(D)
+    q = rng.standard_normal((B, T, H, D)).astype(np.float32)
+    ramp = np.linspace(0.0, 8.0, slots)[None, None, :, None]
+    k16 = (rng.standard_normal((B, Hkv, slots, D)) * (0.2 + ramp)).astype(np.float16)
+    v16 = rng.standard_normal((B, Hkv, slots, D)).astype(np.float16)
+    kd, vd = k16.copy(), v16.copy()
+    for b, n in enumerate(lens):
+        kd[b, :, n:], vd[b, :, n:] = np.nan, np.nan
+    sl = np.asarray(lens, np.int32)
+    out = flash_attention_prefill(ctx, _dev(q), _dev(kd), _dev(vd), _dev(sl), num_heads=H,
+                                  num_kv_heads=Hkv, head_dim=D, max_seq_len=slots,
+                                  scale=scale).cpu().numpy()
+    ctx.check()
+    ref = _reference(oracle.attn_decode, q, k16, v16, sl, T, H, Hkv, D, slots, scale, 0)
+    # f16 rounding of the scaled query (2^-11) in scores of magnitude up to 8 * 4 * log2(e) moves
+    # a weight by up to 2^-11 * 46 * ln 2 = 1.6e-2 of itself; averaged over a row's weights 1e-2
+    assert np.abs(out - ref).max() / np.abs(ref).max() <= 1e-2
+
+
 def test_prefill_kv_writer_equals_single_token_calls(ctx):
     lib = _lib.load()
     B, T, H, Hkv, D, slots, base = 2, 7, 8, 2, 64, 40, 500000.0
