@@ -20,13 +20,13 @@
 //     160 tiles of a 10240-row gate/up pair so take 11 super-block times on 148 SMs instead of
 //     20, the 20 tiles of a 2560-row down projection 6 instead of 40.
 // Warps with fixed roles:
-//   16 or 24   dequantise, in groups of 8 that take the steps of 128 weights in turn; a thread owns
-//              one row and 64 weights of a step and stores them with tcgen05.st.  The first 16
-//              also run the epilogue of a finished tile, after they have refilled the A stages
-//              for the next one;
-//   one        weights: 2-D tensor-map TMA boxes of 64 rows x 256 weights, a ring of 2 to 7 tiles;
-//   one        activations: bulk copies of the step's tiles (f16, operand layout written by the
-//              staging kernel);
+//   16 or 24   dequantise, in groups of 8 that take the A stages in turn; a thread owns one row and
+//              64 weights of every 128 and stores them with tcgen05.st.  The first 16 also run
+//              the epilogue of a finished tile, after they have refilled the A stages for the
+//              next one;
+//   one        weights: 2-D tensor-map TMA boxes of 64 rows x 256 weights, a ring of 2 to 6 tiles;
+//   one        activations: bulk copies of a super-block's tiles (f16, operand layout written by
+//              the staging kernel);
 //   one        an elected thread issues the MMAs (M=128, N=NT tokens, K=16).
 // A gate/up pair is one launch: a tile holds 64 gate rows and the 64 up rows of the same outputs,
 // dealt to the tensor-memory lanes so that a gate lane's up value sits 16 lanes further in the
@@ -39,8 +39,6 @@
 namespace hb {
 
 constexpr int kQmRows = 128;          // weight rows per tile = MMA M
-constexpr int kQmStepK = 128;         // weights per pipeline step (half a super-block)
-constexpr int kQmACols = kQmStepK / 2;  // 64 TMEM columns of f16 pairs per stage
 constexpr int kQmMaxSeg = 4;          // tensors one launch multiplies by the same activations
 
 // NT tokens per pass = MMA N; a unit is the bytes of 256 weights (one Q4_K super-block, eight
@@ -53,25 +51,27 @@ struct QmCfg {
   static constexpr uint32_t kIdesc =
       (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kQmRows >> 4) << 24);
   static constexpr bool kSums = FMT == 12;                  // sub-block sums as extra K columns
-  static constexpr int kAccBufs = NT <= 128 ? 2 : 1;        // accumulators in tensor memory
-  static constexpr int kA0 = kAccBufs * NT;                 // first TMEM column of the A stages
-  static constexpr int kAStages = NT == 64 ? 5 : 3;
-  static constexpr int kE0 = kA0 + kAStages * kQmACols;     // TMEM columns of the min residues:
+  // A stages in tensor memory (two weights per column) hold a whole super-block, or half of one
+  // where a 256-token accumulator leaves no room: a stage costs its warps two barriers, a fence
+  // and the wait for their stores, ~400 cycles whatever it holds
+  static constexpr int kAParts = NT == 256 ? 2 : 1;         // stages per super-block
+  static constexpr int kACols = 128 / kAParts;
+  static constexpr int kAStages = NT == 128 ? 2 : 3;
+  static constexpr int kA0 = NT;                            // after the accumulator
+  static constexpr int kE0 = kA0 + kAStages * kACols;       // columns of the min residues:
   static constexpr int kESlots = kSums ? 8 : 0;             //   8 per super-block
   // staged bytes of a super-block: four blocks of [NT rows][64 f16], then [NT rows][16 f16]
   static constexpr int kSumBytes = kSums ? NT * 32 : 0;
   static constexpr int kSbBytes = NT * 512 + kSumBytes;
-  // activation stages: a whole step, or half of one at 256 tokens (64 KB per step); the last of a
-  // super-block brings the sums along
-  static constexpr int kBPer = NT == 256 ? 2 : 1;
-  static constexpr int kBStep = NT * kQmStepK * 2 / kBPer;  // 16 / 32 / 32 KB
-  static constexpr int kBBytes = kBStep + kSumBytes;
-  static constexpr int kBStages = NT == 64 ? 5 : (NT == 128 ? 3 : 4);
-  static constexpr int kPkStages = FMT == 12 ? (NT == 64 ? 7 : (NT == 128 ? 6 : 3)) : (NT == 256 ? 2 : 3);
-  // dequantising warps, in groups of 8 that take the steps in turn: a step is a chain of ~1000
-  // cycles (barrier, shared memory, conversion, store) of which a warp issues 150, so below
-  // 256 tokens, where the dequantiser is the bound, six warps per scheduler beat four
-  static constexpr int kGroups = NT == 256 ? 2 : 3;
+  // activation stages: a super-block, or a quarter of one at 256 tokens; the last brings the sums
+  static constexpr int kBParts = NT == 256 ? 4 : 1;
+  static constexpr int kBPart = NT * 512 / kBParts;         // 32 / 64 / 32 KB
+  static constexpr int kBBytes = kBPart + kSumBytes;
+  static constexpr int kBStages = NT == 64 ? 3 : (NT == 128 ? 2 : 4);
+  static constexpr int kPkStages = FMT == 12 ? (NT == 64 ? 6 : (NT == 128 ? 4 : 3)) : (NT == 64 ? 3 : 2);
+  // dequantising warps, in groups of 8 that take the stages in turn: filling one is a chain of
+  // 1000 to 2000 cycles of which a warp issues a fifth
+  static constexpr int kGroups = NT == 64 ? 3 : 2;
   static constexpr int kExpWarps = 8 * kGroups;
   static constexpr int kThreads = (kExpWarps + 3) * 32;
   static constexpr int kSmem = 2048 + kPkStages * kPkBytes + kBStages * kBBytes;
@@ -315,8 +315,9 @@ template <int NT, int FMT>
 __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(const __grid_constant__ QmParams p) {
   using Cfg = QmCfg<NT, FMT>;
   constexpr int kPkStages = Cfg::kPkStages, kPkBytes = Cfg::kPkBytes, kUnit = Cfg::kUnit;
-  constexpr int kAStages = Cfg::kAStages, kBStages = Cfg::kBStages, kBBytes = Cfg::kBBytes;
-  constexpr int kBPer = Cfg::kBPer, kA0 = Cfg::kA0, kAccBufs = Cfg::kAccBufs, kGroups = Cfg::kGroups;
+  constexpr int kAStages = Cfg::kAStages, kAParts = Cfg::kAParts, kACols = Cfg::kACols, kA0 = Cfg::kA0;
+  constexpr int kBStages = Cfg::kBStages, kBParts = Cfg::kBParts, kBBytes = Cfg::kBBytes;
+  constexpr int kGroups = Cfg::kGroups;
   // a box dimension holds at most 256 elements: the 272-byte Q8_0 unit is mapped as 68 words
   constexpr int kBoxX = FMT == 12 ? 144 : 68;
   constexpr int kEpiWarps = 16;
@@ -327,13 +328,13 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
 
   uint64_t* pk_full = reinterpret_cast<uint64_t*>(smem);  // [kPkStages] two boxes landed
   uint64_t* pk_free = pk_full + kPkStages;                // [kPkStages] every expander warp left it
-  uint64_t* a_full = pk_free + kPkStages;    // [kAStages] stored by the step's 8 warps
+  uint64_t* a_full = pk_free + kPkStages;    // [kAStages] stored by a group's 8 warps
   uint64_t* a_free = a_full + kAStages;      // [kAStages] the MMAs that read it have retired
   uint64_t* b_full = a_free + kAStages;      // [kBStages] activations landed
   uint64_t* b_free = b_full + kBStages;      // [kBStages]
-  uint64_t* acc_full = b_free + kBStages;    // [kAccBufs] a tile's products are complete
-  uint64_t* acc_free = acc_full + kAccBufs;  // [kAccBufs] the epilogue has read them
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + kAccBufs);
+  uint64_t* acc_full = b_free + kBStages;    // a tile's products are complete
+  uint64_t* acc_free = acc_full + 1;         // the epilogue has read them
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
   float* rs_s = reinterpret_cast<float*>(smem + 1024);  // [NT] row scales
   uint8_t* pk = smem + 2048;
   uint8_t* bstg = pk + kPkStages * kPkBytes;
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
   if (tid == 0) {
     for (int i = 0; i < kPkStages; ++i) {
       mbar_init(&pk_full[i], 1);
-      mbar_init(&pk_free[i], 16);  // two steps of 8 warps
+      mbar_init(&pk_free[i], 8 * kAParts);
     }
     for (int i = 0; i < kAStages; ++i) {
       mbar_init(&a_full[i], 8);
@@ -351,10 +352,8 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
       mbar_init(&b_full[i], 1);
       mbar_init(&b_free[i], 1);
     }
-    for (int i = 0; i < kAccBufs; ++i) {
-      mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_free[i], kEpiWarps);
-    }
+    mbar_init(acc_full, 1);
+    mbar_init(acc_free, kEpiWarps);
     fence_mbar_init();
   }
   if (warp == kMmaWarp) {
@@ -410,8 +409,8 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
       const uint8_t* src = p.xb + (size_t)job.b0 * Cfg::kSbBytes;
       for (int s = 0; s < job.n && ok; ++s) {
 #pragma unroll
-        for (int h = 0; h < 2 * kBPer; ++h, r.advance()) {
-          const uint32_t bytes = h == 2 * kBPer - 1 ? kBBytes : Cfg::kBStep;
+        for (int h = 0; h < kBParts; ++h, r.advance()) {
+          const uint32_t bytes = h == kBParts - 1 ? kBBytes : Cfg::kBPart;
           ok = tc_wait_w(&b_free[r.i], r.phase ^ 1, p.status);
           if (!ok) break;
           if (tc_elect()) {
@@ -425,41 +424,44 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
     }
   } else if (warp == kMmaWarp) {
     // ================= MMA issue: the whole warp runs the loop, one lane issues =================
+    // Nothing in the loop's control flow depends on a wait's outcome: ring positions stay provably
+    // uniform, so the addresses are computed in the uniform datapath instead of being moved there
+    // for every MMA (the warp shares its scheduler with six busy ones).  After an expired wait
+    // the products run on whatever is there; the status word says so.
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      if (!mbar_try_wait(bar, parity) && ok) ok = tc_wait_slow(smem_u32(bar), parity, p.status);
+    };
     TcRing<kAStages> ra;
     TcRing<kBStages> rb;
-    TcRing<kAccBufs> rd;
-    uint32_t eslot = 0;
+    uint32_t eslot = 0, dphase = 0;
     const uint32_t b0 = tc_desc_lo(smem_u32(bstg), 128);
-    for (int j = 0; j < njobs && ok; ++j, rd.advance()) {
+    for (int j = 0; j < njobs; ++j, dphase ^= 1) {
       const int nu = qm_job(p.deal, j).n;
-      const uint32_t tmem_d = tmem + rd.i * NT;
-      ok = tc_wait_w(&acc_free[rd.i], rd.phase ^ 1, p.status);
-      if (!ok) break;
+      wait(acc_free, dphase ^ 1);
       uint32_t accum = 0;
-      for (int u = 0; u < nu && ok; ++u) {
+      for (int u = 0; u < nu; ++u) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half, ra.advance()) {
-          ok = tc_wait_w(&a_full[ra.i], ra.phase, p.status);
-          if (!ok) break;
-          const uint32_t a_t = tmem + kA0 + ra.i * kQmACols;
+        for (int ap = 0; ap < kAParts; ++ap, ra.advance()) {
+          wait(&a_full[ra.i], ra.phase);
+          const uint32_t a_t = tmem + kA0 + ra.i * kACols;
+          constexpr int kPer = kBParts / kAParts;
 #pragma unroll
-          for (int hh = 0; hh < kBPer; ++hh, rb.advance()) {
-            ok = tc_wait_w(&b_full[rb.i], rb.phase, p.status);
-            if (!ok) break;
+          for (int bp = 0; bp < kPer; ++bp, rb.advance()) {
+            wait(&b_full[rb.i], rb.phase);
             tc_after_sync();
             const uint32_t bdesc = b0 + rb.i * (kBBytes >> 4);
-            constexpr int kMma = kQmStepK / 16 / kBPer;  // K = 16 per instruction: 8 columns of A
+            constexpr int kMma = 16 / kBParts;  // K = 16 per instruction: 8 columns of A
 #pragma unroll
             for (int m = 0; m < kMma; ++m) {
               tc_mma_f16_ta_w<tc_desc_hi(1024), Cfg::kIdesc>(
-                  tmem_d, a_t + (hh * kMma + m) * 8,
+                  tmem, a_t + (bp * kMma + m) * 8,
                   bdesc + (((m >> 2) * (NT * 128) + (m & 3) * 256) >> 4), accum);
               accum = 1;
             }
             if constexpr (Cfg::kSums)
-              if (half == 1 && hh == kBPer - 1) {  // residues of the super-block's mins
-                tc_mma_f16_ta_w<tc_desc_hi(256), Cfg::kIdesc>(tmem_d, tmem + Cfg::kE0 + eslot * 8,
-                                                              bdesc + (Cfg::kBStep >> 4), 1u);
+              if (ap == kAParts - 1 && bp == kPer - 1) {  // residues of the super-block's mins
+                tc_mma_f16_ta_w<tc_desc_hi(256), Cfg::kIdesc>(tmem, tmem + Cfg::kE0 + eslot * 8,
+                                                              bdesc + (Cfg::kBPart >> 4), 1u);
                 eslot = (eslot + 1) % Cfg::kESlots;
               }
             tc_commit_w(&b_free[rb.i]);
@@ -467,12 +469,12 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
           tc_commit_w(&a_free[ra.i]);
         }
       }
-      tc_commit_w(&acc_full[rd.i]);
+      tc_commit_w(acc_full);
     }
   } else {
     // ================= dequantise into tensor memory, epilogue ==================================
-    const int q = warp & 3, c2 = (warp >> 2) & 1, grp = warp >> 3;  // lane quarter, 64-weight
-                                                                    // chunk of the step, group
+    const int q = warp & 3, c2 = (warp >> 2) & 1, grp = warp >> 3;  // lane quarter, which 64 of
+                                                                    // every 128 weights, group
     // row of the tile that this tensor-memory lane holds: a gate/up tile has 16 gate rows and the
     // 16 up rows of the same outputs in every lane quarter
     const int erow = p.glu ? (lane & 15) + 16 * q + (lane >> 4) * 64 : q * 32 + lane;
@@ -482,8 +484,7 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
     // ---- epilogue of a job: this warp's NT / 4 tokens of its 32 lanes --------------------------
     auto epilogue = [&](int j) {
       const QmJob job = qm_job(p.deal, j);
-      const int buf = j % kAccBufs;
-      ok = ok && tc_wait_w(&acc_full[buf], (uint32_t)((j / kAccBufs) & 1), p.status);
+      ok = ok && tc_wait_w(acc_full, (uint32_t)(j & 1), p.status);
       tc_after_sync();
       int si = 0;
       if (!p.glu) {
@@ -495,7 +496,7 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
       const int row = p.glu ? job.tile * 64 + 16 * q + (lane & 15)
                             : (job.tile - sg.tile0) * kQmRows + q * 32 + lane;
       const bool row_ok = ok && row < sg.N;
-      // the whole share into registers, then the accumulator is free for the job after next
+      // the whole share into registers, then the accumulator is free for the next job
       uint32_t va[NT / 64][16];
 #pragma unroll
       for (int g = 0; g < NT / 64; ++g) {  // 16 tokens at a time
@@ -506,12 +507,12 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
               "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
               "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(lane_base + (uint32_t)(buf * NT + (warp >> 2) * (NT / 4) + 16 * g)));
+            : "r"(lane_base + (uint32_t)((warp >> 2) * (NT / 4) + 16 * g)));
       }
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       tc_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_free[buf]);
+      if (lane == 0) mbar_arrive(acc_free);
 #pragma unroll
       for (int g = 0; g < NT / 64; ++g) {
         const int m0 = (warp >> 2) * (NT / 4) + 16 * g;
@@ -582,21 +583,20 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
       }
     }
     const bool epi = warp < kEpiWarps;
-    int s = grp;       // this warp's steps: grp, grp + kGroups, ...
-    int end = 0;       // first step of the next job
+    int s = grp;       // this warp's stages: grp, grp + kGroups, ...
+    int end = 0;       // first stage of the next job
     int pending = -1;  // job whose epilogue is due
     TcRing<kPkStages> rp;
     TcRing<kAStages> ra;
-    rp.advance(grp >> 1);
+    rp.advance(grp / kAParts);
     ra.advance(grp);
     for (int j = 0; j < njobs; ++j) {
-      end += 2 * qm_job(p.deal, j).n;
+      end += kAParts * qm_job(p.deal, j).n;
       int since = 0;
       for (; s < end; s += kGroups) {
-        const int c = 2 * (s & 1) + c2;  // sub-blocks 2c, 2c+1 of unit s / 2
         ok = ok && tc_wait_w(&pk_full[rp.i], rp.phase, p.status);
         const uint8_t* blk = pk + (size_t)rp.i * kPkBytes + (size_t)erow * kUnit;
-        const uint32_t a_t = a_base + ra.i * kQmACols;
+        const uint32_t a_t = a_base + ra.i * kACols;
         auto stage_free = [&]() {
           ok = ok && tc_wait_w(&a_free[ra.i], ra.phase ^ 1, p.status);
           tc_after_sync();
@@ -610,62 +610,70 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
               "r"(o[15])
               : "memory");
         };
-        if constexpr (FMT == 12) {
-          // super-block of this row: f16 d, f16 dmin, 12 bytes of 6-bit scales and mins, 128 bytes
-          // of nibbles (Hesper/Quantization/Q4_K_M.lean:13-52,120-144)
-          const uint4 hdr = *reinterpret_cast<const uint4*>(blk);
-          const uint4 qa = *reinterpret_cast<const uint4*>(blk + 16 + 32 * c);
-          const uint4 qb = *reinterpret_cast<const uint4*>(blk + 32 + 32 * c);
-          // scale / min bytes j and j+1 (j = 2c) out of the 12 packed bytes hdr.y, hdr.z, hdr.w
-          uint32_t sc2, m2;  // two 6-bit values each, in bytes 0 and 1
-          const int sh = 16 * c2;
-          if (!(s & 1)) {
-            sc2 = (hdr.y >> sh) & 0x3F3Fu;
-            m2 = (hdr.z >> sh) & 0x3F3Fu;
+        uint4 hdr;
+        if constexpr (FMT == 12) hdr = *reinterpret_cast<const uint4*>(blk);
+#pragma unroll
+        for (int hh = 0; hh < 2 / kAParts; ++hh) {
+          const int half = kAParts == 1 ? hh : (s & 1);
+          const int c = 2 * half + c2;  // sub-blocks 2c, 2c+1
+          const uint32_t col0 = 64u * hh;
+          if constexpr (FMT == 12) {
+            // super-block of this row: f16 d, f16 dmin, 12 bytes of 6-bit scales and mins, 128 bytes
+            // of nibbles (Hesper/Quantization/Q4_K_M.lean:13-52,120-144)
+            const uint4 qa = *reinterpret_cast<const uint4*>(blk + 16 + 32 * c);
+            const uint4 qb = *reinterpret_cast<const uint4*>(blk + 32 + 32 * c);
+            // scale / min bytes j and j+1 (j = 2c) out of the 12 packed bytes hdr.y, hdr.z, hdr.w
+            uint32_t sc2, m2;  // two 6-bit values each, in bytes 0 and 1
+            const int sh = 16 * c2;
+            if (half == 0) {
+              sc2 = (hdr.y >> sh) & 0x3F3Fu;
+              m2 = (hdr.z >> sh) & 0x3F3Fu;
+            } else {
+              sc2 = ((hdr.w >> sh) & 0x0F0Fu) | ((hdr.y >> (sh + 2)) & 0x3030u);
+              m2 = ((hdr.w >> (sh + 4)) & 0x0F0Fu) | ((hdr.z >> (sh + 2)) & 0x3030u);
+            }
+            // {scale 2c, scale 2c+1} as f16, then multiplier and addend of the two nibble positions
+            const __half2 k1024 = __floats2half2_rn(1024.f, 1024.f);
+            const __half2 sc = __hsub2(as_h2(__byte_perm(sc2, 0x64646464u, 0x4140)), k1024);
+            const __half2 mn = __hsub2(as_h2(__byte_perm(m2, 0x64646464u, 0x4140)), k1024);
+            const __half2 mul = __hmul2(sc, __floats2half2_rn(1.f, 0.0625f));
+            const __half2 add = __hmul2(sc, __floats2half2_rn(-1024.f, -64.f));
+            // c = -dmin * m rounded to f16, and 32 times what that lost (an f16 fma forms dmin * m + c
+            // exactly up to its own rounding)
+            const __half2 dm = __high2half2(as_h2(hdr.x));
+            const __half2 cc = __hneg2(__hmul2(dm, mn));
+            const __half2 lost = __hmul2(__hfma2(dm, mn, cc), __floats2half2_rn(-32.f, -32.f));
+            const uint32_t qq[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+            const __half2 d = __low2half2(as_h2(hdr.x));
+            uint32_t o[16];
+            q4k_expand<false>(qq, d, __low2half2(mul), __low2half2(add), __low2half2(cc), o);
+            if (hh == 0) stage_free();
+            store16(col0, o);
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(
+                             lane_base + (uint32_t)(Cfg::kE0 + 8 * ((s / kAParts) % Cfg::kESlots) + c)),
+                         "r"(as_u32(lost))
+                         : "memory");
+            q4k_expand<true>(qq, d, __high2half2(mul), __high2half2(add), __high2half2(cc), o);
+            store16(col0 + 16, o);
           } else {
-            sc2 = ((hdr.w >> sh) & 0x0F0Fu) | ((hdr.y >> (sh + 2)) & 0x3030u);
-            m2 = ((hdr.w >> (sh + 4)) & 0x0F0Fu) | ((hdr.z >> (sh + 2)) & 0x3030u);
+            // Q8_0 (Hesper/Layers/Linear.lean:6207-6223): blocks 2c and 2c+1 of the row's eight, 34
+            // bytes each -- f16 d, then 32 int8.  The chunk starts on a word; block 2c's quants sit
+            // two bytes into it (funnel shifts), block 2c+1's are word aligned.
+            const uint32_t* wq = reinterpret_cast<const uint32_t*>(blk + 68 * c);
+            uint32_t w[9], o[16];
+#pragma unroll
+            for (int i = 0; i < 9; ++i) w[i] = wq[i];
+            const __half2 d0 = __half2half2(__ushort_as_half((unsigned short)(w[0] & 0xFFFFu)));
+            const __half2 d1 = __half2half2(__ushort_as_half((unsigned short)(w[8] >> 16)));
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              q80_word(__funnelshift_r(w[i], w[i + 1], 16), d0, o[2 * i], o[2 * i + 1]);
+            if (hh == 0) stage_free();
+            store16(col0, o);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q80_word(wq[9 + i], d1, o[2 * i], o[2 * i + 1]);
+            store16(col0 + 16, o);
           }
-          // {scale 2c, scale 2c+1} as f16, then multiplier and addend of the two nibble positions
-          const __half2 sc = __hsub2(as_h2(__byte_perm(sc2, 0x64646464u, 0x4140)), __floats2half2_rn(1024.f, 1024.f));
-          const __half2 mn = __hsub2(as_h2(__byte_perm(m2, 0x64646464u, 0x4140)), __floats2half2_rn(1024.f, 1024.f));
-          const __half2 mul = __hmul2(sc, __floats2half2_rn(1.f, 0.0625f));
-          const __half2 add = __hmul2(sc, __floats2half2_rn(-1024.f, -64.f));
-          // c = -dmin * m rounded to f16, and 32 times what that lost (an f16 fma forms dmin * m + c
-          // exactly up to its own rounding)
-          const __half2 dm = __high2half2(as_h2(hdr.x));
-          const __half2 cc = __hneg2(__hmul2(dm, mn));
-          const __half2 lost = __hmul2(__hneg2(__hfma2(dm, mn, cc)), __floats2half2_rn(32.f, 32.f));
-          const uint32_t qq[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-          const __half2 d = __low2half2(as_h2(hdr.x));
-          uint32_t o[16];
-          q4k_expand<false>(qq, d, __low2half2(mul), __low2half2(add), __low2half2(cc), o);
-          stage_free();
-          store16(0, o);
-          asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(
-                           lane_base + (uint32_t)(Cfg::kE0 + 8 * ((s >> 1) % Cfg::kESlots) + c)),
-                       "r"(as_u32(lost))
-                       : "memory");
-          q4k_expand<true>(qq, d, __high2half2(mul), __high2half2(add), __high2half2(cc), o);
-          store16(16, o);
-        } else {
-          // Q8_0 (Hesper/Layers/Linear.lean:6207-6223): blocks 2c and 2c+1 of the row's eight, 34
-          // bytes each -- f16 d, then 32 int8.  The chunk starts on a word; block 2c's quants sit
-          // two bytes into it (funnel shifts), block 2c+1's are word aligned.
-          const uint32_t* wq = reinterpret_cast<const uint32_t*>(blk + 68 * c);
-          uint32_t w[9], o[16];
-#pragma unroll
-          for (int i = 0; i < 9; ++i) w[i] = wq[i];
-          const __half2 d0 = __half2half2(__ushort_as_half((unsigned short)(w[0] & 0xFFFFu)));
-          const __half2 d1 = __half2half2(__ushort_as_half((unsigned short)(w[8] >> 16)));
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            q80_word(__funnelshift_r(w[i], w[i + 1], 16), d0, o[2 * i], o[2 * i + 1]);
-          stage_free();
-          store16(0, o);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) q80_word(wq[9 + i], d1, o[2 * i], o[2 * i + 1]);
-          store16(16, o);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&pk_free[rp.i]);
@@ -674,7 +682,7 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
         __syncwarp();
         if (lane == 0) mbar_arrive(&a_full[ra.i]);
         ra.advance(kGroups);
-        rp.advance(((s & 1) + kGroups) >> 1);
+        rp.advance(kAParts == 1 ? kGroups : ((s & 1) + kGroups) >> 1);
         // the A stages are refilled for this job: now the previous job's accumulator
         if (pending >= 0 && ++since == kAStages / kGroups) {
           wait_previous();
