@@ -49,7 +49,7 @@ struct KQParams {
   int K;
   int M;
   int stages;   // tiles a warp keeps in flight
-  int nslots;   // stage slots of the CTA: min(warps*stages, most tiles any CTA owns)
+  int nslots;   // stage slots of the CTA: warps*stages; for one token at most the tiles any CTA owns
   const float* x;
   const float* gamma;
   float eps;
@@ -615,7 +615,10 @@ struct KQPlan {
 //      prefetch (tallest tile wins);
 //  (b) a ring of >= 2 stages inside half of the shared memory, most bytes in flight;
 //  (c) the same inside the whole shared memory;  (d) whatever fits.
-static bool kq_plan(const hb200_ctx* ctx, long rows, int K, int rowbytes, bool gu, bool pre,
+// With one token a warp never fills more slots than it has tiles, and slots past the CTA's last
+// tile are not laid out.  Later tokens go around the ring again from wherever the last one
+// stopped: every warp then has all its slots.
+static bool kq_plan(const hb200_ctx* ctx, long rows, int K, int M, int rowbytes, bool gu, bool pre,
                     KQPlan* out) {
   // One CTA per SM (the kernel wants ~166 registers per thread; capping it at the 80 that
   // would let two launches share an SM made it re-derive addresses and constants inside
@@ -631,7 +634,7 @@ static bool kq_plan(const hb200_ctx* ctx, long rows, int K, int rowbytes, bool g
       const int tpw = (tpc + kKQWarps - 1) / kKQWarps;
       const int srows = gu ? 2 * rt : rt;
       for (int st = (tpw < 4 ? tpw : 4); st >= 1; --st) {
-        const int nslots = kKQWarps * st < tpc ? kKQWarps * st : tpc;
+        const int nslots = M > 1 || kKQWarps * st < tpc ? kKQWarps * st : tpc;
         const size_t sm = kq_smem_bytes(nslots, srows, K, rowbytes, pre);
         bool ok = false;
         if (pass == 0) ok = st == tpw && sm <= half;
@@ -735,7 +738,7 @@ static int kq_forward_multi_impl(hb200_ctx* ctx, int fmt, const hb200_kquant_seg
   }
   const int rowbytes = kq_rowbytes(fmt, K);
   KQPlan plan;
-  if (!kq_plan(ctx, rows, K, rowbytes, false, pre.gamma != nullptr, &plan)) {
+  if (!kq_plan(ctx, rows, K, M, rowbytes, false, pre.gamma != nullptr, &plan)) {
     set_error("kquant: K=%d does not fit the shared-memory budget", K);
     return HB200_ERR_UNSUPPORTED;
   }
@@ -819,7 +822,7 @@ static int kq_gateup_impl(hb200_ctx* ctx, int fmt, const void* d_blocks_gate,
   }
   const int rowbytes = kq_rowbytes(fmt, K);
   KQPlan plan;
-  if (!kq_plan(ctx, N, K, rowbytes, true, pre.gamma != nullptr, &plan)) {
+  if (!kq_plan(ctx, N, K, M, rowbytes, true, pre.gamma != nullptr, &plan)) {
     set_error("kquant gate/up: K=%d does not fit the shared-memory budget", K);
     return HB200_ERR_UNSUPPORTED;
   }

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 import torch
 
+import hesper_b200 as hb
 from hesper_b200 import LinearLayer, QuantFormat, formats
 from test_oracle_kquant import reference_q4k_block
 
@@ -39,6 +40,25 @@ def test_matvec_shapes(ctx, oracle, fmt, K, N):
     ctx.check()
     err = _check(y, ref)
     assert err < 2e-4  # the kernel's own design point: 16-bit block-scaled activations
+
+
+@pytest.mark.parametrize("fmt", [12, 8])
+@pytest.mark.parametrize("M", [2, 17])
+def test_streaming_kernel_several_tokens(oracle, monkeypatch, fmt, M):
+    """The streaming kernel sends every token around its ring of weight tiles again.  18 and 35
+    tiles per CTA on 12 warps: some warps hold a tile more than others, so the second token starts
+    at different ring positions."""
+    monkeypatch.setenv("HB200_NO_MMA", "1")
+    K, N = 2560, 10240
+    rng = np.random.default_rng(M + fmt)
+    blocks = formats.random_kquant(rng, fmt, N, K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    c = hb.Context(0)
+    y = LinearLayer.create_from_bytes(c, blocks, fmt, K, N).forward(_dev(x))
+    c.check()
+    c.close()
+    rows = [0, 1, M - 1]
+    assert _check(y[rows], oracle.kquant_matvec(fmt, blocks, K, N, x[rows])) < 2e-4
 
 
 def test_reference_block_fixture(ctx, oracle):
