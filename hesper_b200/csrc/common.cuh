@@ -251,6 +251,14 @@ int hb_kq_stage(struct hb200_ctx* ctx, int fmt, int K, int NT, const float* d_x,
                 const float* d_pre_base, const float* d_pre_gamma, float* d_pre_out,
                 const float* d_rms_gamma, float rms_eps, cudaStream_t st);
 
+int hb_kq_stage_i8(struct hb200_ctx* ctx, int fmt, int K, int ntl, const float* d_x, int M,
+                   const float* d_pre_base, const float* d_pre_gamma, float* d_pre_out,
+                   const float* d_rms_gamma, float rms_eps, cudaStream_t st);
+// Q4_K / Q8_0 product of 2 to 15 tokens on mma.sync (kquant_sb.cu); 1 = shape not covered
+int hb_kq_sb_run(struct hb200_ctx* ctx, int fmt, const hb200_kquant_seg* segs, int nseg, int K, int gu,
+                 const float* d_x, int M, const float* pre_base, const float* pre_gamma, float* pre_out,
+                 const float* gamma, float eps, cudaStream_t st);
+
 struct hb200_ctx {
   int device;
   int sm_count;

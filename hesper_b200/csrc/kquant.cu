@@ -594,6 +594,15 @@ static int kq_batched_fused(hb200_ctx* ctx, int fmt, const KQBatchSeg* segs, int
   return HB200_OK;
 }
 
+// Whether 2 to 15 tokens take the kernel of kquant_sb.cu rather than this one, whose time grows by
+// a whole product per token.  Measured, us (this / that kernel): Q4_K K=2560 N=10240 at 2, 7, 15
+// tokens 10.1 / 9.2, 28.9 / 9.3, 58.7 / 11.8; Q8_0 12.8 / 10.6, 36.9 / 11.7, 74.7 / 12.2; Q4_K
+// K=10240 N=2560 14.2 / 15.7, 45.5 / 15.7, 95.6 / 17.8; K=2560 N=512 4.8 / 5.0, 13.9 / 5.0, 28.5 / 5.6.
+// So only two tokens on Q4_K with fewer rows than K stay.
+static bool kq_few_tokens(const hb200_ctx* ctx, int fmt, long rows, int K, int M) {
+  return M >= 2 && M < kKQBatchedFrom && !ctx->no_mma && (M > 2 || fmt == HB200_FMT_Q8_0 || rows >= K);
+}
+
 // ---- host side --------------------------------------------------------------------
 
 static size_t kq_smem_bytes(int nslots, int rows, int K, int rowbytes, bool pre) {
@@ -735,6 +744,9 @@ static int kq_forward_multi_impl(hb200_ctx* ctx, int fmt, const hb200_kquant_seg
     rc = hb_kq_mv_run(ctx, fmt, segs, nseg, K, 0, d_x, pre.base, pre.gamma, pre.out, d_rms_gamma,
                       rms_eps, st);
     if (rc <= 0) return rc;
+  } else if (kq_few_tokens(ctx, fmt, rows, K, M)) {
+    rc = hb_kq_sb_run(ctx, fmt, segs, nseg, K, 0, d_x, M, pre.base, pre.gamma, pre.out, d_rms_gamma, rms_eps, st);
+    if (rc <= 0) return rc;
   }
   const int rowbytes = kq_rowbytes(fmt, K);
   KQPlan plan;
@@ -814,10 +826,13 @@ static int kq_gateup_impl(hb200_ctx* ctx, int fmt, const void* d_blocks_gate,
     return kq_batched_fused(ctx, fmt, g, 2, 1, K, d_x, M, pre, d_rms_gamma, rms_eps, st);
   }
   HB_REQUIRE(M <= 64, "kquant gate/up: M=%d needs the batched path", M);
+  const hb200_kquant_seg gs[2] = {{d_blocks_gate, nullptr, d_y, N}, {d_blocks_up, nullptr, d_y, N}};
   if (M == 1) {
-    const hb200_kquant_seg gs[2] = {{d_blocks_gate, nullptr, d_y, N}, {d_blocks_up, nullptr, d_y, N}};
     rc = hb_kq_mv_run(ctx, fmt, gs, 2, K, 1, d_x, pre.base, pre.gamma, pre.out, d_rms_gamma,
                       rms_eps, st);
+    if (rc <= 0) return rc;
+  } else if (kq_few_tokens(ctx, fmt, 2L * N, K, M)) {
+    rc = hb_kq_sb_run(ctx, fmt, gs, 2, K, 1, d_x, M, pre.base, pre.gamma, pre.out, d_rms_gamma, rms_eps, st);
     if (rc <= 0) return rc;
   }
   const int rowbytes = kq_rowbytes(fmt, K);

@@ -182,6 +182,12 @@ __device__ __forceinline__ QmJob qm_job(const QmDeal& d, int j) {
 // second half zero).  The four bytes of a weight word pair up as {0, 2}, {1, 3}: so do the k here.
 // Latency is all there is to it (a row, three block-wide reductions at most), so the row stays
 // in registers from its one read and the norm weights are fetched before the wait.
+//
+// I8: the operand of the few-token kernel instead (kquant_sb.cu).  Every 32 elements become 16-bit
+// integers of their own scale, x ~ dx * (256*hi + lo) with hi and lo signed bytes, laid out as
+// mma.sync's B fragments per (sub-block, 8 tokens): lane 4 * (token % 8) + t holds {hi, hi, lo, lo}
+// of elements 8t..8t+7; behind them {dx, dx, sum, sum} of two tokens per entry.  Rows past the last
+// token are zero.
 struct QmStage {
   const float *x, *gamma, *pre_base, *pre_gamma;
   float* pre_out;
@@ -191,9 +197,10 @@ struct QmStage {
   size_t sb_bytes;   // bytes of a super-block
   int sums_off;      // where its sums start, 0: none
   float* rowscale;
+  int M, ntl;        // I8 only: tokens, token columns / 8
 };
 
-template <int G>
+template <int G, bool I8>
 __global__ void __launch_bounds__(1024) kq_stage_kernel(const __grid_constant__ QmStage p) {
   __shared__ double red[2][32];
   __shared__ float redf[32];
@@ -219,12 +226,13 @@ __global__ void __launch_bounds__(1024) kq_stage_kernel(const __grid_constant__ 
     if (i < n8 && p.pre_gamma) load8(pg[j], p.pre_gamma, i, true);
   }
   pdl_wait();
+  const bool real = !I8 || m < p.M;  // I8: the whole CTA of a row past the last token stays at zero
 #pragma unroll
   for (int j = 0; j < G; ++j) {
     const int i = tid + j * blockDim.x;
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[j][e] = 0.f;
-    if (i < n8) load8(v[j], p.x + (size_t)m * p.K, i, false);
+    if (real && i < n8) load8(v[j], p.x + (size_t)m * p.K, i, false);
   }
   auto row_rinv = [&](double* scr) {  // 1 / rms of the row held in v (block-wide)
     double ss = 0.0;
@@ -238,7 +246,7 @@ __global__ void __launch_bounds__(1024) kq_stage_kernel(const __grid_constant__ 
     ss = warp_sum(lane < nwarps ? scr[lane] : 0.0);
     return (float)(1.0 / sqrt(ss / (double)p.K + (double)p.eps));
   };
-  if (p.pre_gamma) {
+  if (real && p.pre_gamma) {
     float b[G][8];
 #pragma unroll
     for (int j = 0; j < G; ++j) {
@@ -259,7 +267,7 @@ __global__ void __launch_bounds__(1024) kq_stage_kernel(const __grid_constant__ 
       }
     }
   }
-  if (p.gamma) {
+  if (real && p.gamma) {
     const float rinv = row_rinv(red[1]);
 #pragma unroll
     for (int j = 0; j < G; ++j)
@@ -267,6 +275,41 @@ __global__ void __launch_bounds__(1024) kq_stage_kernel(const __grid_constant__ 
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[j][e] = __fmul_rn(__fmul_rn(v[j][e], rinv), g[j][e]);
       }
+  }
+  if constexpr (I8) {
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      const int i = tid + j * blockDim.x;
+      float amax = 0.f, sum = 0.f;  // of the four lanes that share 32 elements
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        amax = fmaxf(amax, fabsf(v[j][e]));
+        sum += v[j][e];
+      }
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      }
+      if (i >= n8) continue;
+      const float inv = amax > 0.f ? 32512.0f / amax : 0.f;
+      uint32_t q[8];  // q + 128 = 256 * hi + (lo + 128): hi is its byte 1, lo its byte 0 ^ 0x80
+#pragma unroll
+      for (int e = 0; e < 8; ++e) q[e] = (uint32_t)(__float2int_rn(v[j][e] * inv) + 128);
+      auto bytes = [&](int a, uint32_t sel) {
+        return __byte_perm(__byte_perm(q[a], q[a + 1], sel), __byte_perm(q[a + 2], q[a + 3], sel), 0x5410);
+      };
+      const int sj = (i >> 2) & 7, t = i & 3, nt = m >> 3, g = m & 7;
+      uint8_t* sb = p.xb + (size_t)(i >> 5) * p.sb_bytes;
+      *reinterpret_cast<uint4*>(sb + ((sj * p.ntl + nt) * 32 + 4 * g + t) * 16) =
+          make_uint4(bytes(0, 0x0051), bytes(4, 0x0051), bytes(0, 0x0040) ^ 0x80808080u,
+                     bytes(4, 0x0040) ^ 0x80808080u);
+      float* tab = reinterpret_cast<float*>(sb + p.ntl * 4096 + ((sj * p.ntl + nt) * 4 + (g >> 1)) * 16) + (g & 1);
+      // Q4_K multiplies the high nibbles in place: their 16 is taken off here
+      if (t == 0) tab[0] = amax / 32512.0f * (p.sums_off && (sj & 1) ? 0.0625f : 1.f);
+      if (t == 1) tab[2] = sum;
+    }
+    return;
   }
   float amax = 0.f;
 #pragma unroll
@@ -875,6 +918,16 @@ int hb_kq_mma_max_tokens(int fmt, int K) {
   return 64;
 }
 
+template <bool I8>
+static int qm_stage_launch(hb200_ctx* ctx, const QmStage& p, int rows, cudaStream_t st) {
+  const int n8 = p.K / 8;  // groups of 8 elements; one or two per thread, eight for a huge row
+  const int G = n8 <= 640 ? 1 : (n8 <= 2048 ? 2 : 8);
+  const int threads = ((n8 + G - 1) / G + 31) & ~31;
+  auto kern = G == 1 ? kq_stage_kernel<1, I8> : (G == 2 ? kq_stage_kernel<2, I8> : kq_stage_kernel<8, I8>);
+  HB_CUDA(launch_pdl(kern, dim3(rows), dim3(threads), 0, st, ctx->pdl, p));
+  return HB200_OK;
+}
+
 // x[M][K] (M <= NT) -> f16 operand layout and row scales in the context scratch; optional pre-step
 // x' = d_pre_base + rmsnorm(d_x) * d_pre_gamma (written to d_pre_out), optional RMSNorm.
 int hb_kq_stage(hb200_ctx* ctx, int fmt, int K, int NT, const float* d_x, int M,
@@ -894,14 +947,27 @@ int hb_kq_stage(hb200_ctx* ctx, int fmt, int K, int NT, const float* d_x, int M,
   p.K = K;
   p.xb = static_cast<uint8_t*>(ctx->d_scratch) + kScratchLmSplit;
   p.rowscale = reinterpret_cast<float*>(static_cast<uint8_t*>(ctx->d_scratch) + kScratchRowScale);
-  const int n8 = K / 8;  // groups of 8 elements; one or two per thread, eight for a huge row
-  const int G = n8 <= 640 ? 1 : (n8 <= 2048 ? 2 : 8);
-  const int threads = ((n8 + G - 1) / G + 31) & ~31;
-  if (G == 1)
-    HB_CUDA(launch_pdl(kq_stage_kernel<1>, dim3(M), dim3(threads), 0, st, ctx->pdl, p));
-  else if (G == 2)
-    HB_CUDA(launch_pdl(kq_stage_kernel<2>, dim3(M), dim3(threads), 0, st, ctx->pdl, p));
-  else
-    HB_CUDA(launch_pdl(kq_stage_kernel<8>, dim3(M), dim3(threads), 0, st, ctx->pdl, p));
-  return HB200_OK;
+  return qm_stage_launch<false>(ctx, p, M, st);
+}
+
+// The same for the few-token kernel (kquant_sb.cu): ntl * 8 token columns, M of them real.
+int hb_kq_stage_i8(hb200_ctx* ctx, int fmt, int K, int ntl, const float* d_x, int M, const float* d_pre_base,
+                   const float* d_pre_gamma, float* d_pre_out, const float* d_rms_gamma, float rms_eps,
+                   cudaStream_t st) {
+  QmStage p = {};
+  p.sb_bytes = (size_t)ntl * 4608;
+  p.sums_off = fmt == HB200_FMT_Q4_K;
+  HB_REQUIRE(p.sb_bytes * (size_t)(K / 256) <= kScratchRowScale - kScratchLmSplit && K <= 65536,
+             "kquant (few tokens): K=%d does not fit the activation scratch", K);
+  p.x = d_x;
+  p.gamma = d_rms_gamma;
+  p.pre_base = d_pre_base;
+  p.pre_gamma = d_pre_gamma;
+  p.pre_out = d_pre_out;
+  p.eps = rms_eps;
+  p.K = K;
+  p.M = M;
+  p.ntl = ntl;
+  p.xb = static_cast<uint8_t*>(ctx->d_scratch) + kScratchLmSplit;
+  return qm_stage_launch<true>(ctx, p, ntl * 8, st);
 }

@@ -61,7 +61,7 @@ typedef void *hb200_stream;
  * allocates afterwards; a context serves one stream at a time (a call that arrives on
  * another stream than the previous scratch user's is ordered behind it with an event).
  * Environment: HB200_NO_PDL=1 launches without programmatic dependent launch,
- * HB200_NO_MMA=1 keeps the batched (>= 16 token) operators off the tensor-core kernels,
+ * HB200_NO_MMA=1 keeps the batched operators (16 tokens, k-quants 2) off the tensor-core kernels,
  * HB200_MV=0 / 2 keeps one-token matvecs off the mma.sync kernels / uses them wherever the
  * shape fits (default 1: ternary wherever two launches share an SM, k-quants where that holds
  * and it measured faster than the streaming kernel).

@@ -102,6 +102,39 @@ def test_gate_up_gelu(ctx, oracle, fmt, K, N, M):
     _check(y, ref)
 
 
+@pytest.mark.parametrize("fmt", [12, 8])
+@pytest.mark.parametrize("K,Ns,M,gate_up", [
+    (256, [1], 3, False),            # one super-block, one row: most warps idle
+    (768, [5, 640], 8, False),       # rows of two tensors on disjoint CTAs, all 8 columns of a tile
+    (2560, [2048, 512, 130], 9, False),  # second column tile with one token
+    (512, [148 * 128 + 37], 15, False),  # two passes per CTA, the second one ragged
+    (1024, [148 * 64 + 11], 3, True),    # gate/up, two passes
+    (2560, [333], 12, True), (2560, [2600], 2, False)])
+def test_few_tokens(ctx, oracle, fmt, K, Ns, M, gate_up):
+    """2 to 15 tokens: 16-bit block-quantised activations, exact integer products.  An activation
+    is off by at most 2^-16 of its block's largest: 2e-4 of max|y| as for one token."""
+    rng = np.random.default_rng(K + sum(Ns) + M + fmt)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    gamma = (1.0 + 0.1 * rng.standard_normal(K)).astype(np.float32)
+    xn = np.stack([oracle.rmsnorm_f64(x[m], gamma, 1e-6) for m in range(M)]).astype(np.float32)
+    if gate_up:
+        bg, bu = (formats.random_kquant(rng, fmt, Ns[0], K) for _ in range(2))
+        g, u = (LinearLayer.create_from_bytes(ctx, b, fmt, K, Ns[0]) for b in (bg, bu))
+        y = LinearLayer.forward_fused_gate_up(g, u, _dev(x), rms_gamma=_dev(gamma), eps=1e-6)
+        ctx.check()
+        assert _check(y, oracle.kquant_gateup_gelu(bg, bu, fmt, K, Ns[0], xn)) < 2e-4
+        return
+    blocks = [formats.random_kquant(rng, fmt, n, K) for n in Ns]
+    layers = [LinearLayer.create_from_bytes(ctx, b, fmt, K, n) for b, n in zip(blocks, Ns)]
+    res = rng.standard_normal((M, Ns[0])).astype(np.float32)
+    y = layers[0].forward(_dev(x), residual=_dev(res))
+    assert _check(y, oracle.kquant_matvec(fmt, blocks[0], K, Ns[0], x, residual=res)) < 2e-4
+    ys = LinearLayer.forward_multi(layers, _dev(x), rms_gamma=_dev(gamma), eps=1e-6)
+    ctx.check()
+    for b, n, y in zip(blocks, Ns, ys):
+        assert _check(y, oracle.kquant_matvec(fmt, b, K, n, xn)) < 2e-4
+
+
 def test_fused_qkv_multi(ctx, oracle):
     K = 2560
     rng = np.random.default_rng(8)
