@@ -528,8 +528,8 @@ extern "C" int hb200_bitlinear_forward_multi(hb200_ctx* ctx, const hb200_bitline
     rows += segs[s].N;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // tokens per pass over the weights: 128 on the tensor cores, 64 on the dp4a kernel
-  const int pass = (K <= 12288 && !ctx->no_mma) ? 128 : 64;
+  // tokens per call: 512 on the tensor cores, 64 on the dp4a kernel
+  const int pass = (K <= 12288 && !ctx->no_mma) ? kBlMmaTokens : 64;
   if (M > pass) {
     for (int m0 = 0; m0 < M; m0 += pass) {
       const int mc = M - m0 < pass ? M - m0 : pass;
@@ -549,7 +549,7 @@ extern "C" int hb200_bitlinear_forward_multi(hb200_ctx* ctx, const hb200_bitline
   }
   // 16 or more tokens: a real contraction -> tensor cores (weights still streamed once)
   if (M >= 16 && K <= 12288 && !ctx->no_mma)
-    return hb_bitlinear_mma_run(ctx, segs, nseg, K, d_x, M, d_rms_gamma, rms_eps, d_act_scale, st);
+    return hb_bitlinear_mma_run(ctx, segs, nseg, K, 0, d_x, M, d_rms_gamma, rms_eps, d_act_scale, st);
   if (M == 1) {  // one token: integer tensor-core matvec when the rows fit shared memory
     rc = hb_bl_mv_run(ctx, segs, nseg, K, 0, d_x, d_rms_gamma, rms_eps, d_act_scale, st);
     if (rc <= 0) return rc;
@@ -626,11 +626,8 @@ extern "C" int hb200_bitlinear_gateup_relu2(hb200_ctx* ctx, const void* d_packed
   HB_REQUIRE(((reinterpret_cast<uintptr_t>(d_packed_gate) |
                reinterpret_cast<uintptr_t>(d_packed_up)) & 15) == 0,
              "bitlinear gate/up: weights must be 16-byte aligned");
-  // tokens per pass: 128 where both products run on the tensor cores into the scratch, else 64
-  const int pass = (K <= 12288 && !ctx->no_mma &&
-                    kScratchGlu + (size_t)2 * 128 * N * sizeof(float) <= kScratchRowScale)
-                       ? 128
-                       : 64;
+  // tokens per call: 512 on the tensor cores, 64 on the dp4a kernel
+  const int pass = (K <= 12288 && !ctx->no_mma) ? kBlMmaTokens : 64;
   if (M > pass) {
     for (int m0 = 0; m0 < M; m0 += pass) {
       const int mc = M - m0 < pass ? M - m0 : pass;
@@ -641,19 +638,12 @@ extern "C" int hb200_bitlinear_gateup_relu2(hb200_ctx* ctx, const void* d_packed
     }
     return HB200_OK;
   }
-  if (M >= 16 && K <= 12288 && !ctx->no_mma &&
-      kScratchGlu + (size_t)2 * M * N * sizeof(float) <= kScratchRowScale) {
-    // batched: both products on the tensor cores into scratch (the region may run into the
-    // staging area of the 16-bit products, which no ternary operator uses), then the GLU
-    ScratchUse use(ctx, static_cast<cudaStream_t>(stream));
-    float* g = reinterpret_cast<float*>(static_cast<uint8_t*>(ctx->d_scratch) + kScratchGlu);
-    float* u = g + (size_t)M * N;
-    hb200_bitlinear_seg segs[2] = {{d_packed_gate, d_scale_gate, nullptr, g, nullptr, N},
-                                   {d_packed_up, d_scale_up, nullptr, u, nullptr, N}};
-    rc = hb_bitlinear_mma_run(ctx, segs, 2, K, d_x, M, d_rms_gamma, rms_eps, nullptr,
-                              static_cast<cudaStream_t>(stream));
-    if (rc) return rc;
-    return hb200_relu2_mul(ctx, g, u, (long)M * N, d_y, stream);
+  if (M >= 16 && K <= 12288 && !ctx->no_mma) {
+    // batched: both products on the tensor cores in one launch, the GLU in its epilogue
+    const hb200_bitlinear_seg segs[2] = {{d_packed_gate, d_scale_gate, nullptr, d_y, nullptr, N},
+                                         {d_packed_up, d_scale_up, nullptr, d_y, nullptr, N}};
+    return hb_bitlinear_mma_run(ctx, segs, 2, K, 1, d_x, M, d_rms_gamma, rms_eps, nullptr,
+                                static_cast<cudaStream_t>(stream));
   }
   if (M == 1) {
     const hb200_bitlinear_seg gs[2] = {{d_packed_gate, d_scale_gate, nullptr, d_y, nullptr, N},

@@ -1,4 +1,4 @@
-// bitlinear_mma.cu -- batched (16..64 tokens) ternary i2_s x int8 product on the 5th-generation
+// bitlinear_mma.cu -- batched (16 tokens or more) ternary i2_s x int8 product on the 5th-generation
 // tensor cores: tcgen05.mma kind::i8 with the int32 accumulator in tensor memory.
 //
 // Same arithmetic contract as the batch-1 kernel (bit-exact int32 accumulators, then
@@ -11,34 +11,38 @@
 //                      int8 activations are written straight in the shared-memory operand
 //                      layout (K-major, 8x16-byte core matrices), one 8 KB block per
 //                      128-wide K group, so the GEMM kernel fetches a B tile with ONE bulk copy
-//   bitlinear_mma_kernel  one CTA per 128 weight rows, 11 warps with fixed roles:
-//     * warp 9 issues every copy: the packed weights as boxes of 128 rows x 128 bytes
-//       (4 groups) through a 2-D tensor map with the 128-byte swizzle, ONE instruction per
-//       16 KB on a 4-deep ring (per-row 1-D bulk copies cost ~35 ns each at the TMA unit and
-//       throttled the stream), and each step's activations with one 16 KB bulk copy;
-//     * warps 0-7 expand two 128-wide groups per step from 2-bit codes to unsigned bytes
-//       (0,1,2) and store them with tcgen05.st straight into TENSOR MEMORY as the A operand
-//       (lane = weight row, 4 K-bytes per column): the expanded weights never touch shared
-//       memory, whose bandwidth bounded the earlier shared-memory-A version of this kernel;
-//     * warps 8 and 10 each issue the MMAs of every other step from one thread into their own
+//   bitlinear_mma_kernel  one CTA per 128 weight rows, block of 64 or 128 tokens and K range, 20
+//   warps with fixed roles (w = 0 the first behind the expanders):
+//     * warp 3 copies the packed weights as boxes of 64 rows x 128 bytes (4 groups) through a 2-D
+//       tensor map with the 128-byte swizzle, two per 16 KB slot of a 4-deep ring (per-row 1-D
+//       bulk copies cost ~35 ns each at the TMA unit); warp 1 each step's activations with one bulk
+//       copy.  Two warps: in one, a box was only asked for behind the waits of the activations;
+//     * 16 warps in two groups that take the steps in turn expand two 128-wide groups per step
+//       from 2-bit codes to unsigned bytes (0,1,2) and store them with tcgen05.st straight into
+//       TENSOR MEMORY as the A operand (lane = weight row, 4 K-bytes per column): the expanded
+//       weights never touch shared memory.  A step is a chain of ~1000 cycles of which its warps
+//       issue a tenth: this chain, not the tensor pipe, is what a 64-token CTA waits for;
+//     * warps 0 and 2 each issue the MMAs of every other step from one thread into their own
 //       accumulator (tcgen05.mma kind::i8, A from tensor memory, B by a shared-memory
-//       descriptor, M=128, N=64 tokens, K=32 per instruction; 2 x 64 columns of int32): one
-//       thread alone spends ~45 ns per MMA, two keep the tensor pipe busy.  One barrier per
-//       step gathers the 8 expander arrivals and the activation bytes; one tcgen05.commit
-//       per step releases the stage (6 stages = 384 columns of A);
-//     * epilogue: 8 warps read 32 lanes x 32 columns of both accumulators (tcgen05.ld
-//       32x32b), add them, subtract sum(q) per token (value = code - 1), scale and store;
-//     * split-K: a launch with few tiles (o_proj and down_proj have 20) splits K over several
-//       CTAs per tile; each publishes its int32 partial, the last to arrive (a ticket per
-//       tile) adds the others' and runs the epilogue -- exact, since integers commute.
+//       descriptor, M=128, N = tokens, K=32 per instruction).  One barrier per step gathers the 8
+//       expander arrivals and the activation bytes; one tcgen05.commit per step releases the stage;
+//     * epilogue: 16 warps read 32 lanes x 16 columns of both accumulators (tcgen05.ld 32x32b),
+//       add them, subtract sum(q) per token (value = code - 1), scale and store.  A gate/up pair is
+//       one launch: a tile holds 64 gate rows and the 64 up rows of the same outputs, a gate lane's
+//       up value sits 16 lanes further in the same warp;
+//     * split-K: each CTA publishes its int32 partial, the last to arrive (a ticket per tile and
+//       token block) adds the others' and runs the epilogue -- exact, since integers commute.
+// All tokens of a call (up to 512) go in one launch of each kernel: in passes of 128 a 256-token
+// prompt paid both launches' latency twice.  Measured, 256 tokens, K=2560: q/k/v (3840 rows), o_proj,
+// gate/up (2 x 6912, with the GLU) and down_proj (K=6912) together 150 -> 59 us.
 // Every mbarrier wait is bounded; on expiry the kernel still releases its tensor memory.
 #include "tcgen05.cuh"
 
 namespace hb {
 
-constexpr int kMmaThreads = 256;
+constexpr int kExpGroups = 2;   // groups of 8 expanding warps, taking the steps in turn
+constexpr int kMmaThreads = kExpGroups * 256;
 constexpr int kMmaRows = 128;    // weight rows per CTA = MMA M
-constexpr int kMmaTokens = 64;   // MMA N of the narrow variant (16..64 tokens)
 constexpr int kChunkGroups = 4;  // 128-weight groups per packed box: 128 bytes of every row
 constexpr int kPkStages = 4;     // packed ring
 constexpr int kPkBytes = kMmaRows * kChunkGroups * 32;  // 16 KB box
@@ -46,8 +50,7 @@ constexpr int kStepGroups = 2;   // groups per pipeline step: one barrier round 
 constexpr int kAGroupCols = 32;  // TMEM columns of one expanded group: 128 K-bytes per row
 constexpr int kMmaCtrl = 2048;   // barriers, tensor-memory slot, d[NT], sum(q)[NT]
 
-// NT tokens per pass = MMA N: 64, or 128 for the prompt passes (half the weight passes per
-// token).  Tensor memory, 512 columns: accumulator of the first issuing warp at 0, the A stages
+// NT tokens of a CTA = MMA N: 64 or 128.  Tensor memory, 512 columns: accumulator of the first issuing warp at 0, the A stages
 // behind it, the second warp's accumulator in the last NT columns.
 template <int NT>
 struct MmaCfg {
@@ -74,15 +77,17 @@ struct MmaSeg {
 };
 
 struct MmaParams {
-  CUtensorMap tmap[4];  // per segment: packed weights as [N rows][K/4 bytes], 128 x 128 boxes
+  CUtensorMap tmap[4];  // per segment: packed weights as [N rows][K/4 bytes], boxes of 64 rows x 128
   MmaSeg seg[4];
   int nseg, K, M;
+  int glu;             // seg 0 = gate, seg 1 = up: y = relu(gate)^2 * up into seg 0's y
+  int ntb;             // blocks of NT tokens; CTA = (tile * nsplit + split) * ntb + token block
   int nsplit, gps;     // split-K: CTAs per tile, groups per split
-  int32_t* part;       // [tile][split][NT tokens][128 rows] partial accumulators (nsplit > 1)
-  int* tickets;        // [tile] arrival counters, zero between launches
-  const uint8_t* xq;   // [K/128][NT tokens x 128 bytes, core-matrix layout]
-  const float* d;      // [NT] activation scales
-  const int32_t* sumq; // [NT]
+  int32_t* part;       // [tile][token block][split][NT tokens][128 rows] partials (nsplit > 1)
+  int* tickets;        // [tile][token block] arrival counters, zero between launches
+  const uint8_t* xq;   // [token block][K/128][NT tokens x 128 bytes, core-matrix layout]
+  const float* d;      // [ntb * NT] activation scales
+  const int32_t* sumq; // [ntb * NT]
   uint32_t* status;
 };
 
@@ -97,7 +102,7 @@ struct QuantParams {
   float* d;
   int32_t* sumq;
   float* act_scale;    // nullable user copy of d
-  int bbytes;          // bytes of one 128-wide K group of the tile: tokens per pass x 128
+  int bbytes;          // bytes of one 128-wide K group of a token block: NT x 128
 };
 
 __global__ void __launch_bounds__(256) quant_act_kernel(const __grid_constant__ QuantParams p) {
@@ -112,13 +117,15 @@ __global__ void __launch_bounds__(256) quant_act_kernel(const __grid_constant__ 
   pdl_wait();
   const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int K = p.K, nvec = K >> 2;
+  const int NT = p.bbytes >> 7, mt = m % NT;  // row of its token block
+  uint8_t* const xq = p.xq + (size_t)(m / NT) * (K >> 7) * p.bbytes;
   auto dst_of = [&](int i) {  // float4 index -> byte offset of its 4 int8 in the operand layout
     const int k = i << 2;
-    return (size_t)(k >> 7) * p.bbytes + (size_t)(m >> 3) * 1024 + (size_t)((k & 127) >> 4) * 128 +
-           (size_t)(m & 7) * 16 + (k & 15);
+    return (size_t)(k >> 7) * p.bbytes + (size_t)(mt >> 3) * 1024 + (size_t)((k & 127) >> 4) * 128 +
+           (size_t)(mt & 7) * 16 + (k & 15);
   };
   if (m >= p.M) {  // padding token of the tile
-    for (int i = tid; i < nvec; i += 256) *reinterpret_cast<uint32_t*>(p.xq + dst_of(i)) = 0u;
+    for (int i = tid; i < nvec; i += 256) *reinterpret_cast<uint32_t*>(xq + dst_of(i)) = 0u;
     if (tid == 0) {
       p.d[m] = 0.f;
       p.sumq[m] = 0;
@@ -175,7 +182,7 @@ __global__ void __launch_bounds__(256) quant_act_kernel(const __grid_constant__ 
     const int q0 = __float2int_rn(__fmul_rn(v.x, inv)), q1 = __float2int_rn(__fmul_rn(v.y, inv));
     const int q2 = __float2int_rn(__fmul_rn(v.z, inv)), q3 = __float2int_rn(__fmul_rn(v.w, inv));
     sumq += (q0 + q1) + (q2 + q3);
-    *reinterpret_cast<uint32_t*>(p.xq + dst_of(i)) =
+    *reinterpret_cast<uint32_t*>(xq + dst_of(i)) =
         (uint32_t)(q0 & 0xff) | ((uint32_t)(q1 & 0xff) << 8) | ((uint32_t)(q2 & 0xff) << 16) |
         ((uint32_t)q3 << 24);
   }
@@ -205,26 +212,29 @@ __device__ __forceinline__ void umma_i8_ta(uint32_t tmem_d, uint32_t tmem_a, uin
 }
 
 template <int NT>
-__global__ void __launch_bounds__(kMmaThreads + 96, 1)
+__global__ void __launch_bounds__(kMmaThreads + 128, 1)
     bitlinear_mma_kernel(const __grid_constant__ MmaParams p) {
   using Cfg = MmaCfg<NT>;
   constexpr int kStages = Cfg::kStages, kBBytes = Cfg::kBBytes;
-  constexpr int NCH = NT / 64;  // 32-token chunks an epilogue warp owns
+  constexpr int NCH = NT / 64;  // 16-token chunks an epilogue warp owns
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // this CTA's K range (split-K over 128-wide groups; a whole row when nsplit == 1)
-  const int tile = (int)blockIdx.x / p.nsplit, split = (int)blockIdx.x % p.nsplit;
+  const int tb = (int)blockIdx.x % p.ntb, ts = (int)blockIdx.x / p.ntb;
+  const int tile = ts / p.nsplit, split = ts % p.nsplit;
+  const int M = min(NT, p.M - tb * NT);  // tokens of this block
+  const uint8_t* const xq = p.xq + (size_t)tb * (p.K >> 7) * Cfg::kBBytes;
   const int gbase = split * p.gps;
   const int ngroups = min(p.gps, (p.K >> 7) - gbase);
   const int nchunks = (ngroups + kChunkGroups - 1) / kChunkGroups;
   const int nsteps = (ngroups + kStepGroups - 1) / kStepGroups;
-  constexpr int kExpWarps = kMmaThreads / 32;  // warps 0..7 expand, warp 8 issues MMAs, warp 9 copies
-  constexpr int kMmaWarp = kExpWarps, kCopyWarp = kExpWarps + 1;
+  constexpr int kExpWarps = kMmaThreads / 32;  // these expand; then MMA, copy, MMA, copy
+  constexpr int kMmaWarp = kExpWarps, kActWarp = kExpWarps + 1, kPkWarp = kExpWarps + 3;
 
   // control block, then the packed ring and the activation stages (1 KB aligned)
   uint64_t* pk_full = reinterpret_cast<uint64_t*>(smem);  // [kPkStages] box landed (tx bytes)
   uint64_t* pk_free = pk_full + kPkStages;                 // [kPkStages] every expander warp left it
-  uint64_t* full = pk_free + kPkStages;   // [kStages] A stored by 8 warps + B landed (tx bytes)
+  uint64_t* full = pk_free + kPkStages;   // [kStages] A stored by a group's 8 warps + B landed (tx bytes)
   uint64_t* mma_done = full + kStages;    // [kStages] the MMAs that read the stage have retired
   uint64_t* done = mma_done + kStages;    // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
@@ -235,20 +245,22 @@ __global__ void __launch_bounds__(kMmaThreads + 96, 1)
 
   // tile -> (segment, first row)
   int seg = 0;
+  if (!p.glu) {
 #pragma unroll
-  for (int s = 1; s < 4; ++s)
-    if (s < p.nseg && tile >= p.seg[s].tile0) seg = s;
+    for (int s = 1; s < 4; ++s)
+      if (s < p.nseg && tile >= p.seg[s].tile0) seg = s;
+  }
   const int seg_N = p.seg[seg].N;
-  const int row0 = (tile - p.seg[seg].tile0) * kMmaRows;
-  const int nrows = min(kMmaRows, seg_N - row0);
+  // a gate/up tile holds 64 gate rows and the 64 up rows of the same outputs
+  const int row0 = p.glu ? tile * 64 : (tile - p.seg[seg].tile0) * kMmaRows;
 
   if (tid == 0) {
     for (int i = 0; i < kPkStages; ++i) {
       mbar_init(&pk_full[i], 1);
-      mbar_init(&pk_free[i], kExpWarps);
+      mbar_init(&pk_free[i], kExpWarps);  // a box is two steps: one of each group
     }
     for (int i = 0; i < kStages; ++i) {
-      mbar_init(&full[i], kExpWarps + 1);
+      mbar_init(&full[i], 8 + 1);
       mbar_init(&mma_done[i], 1);
     }
     mbar_init(done, 2);
@@ -264,55 +276,44 @@ __global__ void __launch_bounds__(kMmaThreads + 96, 1)
   tc_after_sync();
   const uint32_t tmem = *tmem_slot;
   bool ok = true;
+  pdl_trigger();
 
-  if (warp == kCopyWarp) {
-    // ================= copy warp: packed weight boxes and activation tiles ==================
+  if (warp == kPkWarp) {
+    // ================= packed weight boxes: constant, so no wait on the previous kernel ==========
+    // A warp of its own: behind the activations' waits a box was only asked for when it was needed
+    // (K=6912 unsplit, 64 tokens: 37 us).
     const uint64_t pol = policy_evict_first();
     const CUtensorMap* tm = &p.tmap[seg];
-    int cnext = 0;
-    if (lane == 0) {
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tm)) : "memory");
-      for (; cnext < kPkStages && cnext < nchunks; ++cnext) {  // weights: no dependency
-        mbar_arrive_expect_tx(&pk_full[cnext], kPkBytes);
-        tc_tma_box_2d(pk + (size_t)cnext * kPkBytes, tm, (gbase + cnext * kChunkGroups) * 32, row0,
-                   &pk_full[cnext], pol);
+    const CUtensorMap* tm1 = p.glu ? &p.tmap[1] : tm;
+    const int row1 = p.glu ? row0 : row0 + 64;
+    TcRing<kPkStages> r;
+    for (int c = 0; c < nchunks; ++c, r.advance()) {
+      ok = tc_wait_w(&pk_free[r.i], r.phase ^ 1, p.status);
+      if (!ok) break;
+      if (tc_elect()) {  // two halves of 64 rows
+        uint8_t* dst = pk + (size_t)r.i * kPkBytes;
+        const int x = (gbase + c * kChunkGroups) * 32;
+        mbar_arrive_expect_tx(&pk_full[r.i], kPkBytes);
+        tc_tma_box_2d(dst, tm, x, row0, &pk_full[r.i], pol);
+        tc_tma_box_2d(dst + kPkBytes / 2, tm1, x, row1, &pk_full[r.i], pol);
       }
+      __syncwarp();
     }
-    cnext = min(kPkStages, nchunks);
-    pdl_trigger();
-    pdl_wait();  // the quantised activations come from the kernel before this one
-    for (int s = 0; s < nsteps; ++s) {
-      const int st = s % kStages;
-      if (s >= kStages)  // the MMAs that read this stage kStages steps ago must have retired
-        ok = tc_wait(ok, &mma_done[st], (uint32_t)(((s / kStages) - 1) & 1), p.status);
-      if (lane == 0) {  // activations of the step's groups: contiguous in the operand layout
+  } else if (warp == kActWarp) {
+    // ================= activation tiles: written by the kernel before this one ===================
+    pdl_wait();
+    TcRing<kStages> r;
+    for (int s = 0; s < nsteps; ++s, r.advance()) {
+      ok = tc_wait_w(&mma_done[r.i], r.phase ^ 1, p.status);  // the MMAs that read the stage last
+      if (!ok) break;
+      if (tc_elect()) {  // the step's groups are contiguous in the operand layout
         const int g0 = s * kStepGroups;
         const uint32_t bytes = (uint32_t)min(kStepGroups, ngroups - g0) * kBBytes;
-        mbar_arrive_expect_tx(&full[st], bytes);
-        bulk_g2s(bstg + (size_t)st * kStepGroups * kBBytes, p.xq + (size_t)(gbase + g0) * kBBytes, bytes,
-                 &full[st]);
+        mbar_arrive_expect_tx(&full[r.i], bytes);
+        bulk_g2s(bstg + (size_t)r.i * kStepGroups * kBBytes, xq + (size_t)(gbase + g0) * kBBytes, bytes,
+                 &full[r.i]);
       }
-      // refill the packed ring as soon as every expander warp has left the oldest box
-      if (cnext < nchunks && mbar_try_wait(&pk_free[cnext % kPkStages],
-                                           (uint32_t)(((cnext / kPkStages) - 1) & 1))) {
-        if (lane == 0) {
-          mbar_arrive_expect_tx(&pk_full[cnext % kPkStages], kPkBytes);
-          tc_tma_box_2d(pk + (size_t)(cnext % kPkStages) * kPkBytes, tm,
-                     (gbase + cnext * kChunkGroups) * 32, row0, &pk_full[cnext % kPkStages], pol);
-        }
-        ++cnext;
-      }
-    }
-    while (cnext < nchunks) {  // boxes still owed (their slot frees up as the expanders go)
-      ok = tc_wait(ok, &pk_free[cnext % kPkStages], (uint32_t)(((cnext / kPkStages) - 1) & 1),
-                    p.status);
-      if (!ok) break;
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&pk_full[cnext % kPkStages], kPkBytes);
-        tc_tma_box_2d(pk + (size_t)(cnext % kPkStages) * kPkBytes, tm,
-                   (gbase + cnext * kChunkGroups) * 32, row0, &pk_full[cnext % kPkStages], pol);
-      }
-      ++cnext;
+      __syncwarp();
     }
   } else if (warp == kMmaWarp || warp == kMmaWarp + 2) {
     // ================= two MMA warps: even steps -> accumulator 0, odd steps -> accumulator 1
@@ -321,7 +322,7 @@ __global__ void __launch_bounds__(kMmaThreads + 96, 1)
     if (tc_elect()) {
       for (int s = which; s < nsteps; s += 2) {
         const int st = s % kStages;
-        ok = tc_wait(ok, &full[st], (uint32_t)((s / kStages) & 1), p.status);
+        ok = ok && tc_wait_w(&full[st], (uint32_t)((s / kStages) & 1), p.status);
         tc_after_sync();
         const uint32_t a_t = tmem + Cfg::kA0 + (uint32_t)st * (kStepGroups * kAGroupCols);
         const uint32_t bbase = smem_u32(bstg + (size_t)st * kStepGroups * kBBytes);
@@ -342,25 +343,26 @@ __global__ void __launch_bounds__(kMmaThreads + 96, 1)
     __syncwarp();
   } else {
     // ================= expander warps ========================================================
-    // warp w owns TMEM lanes (= weight rows) 32*(w&3).., and K-half h = w>>2 of every group:
-    // planes 2h and 2h+1 of the packed bytes = K bytes 64h..64h+63 = 16 columns.
-    const int q = warp & 3, h = warp >> 2;
-    const int erow = q * 32 + lane;
+    // warp w of a group owns TMEM lanes (= weight rows) 32*(w&3).., and K-half h = w>>2 of every
+    // 128-wide group: planes 2h and 2h+1 of the packed bytes = K bytes 64h..64h+63 = 16 columns.
+    static_assert(kExpGroups * kStepGroups == kChunkGroups, "a box is one step of every group");
+    const int q = warp & 3, h = (warp >> 2) & 1, grp = warp >> 3;
+    // row of the box that this lane expands: a gate/up tile has 16 gate rows and the 16 up rows
+    // of the same outputs in every lane quarter
+    const int erow = p.glu ? (lane & 15) + 16 * q + (lane >> 4) * 64 : q * 32 + lane;
     const uint32_t lane_addr = tmem + ((uint32_t)(q * 32) << 16) + Cfg::kA0 + 16u * h;
-    for (int s = 0; s < nsteps; ++s) {
-      const int st = s % kStages;
+    for (int s = grp; s < nsteps; s += kExpGroups) {
+      const int st = s % kStages, c = s / kExpGroups;
       if (s >= kStages) {
-        ok = tc_wait(ok, &mma_done[st], (uint32_t)(((s / kStages) - 1) & 1), p.status);
+        ok = ok && tc_wait_w(&mma_done[st], (uint32_t)(((s / kStages) - 1) & 1), p.status);
         tc_after_sync();
       }
+      ok = ok && tc_wait_w(&pk_full[c % kPkStages], (uint32_t)((c / kPkStages) & 1), p.status);
       const int ng = min(kStepGroups, ngroups - s * kStepGroups);
 #pragma unroll
       for (int gg = 0; gg < kStepGroups; ++gg) {
         if (gg >= ng) break;
-        const int g = s * kStepGroups + gg;
-        const int c = g / kChunkGroups, gi = g % kChunkGroups;
-        if (gi == 0)
-          ok = tc_wait(ok, &pk_full[c % kPkStages], (uint32_t)((c / kPkStages) & 1), p.status);
+        const int gi = grp * kStepGroups + gg;  // group of the box
         // the row's 32 packed bytes of this group: units 2gi and 2gi+1 of its swizzled 128 bytes
         const uint8_t* rowp = pk + (size_t)(c % kPkStages) * kPkBytes + (size_t)erow * 128;
         const uint4 w0 = *reinterpret_cast<const uint4*>(rowp + (((2 * gi) ^ (erow & 7)) << 4));
@@ -383,47 +385,40 @@ __global__ void __launch_bounds__(kMmaThreads + 96, 1)
             "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]),
             "r"(o[15])
             : "memory");
-        if (gi == kChunkGroups - 1 || g == ngroups - 1) {  // last read of this packed box
-          __syncwarp();
-          if (lane == 0)
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(
-                             smem_u32(&pk_free[c % kPkStages]))
-                         : "memory");
-        }
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&pk_free[c % kPkStages]);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_before_sync();
       __syncwarp();
-      if (lane == 0)
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[st]))
-                     : "memory");
+      if (lane == 0) mbar_arrive(&full[st]);
     }
     pdl_wait();  // d and sum(q) come from the quantiser
     if (tid < NT) {
-      sd[tid] = p.d[tid];
-      ssum[tid] = p.sumq[tid];
+      sd[tid] = p.d[tb * NT + tid];
+      ssum[tid] = p.sumq[tb * NT + tid];
     }
   }
   ok = tc_wait(true, done, 0, p.status) && ok;
   tc_after_sync();
   __syncthreads();  // sd / ssum visible; every warp past its loop
 
-  // ---- epilogue: TMEM lane = weight row, column = token.  Warps w and w + 4 share a lane
-  //      quarter; a warp owns the 32-token chunks (w >> 2), (w >> 2) + 2, ... ----------------
+  // ---- epilogue: TMEM lane = weight row, column = token.  Warps w, w + 4, w + 8, w + 12 share a
+  //      lane quarter; a warp owns the 16-token chunks (w >> 2), (w >> 2) + 4, ... -------------
   const int q = warp & 3, half = warp >> 2;  // lane quarter, first chunk (expander warps only)
   const int r = q * 32 + lane;
-  uint32_t v[NCH][32];
+  uint32_t v[NCH][16];
   if (warp < kExpWarps) {
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
-      const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((half + 2 * c) * 32);
-      HB_TMEM_LD32(v[c], taddr);
+      const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((half + 4 * c) * 16);
+      HB_TMEM_LD16(v[c], taddr);
       if (nsteps > 1) {  // the second MMA warp's accumulator
-        uint32_t u[32];
-        HB_TMEM_LD32(u, taddr + (uint32_t)Cfg::kAcc1);
+        uint32_t u[16];
+        HB_TMEM_LD16(u, taddr + (uint32_t)Cfg::kAcc1);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int t = 0; t < 32; ++t) v[c][t] += u[t];
+        for (int t = 0; t < 16; ++t) v[c][t] += u[t];
       } else {
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       }
@@ -435,22 +430,23 @@ __global__ void __launch_bounds__(kMmaThreads + 96, 1)
   bool finish = true;
   if (p.nsplit > 1) {
     __shared__ int s_last;
-    int32_t* mine = p.part + ((size_t)(tile * p.nsplit + split) * NT) * kMmaRows;
+    const int tk = tile * p.ntb + tb;
+    int32_t* mine = p.part + ((size_t)(tk * p.nsplit + split) * NT) * kMmaRows;
     if (warp < kExpWarps) {
 #pragma unroll
       for (int c = 0; c < NCH; ++c) {
-        const int m0 = (half + 2 * c) * 32;
-        if (m0 >= p.M) continue;
+        const int m0 = (half + 4 * c) * 16;
+        if (m0 >= M) continue;
 #pragma unroll
-        for (int t = 0; t < 32; ++t) mine[(size_t)(m0 + t) * kMmaRows + r] = (int32_t)v[c][t];
+        for (int t = 0; t < 16; ++t) mine[(size_t)(m0 + t) * kMmaRows + r] = (int32_t)v[c][t];
       }
     }
     __threadfence();
     __syncthreads();
     if (tid == 0) {
-      const int t = atomicAdd(&p.tickets[tile], 1);
+      const int t = atomicAdd(&p.tickets[tk], 1);
       s_last = (t == p.nsplit - 1);
-      if (s_last) p.tickets[tile] = 0;  // every split has arrived: ready for the next launch
+      if (s_last) p.tickets[tk] = 0;  // every split has arrived: ready for the next launch
     }
     __syncthreads();
     finish = s_last != 0;
@@ -458,55 +454,72 @@ __global__ void __launch_bounds__(kMmaThreads + 96, 1)
       __threadfence();
 #pragma unroll
       for (int c = 0; c < NCH; ++c) {
-        const int m0 = (half + 2 * c) * 32;
-        if (m0 >= p.M) continue;
+        const int m0 = (half + 4 * c) * 16;
+        if (m0 >= M) continue;
         for (int s2 = 0; s2 < p.nsplit; ++s2) {
           if (s2 == split) continue;
-          const int32_t* other = p.part + ((size_t)(tile * p.nsplit + s2) * NT + m0) * kMmaRows + r;
+          const int32_t* other = p.part + ((size_t)(tk * p.nsplit + s2) * NT + m0) * kMmaRows + r;
 #pragma unroll
-          for (int t = 0; t < 32; ++t) v[c][t] += (uint32_t)__ldcg(other + (size_t)t * kMmaRows);
+          for (int t = 0; t < 16; ++t) v[c][t] += (uint32_t)__ldcg(other + (size_t)t * kMmaRows);
         }
       }
     }
   }
 
   if (finish && warp < kExpWarps) {
-    const float ws = __ldg(p.seg[seg].scale);
+    const bool up = p.glu && lane >= 16;
+    const int row = p.glu ? row0 + 16 * q + (lane & 15) : row0 + r;
+    const bool row_ok = ok && row < seg_N;
+    const float ws = __ldg(p.seg[up ? 1 : seg].scale);
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
-      const int m0 = (half + 2 * c) * 32;
-      if (r < nrows && ok && m0 < p.M) {
-        const int mcount = min(32, p.M - m0);
-        const size_t o0 = (size_t)m0 * seg_N + row0 + r;
-        float* yp = p.seg[seg].y + o0;
-        const float* rp = p.seg[seg].residual ? p.seg[seg].residual + o0 : nullptr;
-        int32_t* ap = p.seg[seg].acc ? p.seg[seg].acc + o0 : nullptr;
-        // all shared-memory reads first (v[t] becomes the integer total), so that the stores
-        // below, whose target the compiler cannot tell from shared memory, do not serialise them
-        float dsc[32];
+      const int m0 = (half + 4 * c) * 16;
+      if (m0 >= M) continue;  // the same for the whole warp
+      const int mcount = min(16, M - m0);
+      const size_t o0 = (size_t)(tb * NT + m0) * seg_N + row;
+      float* yp = p.seg[seg].y + o0;
+      const float* rp = p.seg[seg].residual ? p.seg[seg].residual + o0 : nullptr;
+      int32_t* ap = p.seg[seg].acc ? p.seg[seg].acc + o0 : nullptr;
+      // all shared-memory reads first (v[t] becomes the integer total), so that the stores
+      // below, whose target the compiler cannot tell from shared memory, do not serialise them
+      float dsc[16];
 #pragma unroll
-        for (int t = 0; t < 32; ++t) {
-          v[c][t] = (uint32_t)((int)v[c][t] - ssum[m0 + t]);
-          dsc[t] = sd[m0 + t];
-        }
-        if (ap) {
-#pragma unroll
-          for (int t = 0; t < 32; ++t)
-            if (t < mcount) ap[(size_t)t * seg_N] = (int)v[c][t];
-        }
-        float res[32];
-        if (rp) {
-#pragma unroll
-          for (int t = 0; t < 32; ++t) res[t] = t < mcount ? rp[(size_t)t * seg_N] : 0.f;
-        }
-#pragma unroll
-        for (int t = 0; t < 32; ++t)
-          if (t < mcount) {
-            float y = __fmul_rn(__fmul_rn((float)(int)v[c][t], dsc[t]), ws);
-            if (rp) y = __fadd_rn(y, res[t]);
-            yp[(size_t)t * seg_N] = y;
-          }
+      for (int t = 0; t < 16; ++t) {
+        v[c][t] = (uint32_t)((int)v[c][t] - ssum[m0 + t]);
+        dsc[t] = sd[m0 + t];
       }
+      if (p.glu) {
+        // gate lanes finish the even tokens, up lanes (16 further) the odd ones
+#pragma unroll
+        for (int t = 0; t < 16; t += 2) {
+          const float a = __fmul_rn(__fmul_rn((float)(int)v[c][t], dsc[t]), ws);
+          const float b = __fmul_rn(__fmul_rn((float)(int)v[c][t + 1], dsc[t + 1]), ws);
+          const float got = __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+          const float gt = up ? got : a, rl = gt > 0.f ? gt : 0.f;
+          const float y = __fmul_rn(__fmul_rn(rl, rl), up ? b : got);
+          const int tt = up ? t + 1 : t;
+          if (row_ok && tt < mcount) yp[(size_t)tt * seg_N] = y;
+        }
+        continue;
+      }
+      if (!row_ok) continue;
+      if (ap) {
+#pragma unroll
+        for (int t = 0; t < 16; ++t)
+          if (t < mcount) ap[(size_t)t * seg_N] = (int)v[c][t];
+      }
+      float res[16];
+      if (rp) {
+#pragma unroll
+        for (int t = 0; t < 16; ++t) res[t] = t < mcount ? rp[(size_t)t * seg_N] : 0.f;
+      }
+#pragma unroll
+      for (int t = 0; t < 16; ++t)
+        if (t < mcount) {
+          float y = __fmul_rn(__fmul_rn((float)(int)v[c][t], dsc[t]), ws);
+          if (rp) y = __fadd_rn(y, res[t]);
+          yp[(size_t)t * seg_N] = y;
+        }
     }
   }
   tc_before_sync();
@@ -519,46 +532,60 @@ __global__ void __launch_bounds__(kMmaThreads + 96, 1)
 
 using namespace hb;
 
-// Batched path of hb200_bitlinear_forward_multi (16 <= M <= 128: one pass of 64 or 128 token
-// slots).  Scratch in the context: quantised activations in operand layout, their scales and
-// sums.
+// How a launch is dealt: token blocks of NT, K ranges per tile.  A block of 64 tokens more costs
+// only its own CTA (the weights come from L2), so it is preferred until the CTAs need a second
+// wave; cutting K pays for few tiles with a long K alone, partials and their fence cost 2 to 4
+// us.  Measured (us, quantiser included; block/K ranges): K=2560 N=2560 at 128 tokens 64/1 9.0, 64/2
+// 10.5, 128/1 10.8, 128/5 15.5; K=6912 N=2560 at 128 tokens 64/1 16.7, 64/3 15.0, 128/2 17.8, at 256
+// 64/1 19.4, 128/2 22.3; K=2560 N=6912 gate/up at 128 tokens 64/1 (216 CTAs) 16.1, 128/1 11.0.  The
+// cost below is in cycles, fitted to these.
+struct BlDeal {
+  int NT, ntb, nsplit, gps;
+};
+static BlDeal bl_deal(const hb200_ctx* ctx, int tiles, int ngroups, int M) {
+  BlDeal best = {};
+  long best_cost = 0;
+  for (int NT = 64; NT <= (M > 64 ? 128 : 64); NT *= 2) {
+    const int ntb = (M + NT - 1) / NT;
+    for (int ns = 1; ns <= (ngroups >= 8 ? ngroups / 4 : 1); ++ns) {  // at least two steps each
+      const long ctas = (long)tiles * ntb * ns;
+      if (ns > 1 && (ctas > ctx->sm_count || tiles * ntb > kCtxTickets ||
+                     (size_t)ctas * NT * kMmaRows * 4 > kScratchBytes - kScratchSplitK))
+        break;
+      const int gps = (ngroups + ns - 1) / ns;
+      const long waves = (ctas + ctx->sm_count - 1) / ctx->sm_count;
+      const long cost = waves * (4500 + 220L * gps + (NT == 128 ? 3500 : 0)) +
+                        (ns > 1 ? 4500 + 11L * ns * NT : 0);
+      if (best.NT == 0 || cost < best_cost) {
+        best_cost = cost;
+        best = {NT, ntb, (ngroups + gps - 1) / gps, gps};  // no empty split
+      }
+    }
+  }
+  return best;
+}
+
 template <int NT>
 static int bl_mma_launch(hb200_ctx* ctx, MmaParams& p, int tiles, cudaStream_t st) {
-  // split-K when the tiles alone leave most SMs idle: as many splits as fit the SMs, each at
-  // least 4 groups (two pipeline steps) long, partials within their scratch region
-  const int ngroups = p.K / 128;
-  int nsplit = ctx->sm_count / tiles;
-  if (nsplit > ngroups / 4) nsplit = ngroups / 4;
-  while (nsplit > 1 &&
-         (size_t)tiles * nsplit * NT * kMmaRows * 4 > kScratchBytes - kScratchSplitK)
-    --nsplit;
-  if (nsplit < 1 || tiles > kCtxTickets) nsplit = 1;
-  p.gps = (ngroups + nsplit - 1) / nsplit;
-  p.nsplit = (ngroups + p.gps - 1) / p.gps;  // no empty split
   const int rc = hb_func_smem(ctx, reinterpret_cast<const void*>(bitlinear_mma_kernel<NT>),
                               (size_t)MmaCfg<NT>::kSmem);
   if (rc != HB200_OK) return rc;
-  HB_CUDA(launch_pdl(bitlinear_mma_kernel<NT>, dim3(tiles * p.nsplit), dim3(kMmaThreads + 96),
+  HB_CUDA(launch_pdl(bitlinear_mma_kernel<NT>, dim3(tiles * p.nsplit * p.ntb), dim3(kMmaThreads + 128),
                      (size_t)MmaCfg<NT>::kSmem, st, ctx->pdl, p));
   return HB200_OK;
 }
 
-int hb_bitlinear_mma_run(hb200_ctx* ctx, const hb200_bitlinear_seg* segs, int nseg, int K,
+// Batched path of the ternary products: 1 <= M <= kBlMmaTokens tokens in one launch of the
+// quantiser and one of the product.  glu: two tensors of equal shape, gate and up, and segs[0].d_y
+// = relu(gate)^2 * up.  Scratch in the context: quantised activations in operand layout, their
+// scales and sums, split-K partials.
+int hb_bitlinear_mma_run(hb200_ctx* ctx, const hb200_bitlinear_seg* segs, int nseg, int K, int glu,
                          const float* d_x, int M, const float* d_rms_gamma, float rms_eps,
                          float* d_act_scale, cudaStream_t st) {
   ScratchUse use(ctx, st);  // quantised activation tiles, split-K partials, tickets
-  HB_REQUIRE(M >= 1 && M <= 128, "bitlinear (batched): %d tokens in one pass (at most 128)", M);
-  const int NT = M <= 64 ? 64 : 128;
-  const size_t xq_bytes = (size_t)(K / 128) * NT * 128;
-  HB_REQUIRE(xq_bytes + 1024 <= kScratchGlu,
-             "bitlinear (batched): K=%d needs %zu bytes of activation scratch", K, xq_bytes);
-  uint8_t* base = static_cast<uint8_t*>(ctx->d_scratch);
-  float* d = reinterpret_cast<float*>(base);            // [128]
-  int32_t* sumq = reinterpret_cast<int32_t*>(base + 512);  // [128]
-  uint8_t* xq = base + 1024;
-  QuantParams q = {d_x, d_rms_gamma, rms_eps, K, M, xq, d, sumq, d_act_scale, NT * 128};
-  HB_CUDA(launch_pdl(quant_act_kernel, dim3(NT), dim3(256), (size_t)K * sizeof(float), st,
-                     ctx->pdl, q));
+  HB_REQUIRE(M >= 1 && M <= kBlMmaTokens, "bitlinear (batched): %d tokens in one pass (at most %d)", M,
+             kBlMmaTokens);
+  HB_REQUIRE(!glu || (nseg == 2 && segs[0].N == segs[1].N), "bitlinear (batched): gate and up differ in shape");
   MmaParams p = {};
   int t = 0;
   TcEncodeTiledFn encode = tc_tensor_map_encoder();
@@ -571,7 +598,7 @@ int hb_bitlinear_mma_run(hb200_ctx* ctx, const hb200_bitlinear_seg* segs, int ns
                "bitlinear (batched): packed weights must be 16-byte aligned");
     const cuuint64_t dims[2] = {(cuuint64_t)(K / 4), (cuuint64_t)segs[s].N};
     const cuuint64_t strides[1] = {(cuuint64_t)(K / 4)};  // bytes between rows
-    const cuuint32_t box[2] = {(cuuint32_t)(kChunkGroups * 32), (cuuint32_t)kMmaRows};
+    const cuuint32_t box[2] = {(cuuint32_t)(kChunkGroups * 32), (cuuint32_t)(kMmaRows / 2)};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult rc = encode(&p.tmap[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
                                const_cast<void*>(segs[s].d_packed), dims, strides, box, estr,
@@ -581,14 +608,30 @@ int hb_bitlinear_mma_run(hb200_ctx* ctx, const hb200_bitlinear_seg* segs, int ns
     HB_REQUIRE(rc == CUDA_SUCCESS, "bitlinear (batched): cuTensorMapEncodeTiled failed (%d)",
                (int)rc);
   }
+  if (glu) t = (segs[0].N + kMmaRows / 2 - 1) / (kMmaRows / 2);
+  const BlDeal deal = bl_deal(ctx, t, K / 128, M);
+  const int slots = deal.ntb * deal.NT;  // token slots, padding included
+  HB_REQUIRE(4096 + (size_t)slots * K <= kScratchLmSplit,
+             "bitlinear (batched): K=%d needs %zu bytes of activation scratch", K, (size_t)slots * K);
+  uint8_t* base = static_cast<uint8_t*>(ctx->d_scratch);
+  float* d = reinterpret_cast<float*>(base);                // [kBlMmaTokens]
+  int32_t* sumq = reinterpret_cast<int32_t*>(base + 2048);  // [kBlMmaTokens]
+  uint8_t* xq = base + 4096;
+  QuantParams q = {d_x, d_rms_gamma, rms_eps, K, M, xq, d, sumq, d_act_scale, deal.NT * 128};
+  HB_CUDA(launch_pdl(quant_act_kernel, dim3(slots), dim3(256), (size_t)K * sizeof(float), st,
+                     ctx->pdl, q));
   p.nseg = nseg;
   p.K = K;
   p.M = M;
+  p.glu = glu;
+  p.ntb = deal.ntb;
+  p.nsplit = deal.nsplit;
+  p.gps = deal.gps;
   p.part = reinterpret_cast<int32_t*>(base + kScratchSplitK);
   p.tickets = ctx->d_tickets;
   p.xq = xq;
   p.d = d;
   p.sumq = sumq;
   p.status = ctx->d_status;
-  return NT == 64 ? bl_mma_launch<64>(ctx, p, t, st) : bl_mma_launch<128>(ctx, p, t, st);
+  return deal.NT == 64 ? bl_mma_launch<64>(ctx, p, t, st) : bl_mma_launch<128>(ctx, p, t, st);
 }

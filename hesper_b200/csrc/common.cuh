@@ -216,9 +216,10 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 
 }  // namespace hb
 
-// batched (16..64 token) ternary path on the tensor cores, bitlinear_mma.cu
+// batched ternary path on the tensor cores (16 tokens or more), bitlinear_mma.cu
+constexpr int kBlMmaTokens = 512;  // most tokens of one call
 int hb_bitlinear_mma_run(struct hb200_ctx* ctx, const hb200_bitlinear_seg* segs, int nseg, int K,
-                         const float* d_x, int M, const float* d_rms_gamma, float rms_eps,
+                         int glu, const float* d_x, int M, const float* d_rms_gamma, float rms_eps,
                          float* d_act_scale, cudaStream_t st);
 
 // batched (16..64 token) LM head on the tensor cores, lmhead_mma.cu
@@ -229,8 +230,7 @@ int hb_lmhead_mma_run(struct hb200_ctx* ctx, const void* d_table, int dtype, lon
 // Layout of the context's device scratch (one stream at a time uses it; regions of ops that
 // never overlap in time may overlap in space):
 constexpr size_t kScratchBytes = (size_t)56 << 20;
-constexpr size_t kScratchActs = 0;                     // batched ternary: d[64], sumq[64], int8 tiles
-constexpr size_t kScratchGlu = (size_t)2 << 20;       // batched gate/up products before the GLU
+constexpr size_t kScratchActs = 0;                     // batched ternary: d[512], sumq[512], int8 tiles
 constexpr size_t kScratchLmSplit = (size_t)8 << 20;   // 16-bit products: hi/lo activation tiles
 constexpr size_t kScratchRowScale = ((size_t)16 << 20) - 4096;  // f16 products: one power-of-two
                                                        // scale per staged activation row
