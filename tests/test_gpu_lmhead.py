@@ -130,3 +130,27 @@ def test_full_vocabulary_shape(ctx, oracle):
         top = np.sort(ref)[-2:]
         if top[1] - top[0] > TOL * scale:
             assert arg[m] == int(np.argmax(ref))
+
+
+@pytest.mark.parametrize("M,K,dtype", [(20, 64, 0), (32, 192, 1), (40, 192, 0), (64, 128, 1)])
+def test_several_rounds_of_row_tiles(ctx, M, K, dtype):
+    """More 128-row tiles than tensor memory holds accumulators for (8 at up to 32 tokens, 4 beyond)
+    on every SM, and K of an odd number of 64-wide blocks.  The first maximum sits in the last,
+    ragged tile for one token and ties with an earlier round for another.  With an f16 table one
+    token's activations lie far above f16's largest value, another's below its smallest normal."""
+    V = 148 * 9 * 128 + 77
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    table = (0.02 * torch.randn(V, K, device="cuda", generator=gen)).to(torch.float16 if dtype else torch.bfloat16)
+    x = torch.randn(M, K, device="cuda", generator=gen)
+    table[V - 1] = (0.5 * x[0]).to(table.dtype)
+    table[V // 2] = table[V // 3] = (0.5 * x[1]).to(table.dtype)
+    x[2] *= 1e6
+    x[3] *= 1e-7
+    logits, arg = _run(ctx, table.view(torch.int16).cpu().numpy().view(np.uint16), dtype, x.cpu().numpy(), None, 0.0)
+    ref = (x.double() @ table.double().T).cpu().numpy()
+    # x - hi - lo is at most 2^-18 |x| (two bf16 roundings); as much again for the f32 sums.  The
+    # planted rows are 25 times longer than the others, so the bound is per logit
+    bound = 2.0 ** -17 * (x.abs().double() @ table.abs().double().T).cpu().numpy()
+    assert np.all(np.abs(logits - ref) <= bound)
+    assert arg[0] == V - 1 and arg[1] == V // 3
+    assert np.array_equal(arg, np.argmax(logits, axis=1))
