@@ -691,6 +691,57 @@ static int attn_launch(hb200_ctx* ctx, const AttnParams& p, cudaStream_t st) {
   }
 }
 
+// Clusters of ns CTAs of the decode kernel that the GPU holds at once (a cluster lives in one GPC,
+// whose SMs bound it), asked for once per context.  0: unknown.
+template <int D, bool PRECISE>
+static int attn_clusters_at_once(hb200_ctx* ctx, int ns) {
+  constexpr int kStages = D >= 256 ? 3 : 4;  // as attn_launch picks them for a grid of one wave
+  using Cfg = AttnCfg<D, kStages>;
+  const void* kern = reinterpret_cast<const void*>(attn_decode_kernel<D, PRECISE, kStages>);
+  int16_t& known = ctx->attn_clusters[PRECISE][D >= 256 ? 2 : (D >= 128 ? 1 : 0)][ns];
+  if (known == 0) {
+    const size_t smem = (size_t)Cfg::kSmem + (D <= 128 ? (size_t)ns * 8 * (D + 2) * sizeof(float) : 0);
+    int n = 0;
+    bool ok = smem <= (size_t)ctx->smem_optin && hb_func_smem(ctx, kern, smem) == HB200_OK;
+    if (ok && !hb_func_flag(ctx, kern)) {
+      ok = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+      if (ok) hb_func_set_flag(ctx, kern);
+    }
+    if (ok) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)ns);
+      cfg.blockDim = dim3(kAttnThreads);
+      cfg.dynamicSmemBytes = smem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)ns;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      ok = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess;
+    }
+    if (!ok) {
+      cudaGetLastError();  // clear the last-error slot
+      n = 0;
+    }
+    known = (int16_t)(n > 0 ? n : -1);
+  }
+  return known > 0 ? known : 0;
+}
+
+// The most splits (2 to `most`) whose clusters all run at once, 0 if there are none.
+static int attn_one_wave_splits(hb200_ctx* ctx, int D, bool precise, long pairs, int most) {
+  for (int ns = most; ns >= 2; --ns) {
+    if (pairs * ns > ctx->sm_count || (ctx->attn_cluster_refused >> ns & 1u)) continue;
+    const int n = D == 64    ? (precise ? attn_clusters_at_once<64, true>(ctx, ns) : attn_clusters_at_once<64, false>(ctx, ns))
+                  : D == 128 ? (precise ? attn_clusters_at_once<128, true>(ctx, ns) : attn_clusters_at_once<128, false>(ctx, ns))
+                             : (precise ? attn_clusters_at_once<256, true>(ctx, ns) : attn_clusters_at_once<256, false>(ctx, ns));
+    if (n >= pairs) return ns;
+  }
+  return 0;
+}
+
 template <int D, bool PRECISE, int NSTAGES>
 static int attn_launch_ns(hb200_ctx* ctx, const AttnParams& p, cudaStream_t st) {
   using Cfg = AttnCfg<D, NSTAGES>;
@@ -815,11 +866,21 @@ static int attn_run(hb200_ctx* ctx, const void* d_q, int q_is_f16, const void* d
   // split stays short (<= 48 chunks of 16 positions), measured: 8000 positions in 16 splits +
   // cluster 12.9 us against 62 splits + ticket 17.6 us, 32768 positions 30.8 against 20.0 us.
   const bool short_splits = p.nsplit <= 16 || (eff_len + kChunk - 1) / kChunk <= 16 * 48;
-  if (p.nsplit > 1 && short_splits &&
-      (long)B * Hkv * (p.nsplit < 16 ? p.nsplit : 16) <= 2L * ctx->sm_count &&
-      ctx->attn_mode != HB200_ATTN_EXACT) {
-    if (p.nsplit > 16) p.nsplit = 16;
-    p.cluster = D <= 128 ? 1 : 2;  // D = 256: the partials reuse the stage region (2 barriers)
+  if (p.nsplit > 1 && ctx->attn_mode != HB200_ATTN_EXACT) {
+    const long pairs = (long)B * Hkv;
+    const int most = p.nsplit < 16 ? p.nsplit : 16;
+    const bool small = short_splits && pairs * most <= 2L * ctx->sm_count;
+    // No more splits than run at once: a CTA's fixed cost (prologue, two merges, ~5 us) is paid
+    // once per wave, and a second wave of clusters holds few.  Measured, us, splits chosen so against
+    // before, D = 256: 8 pairs x 8192 positions 10 splits 17.9, 16 24.3; 16 x 4096 6 16.4, 16 27.8; 32 x
+    // 2048 4 15.1, 8 26.5; 64 x 8192 2 72.9, 5 82.7 (30 positions 6.3, 7.3); D = 128: 20 x 2100 6 8.5,
+    // 16 11.3.  Long splits need most of the SMs at work: the line is 60 %.
+    const int one = attn_one_wave_splits(ctx, D, ctx->attn_mode == HB200_ATTN_PRECISE, pairs, most);
+    const bool wave = one > 1 && (small || pairs * one * 10 >= 6L * ctx->sm_count);
+    if (wave || small) {
+      p.nsplit = wave ? one : most;
+      p.cluster = D <= 128 ? 1 : 2;  // D = 256: the partials reuse the stage region (2 barriers)
+    }
   }
   if (p.nsplit > 1) {
     const size_t po = (size_t)B * Hkv * p.nsplit * 8 * (size_t)D * sizeof(float);

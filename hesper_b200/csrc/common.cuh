@@ -287,6 +287,7 @@ struct hb200_ctx {
   bool scratch_used;
   int scratch_depth;            // nesting of ScratchUse on the calling thread
   uint32_t attn_cluster_refused;  // bit n: the driver refused a cluster of n attention CTAs
+  int16_t attn_clusters[2][3][17];  // [precise][D 64/128/256][n]: clusters of n that run at once, 0 not asked, -1 none
   void* attn_static_addr;         // device address of the built-in attention scratch array here
   bool adopted;                   // lives in the caller's own CUDA context: never switch devices
 };

@@ -69,6 +69,9 @@ def test_literal_fixture_padded(ctx):
     (1, 8, 2, 256, 512), (1, 8, 2, 256, 4096), (2, 8, 2, 256, 1000), (16, 8, 2, 256, 512),
     (1, 20, 5, 128, 2049), (3, 20, 5, 128, 77), (1, 8, 8, 64, 300), (2, 16, 2, 64, 1),
     (1, 8, 1, 128, 33), (4, 4, 2, 256, 17),
+    # splits cut to what runs at once as clusters: 10 or fewer, 4 or fewer, 2, none; D = 128, 64
+    (8, 4, 1, 256, 2500), (16, 4, 2, 256, 700), (32, 2, 2, 256, 520), (48, 2, 2, 256, 300),
+    (4, 5, 5, 128, 1400), (5, 8, 4, 64, 1300),
 ])
 @pytest.mark.parametrize("q_f16", [False, True])
 def test_shapes(ctx, oracle, B, H, Hkv, D, L, q_f16):
