@@ -75,6 +75,7 @@ SIGNATURES = {
     "hb200_bitlinear_forward_multi": (_i, [_vp, C.POINTER(BitLinearSeg), _i, _i, _vp, _i, _vp, _f, _vp, _vp]),
     "hb200_bitlinear_gateup_relu2": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _i, _vp, _f, _vp, _vp]),
     "hb200_kquant_forward": (_i, [_vp, _i, _vp, _i, _i, _vp, _i, _vp, _f, _vp, _vp, _vp]),
+    "hb200_kquant_few_tokens_plan": (_i, [_i, _i, C.POINTER(_i), _i, _i, _i, _i, _i] + 4 * [C.POINTER(_i)]),
     "hb200_kquant_forward_multi": (_i, [_vp, _i, C.POINTER(KQuantSeg), _i, _i, _vp, _i, _vp, _f, _vp]),
     "hb200_kquant_gateup_gelu": (_i, [_vp, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _f, _vp, _vp]),
     "hb200_kquant_forward_multi_pre": (_i, [_vp, _i, C.POINTER(KQuantSeg), _i, _i, _vp, _i, _vp, _vp,

@@ -17,7 +17,11 @@
 //     tensor-map box, plus a second one for the up rows of a gate/up pair -- and its fragments.
 //     The weights of the first stages are fetched before griddepcontrol.wait, under the staging
 //     kernel.  16 warps: one per 16-row tile and K group (warp = kg * tiles + tile, K group kg
-//     takes the super-blocks kg, kg + KG, ...); the K groups meet in shared memory in fixed order.
+//     takes the positions kg, kg + KG, ... of the CTA's walk); the K groups meet in shared memory in
+//     fixed order.
+//     A parity wait tells a slot's lap from the next one only, so whoever waits for a lap has to
+//     know that the one before has landed: every slot belongs to one K group (the ring's stages are
+//     a multiple of KG, the position decides the group), or the ring never wraps (sb_plan).
 //
 // What bounds it: instruction issue -- about 330 instructions per 16 rows x 256 weights at up to
 // 8 tokens, 520 at up to 15 (products, int -> float, scales) -- 2 to 3.5 us at K=2560 N=10240 --
@@ -42,6 +46,8 @@ struct SbSeg {
   int cta0, ctas;  // CTAs [cta0, cta0 + ctas) own this tensor's rows
   int rp;          // rows of a pass (gate/up: outputs)
   int tiles;       // 16-row tiles of a pass
+  int groups;      // K groups of warps
+  int stages;      // stages of this tensor's ring
 };
 
 struct SbParams {
@@ -49,7 +55,7 @@ struct SbParams {
   SbSeg seg[kSbMaxSeg];
   int nseg, gu;   // gu: segments 0 and 1 are gate and up; the result goes to segment 0's y
   int nsb, M;
-  int stages, wbytes;  // stages of the ring, bytes of a stage before its fragments
+  int wbytes;          // bytes of a stage before its fragments
   const uint8_t* xb;
   uint32_t* status;
 };
@@ -186,7 +192,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) kq_sb_kernel(const __grid_const
   uint64_t* empty = full + kSbMaxStages;               // [stages] the tile warps have read it
   float* part = reinterpret_cast<float*>(smem + kSbCtrl);
   uint8_t* ring = smem + kSbCtrl + Cfg::kPart;
-  const int S = p.stages, nsb = p.nsb;
+  const int nsb = p.nsb;
   const size_t stage_bytes = (size_t)p.wbytes + Cfg::kB;
 
   int si = 0;
@@ -196,7 +202,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) kq_sb_kernel(const __grid_const
       if (s < p.nseg && (int)blockIdx.x >= p.seg[s].cta0) si = s;
   }
   const SbSeg& sg = p.seg[si];
-  const int ci = (int)blockIdx.x - sg.cta0, rp = sg.rp, tiles = sg.tiles;
+  const int ci = (int)blockIdx.x - sg.cta0, rp = sg.rp, tiles = sg.tiles, S = sg.stages;
   const int r0 = (int)((long long)sg.N * ci / sg.ctas), r1 = (int)((long long)sg.N * (ci + 1) / sg.ctas);
   const int npass = (r1 - r0 + rp - 1) / rp;
   const int boxbytes = rp * kUnit, up_off = (boxbytes + 127) & ~127;
@@ -249,7 +255,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) kq_sb_kernel(const __grid_const
     }
   } else {
     // ================= products ===================================================================
-    const int KG = kSbWarps / tiles;  // K groups
+    const int KG = sg.groups;
     const int tile = warp % tiles, kg = warp / tiles;
     const bool active = kg < KG;
     const int g = lane >> 2, t = lane & 3;
@@ -267,8 +273,10 @@ __global__ void __launch_bounds__(kSbThreads, 1) kq_sb_kernel(const __grid_const
         const int ra = p.gu ? min(8 * tile + g, nrows - 1) : min(16 * tile + g, nrows - 1);
         const int rb = p.gu ? ra : min(16 * tile + g + 8, nrows - 1);
         const size_t oa = (size_t)ra * kUnit, ob = (size_t)rb * kUnit + (p.gu ? up_off : 0);
-        for (int sb = kg; sb < nsb; sb += KG) {
-          const int pos = ps * nsb + sb, lap = pos / S, st = pos - lap * S;
+        // first position of this pass that is this group's: pos % KG == kg
+        const int pos0 = ps * nsb, end = pos0 + nsb;
+        for (int pos = pos0 + (kg - pos0 % KG + KG) % KG; pos < end; pos += KG) {
+          const int lap = pos / S, st = pos - lap * S;
           ok = tc_wait(ok, &full[st], (uint32_t)(lap & 1), p.status);
           const uint8_t* w = ring + (size_t)st * stage_bytes;
           if constexpr (FMT == 12) sb_unit_q4k<NTL>(w + oa, w + ob, w + p.wbytes, lane, acc);
@@ -277,7 +285,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) kq_sb_kernel(const __grid_const
           if (lane == 0) mbar_arrive(&empty[st]);
         }
       }
-      // the K groups of a tile (at least two: tiles <= 8) meet in shared memory, in order
+      // the K groups of a tile meet in shared memory, in order
       if (active && kg > 0) {
 #pragma unroll
         for (int n = 0; n < NTL; ++n)
@@ -323,18 +331,88 @@ __global__ void __launch_bounds__(kSbThreads, 1) kq_sb_kernel(const __grid_const
 
 using namespace hb;
 
+// How the rows are dealt and how deep each tensor's ring is: host arithmetic only.
+struct SbPlan {
+  int grid, wbytes;    // bytes of a stage before its fragments, the same for every tensor
+  size_t smem;
+  int ctas[kSbMaxSeg], rp[kSbMaxSeg], tiles[kSbMaxSeg], groups[kSbMaxSeg], stages[kSbMaxSeg];
+  int total[kSbMaxSeg];  // positions of the longest walk: passes x super-blocks
+};
+
+// N: rows of the tensors (gu: gate and up).  False: shape not covered.
+static bool sb_plan(int fmt, int K, const int* N, int nseg, int gu, int M, int sms, int smem_optin, SbPlan* out) {
+  if (M < 2 || M > 15 || K < 256 || K % 256 || K > 65536 || nseg < 1 || nseg > kSbMaxSeg || sms < nseg) return false;
+  const int NTL = M <= 8 ? 1 : 2, nsb = K / 256;
+  const int unit = fmt == HB200_FMT_Q4_K ? 144 : 272;
+  const size_t bbytes = (size_t)NTL * (4096 + 512), part = (size_t)kSbWarps * NTL * 512;
+  SbPlan p = {};
+  const int work = gu ? 1 : nseg;  // tensors whose rows are dealt
+  // CTAs per tensor: one each, then always to the one with the most rows per CTA, down to 4 rows
+  for (int s = 0; s < work; ++s) p.ctas[s] = 1;
+  p.grid = work;
+  while (p.grid < sms) {
+    int b = 0;
+    for (int s = 1; s < work; ++s)
+      if ((long long)N[s] * p.ctas[b] > (long long)N[b] * p.ctas[s]) b = s;
+    if ((long long)N[b] <= 4ll * p.ctas[b]) break;
+    ++p.ctas[b];
+    ++p.grid;
+  }
+  const int cap = gu ? kSbRows / 2 : kSbRows;
+  for (int s = 0; s < work; ++s) {
+    const int most = (N[s] + p.ctas[s] - 1) / p.ctas[s], np = (most + cap - 1) / cap;
+    p.rp[s] = (most + np - 1) / np;
+    p.tiles[s] = gu ? (p.rp[s] + 7) / 8 : (p.rp[s] + 15) / 16;
+    p.total[s] = np * nsb;
+    const int wb = ((p.rp[s] * unit + 127) & ~127) * (gu ? 2 : 1);
+    if (wb > p.wbytes) p.wbytes = wb;
+  }
+  if ((size_t)smem_optin < kSbCtrl + part) return false;
+  const size_t stage = (size_t)p.wbytes + bbytes, fit = ((size_t)smem_optin - kSbCtrl - part) / stage;
+  const int S = fit > (size_t)kSbMaxStages ? kSbMaxStages : (int)fit;
+  if (S < 1) return false;
+  int most = 1;
+  for (int s = 0; s < work; ++s) {
+    int g = kSbWarps / p.tiles[s];
+    if (g > S) g = S;
+    if (g > p.total[s]) g = p.total[s];
+    p.groups[s] = g;
+    // a ring that wraps holds a whole number of laps of the groups: each slot is one group's
+    p.stages[s] = p.total[s] <= S ? p.total[s] : S - S % g;
+    if (p.stages[s] > most) most = p.stages[s];
+  }
+  for (int s = work; s < nseg; ++s) {  // the up tensor goes with the gate
+    p.ctas[s] = p.ctas[0], p.rp[s] = p.rp[0], p.tiles[s] = p.tiles[0];
+    p.groups[s] = p.groups[0], p.stages[s] = p.stages[0], p.total[s] = p.total[0];
+  }
+  p.smem = kSbCtrl + part + (size_t)most * stage;
+  *out = p;
+  return true;
+}
+
+extern "C" int hb200_kquant_few_tokens_plan(int fmt, int K, const int* N, int nseg, int gate_up, int M, int sms,
+                                            int smem, int* stages, int* groups, int* tiles, int* total) {
+  HB_REQUIRE(N && stages && groups && tiles && total && (fmt == HB200_FMT_Q4_K || fmt == HB200_FMT_Q8_0) &&
+                 (!gate_up || nseg == 2) && smem > 0,
+             "kquant (few-token plan): bad argument");
+  for (int s = 0; s < nseg; ++s) HB_REQUIRE(N[s] >= 1, "kquant (few-token plan): tensor %d has no rows", s);
+  SbPlan p;
+  if (!sb_plan(fmt, K, N, nseg, gate_up, M, sms, smem, &p)) return HB200_ERR_UNSUPPORTED;
+  for (int s = 0; s < nseg; ++s) {
+    stages[s] = p.stages[s];
+    groups[s] = p.groups[s];
+    tiles[s] = p.tiles[s];
+    total[s] = p.total[s];
+  }
+  return HB200_OK;
+}
+
 template <int FMT, int NTL>
-static int sb_launch(hb200_ctx* ctx, SbParams& p, int grid, int max_total, cudaStream_t st) {
-  using Cfg = SbCfg<FMT, NTL>;
-  const size_t stage = (size_t)p.wbytes + Cfg::kB;
-  size_t S = ((size_t)ctx->smem_optin - kSbCtrl - Cfg::kPart) / stage;
-  if (S > (size_t)kSbMaxStages) S = kSbMaxStages;
-  if (S > (size_t)max_total) S = max_total;
-  p.stages = (int)S;
-  const size_t smem = kSbCtrl + Cfg::kPart + S * stage;
-  const int rc = hb_func_smem(ctx, reinterpret_cast<const void*>(kq_sb_kernel<FMT, NTL>), smem);
+static int sb_launch(hb200_ctx* ctx, const SbParams& p, const SbPlan& plan, cudaStream_t st) {
+  static_assert(SbCfg<FMT, NTL>::kB == NTL * 4608 && SbCfg<FMT, NTL>::kPart == kSbWarps * NTL * 512, "sb_plan");
+  const int rc = hb_func_smem(ctx, reinterpret_cast<const void*>(kq_sb_kernel<FMT, NTL>), plan.smem);
   if (rc != HB200_OK) return rc;
-  HB_CUDA(launch_pdl(kq_sb_kernel<FMT, NTL>, dim3((unsigned)grid), dim3(kSbThreads), smem, st, ctx->pdl, p));
+  HB_CUDA(launch_pdl(kq_sb_kernel<FMT, NTL>, dim3((unsigned)plan.grid), dim3(kSbThreads), plan.smem, st, ctx->pdl, p));
   return HB200_OK;
 }
 
@@ -343,58 +421,44 @@ static int sb_launch(hb200_ctx* ctx, SbParams& p, int grid, int max_total, cudaS
 int hb_kq_sb_run(hb200_ctx* ctx, int fmt, const hb200_kquant_seg* segs, int nseg, int K, int gu, const float* d_x,
                  int M, const float* pre_base, const float* pre_gamma, float* pre_out, const float* gamma, float eps,
                  cudaStream_t st) {
-  const int NTL = M <= 8 ? 1 : 2, nsb = K / 256, sms = ctx->sm_count;
-  if (M < 2 || M > 15 || K % 256 || K > 65536 || nseg < 1 || nseg > kSbMaxSeg || sms < nseg) return 1;
+  const int NTL = M <= 8 ? 1 : 2, nsb = K / 256;
+  int N[kSbMaxSeg] = {};
+  for (int s = 0; s < nseg && s < kSbMaxSeg; ++s) N[s] = segs[s].N;
+  SbPlan plan;
+  if (!sb_plan(fmt, K, N, nseg, gu, M, ctx->sm_count, ctx->smem_optin, &plan)) return 1;
   TcEncodeTiledFn encode = tc_tensor_map_encoder();
   if (encode == nullptr) return 1;
   const int unit = fmt == HB200_FMT_Q4_K ? 144 : 272;
-  const int work = gu ? 1 : nseg;  // tensors whose rows are dealt
-  // CTAs per tensor: one each, then always to the one with the most rows per CTA, down to 4 rows
-  int ctas[kSbMaxSeg], grid = work;
-  for (int s = 0; s < work; ++s) ctas[s] = 1;
-  while (grid < sms) {
-    int b = 0;
-    for (int s = 1; s < work; ++s)
-      if ((long long)segs[s].N * ctas[b] > (long long)segs[b].N * ctas[s]) b = s;
-    if ((long long)segs[b].N <= 4ll * ctas[b]) break;
-    ++ctas[b];
-    ++grid;
-  }
   SbParams p = {};
-  int max_total = 1, cta0 = 0;
-  const int cap = gu ? kSbRows / 2 : kSbRows;
+  int cta0 = 0;
   for (int s = 0; s < nseg; ++s) {
     const hb200_kquant_seg& g = segs[s];
-    const int w = gu ? 0 : s;
-    const int most = (g.N + ctas[w] - 1) / ctas[w], np = (most + cap - 1) / cap, rp = (most + np - 1) / np;
     // Q4_K: bytes; Q8_0: 32-bit words (a box dimension holds at most 256 elements, 272 > 256)
     const int esz = fmt == HB200_FMT_Q4_K ? 1 : 4;
     const int rowbytes = nsb * unit;
     const cuuint64_t dims[2] = {(cuuint64_t)(rowbytes / esz), (cuuint64_t)g.N};
     const cuuint64_t strides[1] = {(cuuint64_t)rowbytes};
-    const cuuint32_t box[2] = {(cuuint32_t)(unit / esz), (cuuint32_t)rp};
+    const cuuint32_t box[2] = {(cuuint32_t)(unit / esz), (cuuint32_t)plan.rp[s]};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult rc =
         encode(&p.tmap[s], esz == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT32, 2,
                const_cast<void*>(g.d_blocks), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     HB_REQUIRE(rc == CUDA_SUCCESS, "kquant (few tokens): cuTensorMapEncodeTiled failed (%d)", (int)rc);
-    p.seg[s] = {g.d_residual, g.d_y, g.N, cta0, ctas[w], rp, gu ? (rp + 7) / 8 : (rp + 15) / 16};
-    if (!gu) cta0 += ctas[s];
-    const int wb = ((rp * unit + 127) & ~127) * (gu ? 2 : 1);
-    if (wb > p.wbytes) p.wbytes = wb;
-    if (np * nsb > max_total) max_total = np * nsb;
+    p.seg[s] = {g.d_residual,  g.d_y,         g.N,           cta0, plan.ctas[s], plan.rp[s], plan.tiles[s],
+                plan.groups[s], plan.stages[s]};
+    if (!gu) cta0 += plan.ctas[s];
   }
   p.nseg = nseg;
   p.gu = gu;
   p.nsb = nsb;
   p.M = M;
+  p.wbytes = plan.wbytes;
   p.xb = static_cast<const uint8_t*>(ctx->d_scratch) + kScratchLmSplit;
   p.status = ctx->d_status;
   ScratchUse use(ctx, st);  // the staged fragments
   const int rc = hb_kq_stage_i8(ctx, fmt, K, NTL, d_x, M, pre_base, pre_gamma, pre_out, gamma, eps, st);
   if (rc != HB200_OK) return rc;
-  if (fmt == HB200_FMT_Q4_K)
-    return NTL == 1 ? sb_launch<12, 1>(ctx, p, grid, max_total, st) : sb_launch<12, 2>(ctx, p, grid, max_total, st);
-  return NTL == 1 ? sb_launch<8, 1>(ctx, p, grid, max_total, st) : sb_launch<8, 2>(ctx, p, grid, max_total, st);
+  if (fmt == HB200_FMT_Q4_K) return NTL == 1 ? sb_launch<12, 1>(ctx, p, plan, st) : sb_launch<12, 2>(ctx, p, plan, st);
+  return NTL == 1 ? sb_launch<8, 1>(ctx, p, plan, st) : sb_launch<8, 2>(ctx, p, plan, st);
 }

@@ -253,6 +253,13 @@ int hb200_kquant_gateup_gelu_pre(hb200_ctx *ctx, int fmt, const void *d_blocks_g
                                  float *d_x_out, const float *d_rms_gamma, float rms_eps,
                                  float *d_y, hb200_stream stream);
 
+/* How the kernel for 2 to 15 tokens (csrc/kquant_sb.cu) deals nseg tensors of N[s] rows on a GPU of
+ * `sms` SMs with `smem` bytes of shared memory per block: host arithmetic, no GPU needed.  Per tensor:
+ * stages of the ring of weights, K groups of warps, 16-row tiles of a pass, and the ring positions
+ * the longest walk of a CTA takes.  HB200_ERR_UNSUPPORTED: not a shape of that kernel. */
+int hb200_kquant_few_tokens_plan(int fmt, int K, const int *N, int nseg, int gate_up, int M,
+                                 int sms, int smem, int *stages, int *groups, int *tiles, int *total);
+
 /* ---- decode attention ------------------------------------------------------ */
 
 /* Bytes of scratch hb200_attn_decode needs for this shape (split-K partials). */

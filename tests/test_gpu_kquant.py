@@ -109,7 +109,13 @@ def test_gate_up_gelu(ctx, oracle, fmt, K, N, M):
     (2560, [2048, 512, 130], 9, False),  # second column tile with one token
     (512, [148 * 128 + 37], 15, False),  # two passes per CTA, the second one ragged
     (1024, [148 * 64 + 11], 3, True),    # gate/up, two passes
-    (2560, [333], 12, True), (2560, [2600], 2, False)])
+    (2560, [333], 12, True), (2560, [2600], 2, False),
+    # the ring of weights wraps (tests/test_kquant_few_tokens_plan.py): one tile per CTA and fewer
+    # stages than warps; unequal tensors; several laps; two passes
+    (4096, [2304], 15, False), (9216, [2304], 9, False), (4096, [1152], 12, True),
+    (4096, [1536, 384, 384], 12, False), (4096, [11000, 16], 3, False),
+    (10240, [2560], 7, False), (10240, [2560], 15, False),
+    (4096, [148 * 128 + 37], 3, False), (4096, [148 * 64 + 11], 12, True)])
 def test_few_tokens(ctx, oracle, fmt, K, Ns, M, gate_up):
     """2 to 15 tokens: 16-bit block-quantised activations, exact integer products.  An activation
     is off by at most 2^-16 of its block's largest: 2e-4 of max|y| as for one token."""
