@@ -118,8 +118,9 @@ __global__ void __launch_bounds__(kPfThreads, 1)
   uint64_t* s_full = kv_free + kSlots;   // [2] S(j) complete
   uint64_t* p_full = s_full + 2;         // [2] P(j) written by the four softmax warps
   uint64_t* q_full = p_full + 2;         // [1] Q in tensor memory
-  uint64_t* o_done = q_full + 1;         // [1] one phase per P V product
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
+  uint64_t* o_done = q_full + 1;         // [2] P V(j) has retired, even and odd j: a parity tells a
+                                         // product from the one two before it, not from the next
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
   uint8_t* ring = smem + 1024;
 
   const int G = p.G, TQ = kPfRows / G;
@@ -134,9 +135,9 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 4);
+      mbar_init(&o_done[i], 1);
     }
     mbar_init(q_full, 4);
-    mbar_init(o_done, 1);
     fence_mbar_init();
   }
   if (warp == kMmaWarp) {
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
             tmem + Cfg::kO0, tmem + Cfg::kS0 + (j & 1) * kPfTile + m * 8, vd + ((m * 2048) >> 4),
             (j > 0 || m > 0) ? 1u : 0u);
       tc_commit_w(&kv_free[vi]);
-      tc_commit_w(o_done);
+      tc_commit_w(&o_done[j & 1]);
       vi += 2;
       if (vi >= kSlots) {
         vi -= kSlots;
@@ -270,6 +271,13 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       if (lane == 0) mbar_arrive(q_full);
     }
 
+    // P V(i) has retired; asked behind s_full(i + 1) or, of the last product, s_full(i).  S(j) was issued
+    // behind P V(j - 2), so the barrier's phase is i's own or the one after it: a parity tells these
+    // apart.  With one barrier for all products a warp that came late to the end of the walk
+    // asked for the phase before last and waited in vain.
+    auto product_done = [&](int i) {
+      ok = ok && tc_wait_w(&o_done[i & 1], (uint32_t)((i >> 1) & 1), p.status);
+    };
     float m = -CUDART_INF_F, l = 0.f;  // reference maximum and sum of the row
     for (int j = 0; j < ntiles; ++j) {
       const PfTileAt at = walk.at(j0 + j);
@@ -308,8 +316,8 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       const bool grow = mt > m + 8.f;  // also the first visible tile: m = -inf
       if (j > 0 && __any_sync(0xffffffffu, grow)) {
-        // rescale O once P V(j - 1) has retired; P V(j - 2) has, S(j) was issued behind it
-        ok = ok && tc_wait_w(o_done, (uint32_t)((j - 1) & 1), p.status);
+        // rescale O once P V(j - 1) has retired
+        product_done(j - 1);
         tc_after_sync();
         const float alpha = grow ? pf_exp2(m - mt) : 1.f;  // m = -inf: 0
 #pragma unroll 1
@@ -347,9 +355,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     }
 
     // ---- O out of tensor memory, normalised or as a partial; whole rows by bulk copies -----------
-    // the last two products may both be in flight: one phase after the other, a parity alone
-    // does not tell phase n - 1 from n - 3
-    for (int i = max(0, ntiles - 2); i < ntiles; ++i) ok = ok && tc_wait_w(o_done, (uint32_t)(i & 1), p.status);
+    if (ntiles > 0) product_done(ntiles - 1);  // products retire in order
     tc_after_sync();
     const float f = p.nsplit > 1 ? 1.f : (l > 0.f ? 1.f / l : 0.f);
     // the K/V ring is idle now: every product has retired

@@ -143,6 +143,30 @@ def test_prefill_rescales_and_ignores_stale_rows(ctx, oracle, H, Hkv, D, slots, 
     assert np.abs(out - ref).max() / np.abs(ref).max() <= 1e-2
 
 
+@pytest.mark.parametrize("D,ramp", [(64, 0.0), (128, 0.0), (256, 8.0)])
+def test_prefill_walks_of_one_to_nine_tiles(ctx, oracle, D, ramp):
+    """The products of a walk are waited for by the parity of their own barrier (even and odd ones),
+    whether or not a tile made the rows rescale (a ramp of the keys does): walks of 1 to 9 tiles in
+    one call, repeated so that the four softmax warps come late in different ways."""
+    H = Hkv = 20  # 160 or more CTAs: the positions are not split
+    T, slots, scale = 9, 576, float(1.0 / np.sqrt(D))
+    lens = [64, 100, 192, 256, 320, 384, 448, 512, 576]
+    B = len(lens)
+    rng = np.random.default_rng(D + 1)
+    q = rng.standard_normal((B, T, H, D)).astype(np.float32)
+    k16 = (rng.standard_normal((B, Hkv, slots, D)) * np.linspace(1.0, 1.0 + ramp, slots)[:, None]).astype(np.float16)
+    v16 = rng.standard_normal((B, Hkv, slots, D)).astype(np.float16)
+    sl = np.asarray(lens, np.int32)
+    dq, dk, dv, dl = _dev(q), _dev(k16), _dev(v16), _dev(sl)
+    outs = [flash_attention_prefill(ctx, dq, dk, dv, dl, num_heads=H, num_kv_heads=Hkv, head_dim=D,
+                                    max_seq_len=slots, scale=scale) for _ in range(50)]
+    ctx.check()
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    ref = _reference(oracle.attn_decode, q, k16, v16, sl, T, H, Hkv, D, slots, scale, 0)
+    # with the ramp: scores up to 9 * 4 * log2(e) = 52, see the bound of the test above
+    assert np.abs(outs[0].cpu().numpy() - ref).max() / np.abs(ref).max() <= (1e-2 if ramp else TOL)
+
+
 def test_prefill_kv_writer_equals_single_token_calls(ctx):
     lib = _lib.load()
     B, T, H, Hkv, D, slots, base = 2, 7, 8, 2, 64, 40, 500000.0
