@@ -288,6 +288,8 @@ __global__ void __launch_bounds__(kMmaThreads + 128, 1)
     const int row1 = p.glu ? row0 : row0 + 64;
     TcRing<kPkStages> r;
     for (int c = 0; c < nchunks; ++c, r.advance()) {
+      // a slot is freed by way of a product once the A stages are full: bounded waits, see tc_wait
+      if (c == kPkStages + kStages / kExpGroups) pdl_wait();
       ok = tc_wait_w(&pk_free[r.i], r.phase ^ 1, p.status);
       if (!ok) break;
       if (tc_elect()) {  // two halves of 64 rows
@@ -319,6 +321,7 @@ __global__ void __launch_bounds__(kMmaThreads + 128, 1)
     // ================= two MMA warps: even steps -> accumulator 0, odd steps -> accumulator 1
     const int which = warp == kMmaWarp ? 0 : 1;
     const uint32_t tmem_d = tmem + (which ? (uint32_t)Cfg::kAcc1 : 0u);
+    pdl_wait();  // the activations come behind it: the waits below are bounded by this kernel's own work
     if (tc_elect()) {
       for (int s = which; s < nsteps; s += 2) {
         const int st = s % kStages;
@@ -354,6 +357,7 @@ __global__ void __launch_bounds__(kMmaThreads + 128, 1)
     for (int s = grp; s < nsteps; s += kExpGroups) {
       const int st = s % kStages, c = s / kExpGroups;
       if (s >= kStages) {
+        if (s < kStages + kExpGroups) pdl_wait();  // freed by a product, which needs the activations
         ok = ok && tc_wait_w(&mma_done[st], (uint32_t)(((s / kStages) - 1) & 1), p.status);
         tc_after_sync();
       }
@@ -399,6 +403,7 @@ __global__ void __launch_bounds__(kMmaThreads + 128, 1)
       ssum[tid] = p.sumq[tb * NT + tid];
     }
   }
+  pdl_wait();
   ok = tc_wait(true, done, 0, p.status) && ok;
   tc_after_sync();
   __syncthreads();  // sd / ssum visible; every warp past its loop

@@ -416,7 +416,10 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
 
   if (warp == kPkWarp) {
     // ================= weights: constant, so no wait on the previous kernel =====================
+    // ... as long as no slot has to be freed by way of a product (bounded waits, see tc_wait)
     const uint64_t pol = policy_evict_first();
+    constexpr int kAhead = kPkStages + kAStages / kAParts;
+    int nth = 0;
     TcRing<kPkStages> r;
     for (int j = 0; j < njobs && ok; ++j) {
       const QmJob job = qm_job(p.deal, j);
@@ -432,6 +435,7 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
       const int y1 = p.glu ? y0 : y0 + 64;
       int x = job.b0 * kBoxX;
       for (int b = 0; b < job.n; ++b, x += kBoxX, r.advance()) {
+        if (nth++ == kAhead) pdl_wait();
         ok = tc_wait_w(&pk_free[r.i], r.phase ^ 1, p.status);
         if (!ok) break;
         if (tc_elect()) {
@@ -474,6 +478,7 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
     auto wait = [&](uint64_t* bar, uint32_t parity) {
       if (!mbar_try_wait(bar, parity) && ok) ok = tc_wait_slow(smem_u32(bar), parity, p.status);
     };
+    pdl_wait();  // the activations come behind it: the waits below are bounded by this kernel's own work
     TcRing<kAStages> ra;
     TcRing<kBStages> rb;
     uint32_t eslot = 0, dphase = 0;
@@ -641,6 +646,7 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
         const uint8_t* blk = pk + (size_t)rp.i * kPkBytes + (size_t)erow * kUnit;
         const uint32_t a_t = a_base + ra.i * kACols;
         auto stage_free = [&]() {
+          if (s >= kAStages) wait_previous();  // freed by a product, which needs the activations
           ok = ok && tc_wait_w(&a_free[ra.i], ra.phase ^ 1, p.status);
           tc_after_sync();
         };

@@ -301,10 +301,12 @@ __global__ void __launch_bounds__(kLmThreads, 1) lmhead_mma_kernel(const __grid_
     // ================= table: constant, so no wait on the previous kernel =======================
     const uint64_t pol = policy_evict_first();
     TcRing<kAS> r;
+    int nth = 0;
     for (int t = t0; t < t1 && ok; t += Cfg::kTiles) {
       const int n = min(Cfg::kTiles, t1 - t);
       for (int ks = 0; ks < nsteps && ok; ++ks)
         for (int i = 0; i < n; ++i, r.advance()) {
+          if (nth++ == kAS) pdl_wait();  // from here on a slot is freed by a product (bounded waits)
           ok = tc_wait_w(&a_free[r.i], r.phase ^ 1, p.status);
           if (!ok) break;
           if (tc_elect()) {

@@ -100,7 +100,9 @@ __device__ __forceinline__ void tc_tma_box_2d(void* dst, const CUtensorMap* tm, 
 }
 
 // Bounded mbarrier wait for kernels whose whole life is microseconds: ~1e5 polls already
-// means something is broken.  Once a wait has failed the later ones are skipped, so a broken
+// means something is broken.  The kernel may be resident long before its predecessor ends (which may
+// itself wait for another GPU), so a wait that depends on what the predecessor writes, directly or by
+// way of another warp, only starts behind pdl_wait.  Once a wait has failed the later ones are skipped, so a broken
 // launch ends quickly (and still releases its tensor memory).
 __device__ __forceinline__ bool tc_wait(bool ok, uint64_t* bar, uint32_t parity, uint32_t* status) {
   if (!ok) return false;
