@@ -253,11 +253,23 @@ int hb_kq_stage(struct hb200_ctx* ctx, int fmt, int K, int NT, const float* d_x,
 
 int hb_kq_stage_i8(struct hb200_ctx* ctx, int fmt, int K, int ntl, const float* d_x, int M,
                    const float* d_pre_base, const float* d_pre_gamma, float* d_pre_out,
-                   const float* d_rms_gamma, float rms_eps, cudaStream_t st);
-// Q4_K / Q8_0 product of 2 to 15 tokens on mma.sync (kquant_sb.cu); 1 = shape not covered
+                   const float* d_rms_gamma, float rms_eps, uint8_t* frag, cudaStream_t st);
+// Q4_K / Q8_0 product of 2 to 15 tokens on mma.sync (kquant_sb.cu); 1 = not covered.  frag: the
+// staged activations' own memory (hb_kq_frag_bytes); null: the context's scratch, which a stream
+// capture does not get (its replays would not be ordered with the scratch's other users)
 int hb_kq_sb_run(struct hb200_ctx* ctx, int fmt, const hb200_kquant_seg* segs, int nseg, int K, int gu,
                  const float* d_x, int M, const float* pre_base, const float* pre_gamma, float* pre_out,
-                 const float* gamma, float eps, cudaStream_t st);
+                 const float* gamma, float eps, uint8_t* frag, cudaStream_t st);
+// The k-quant operators of the C ABI for callers that keep such memory (kquant.cu); pre_gamma null: no
+// pre-step
+constexpr size_t hb_kq_frag_bytes(int K) { return (size_t)(K / 256) * 2 * 4608; }
+int hb_kquant_forward_multi(struct hb200_ctx* ctx, int fmt, const hb200_kquant_seg* segs, int nseg, int K,
+                            const float* d_x, int M, const float* pre_base, const float* pre_gamma,
+                            float* pre_out, const float* gamma, float eps, void* frag, cudaStream_t st);
+int hb_kquant_gateup_gelu(struct hb200_ctx* ctx, int fmt, const void* d_gate, const void* d_up, int K, int N,
+                          const float* d_x, int M, const float* pre_base, const float* pre_gamma,
+                          float* pre_out, const float* gamma, float eps, float* d_y, void* frag,
+                          cudaStream_t st);
 
 struct hb200_ctx {
   int device;

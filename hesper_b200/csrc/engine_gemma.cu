@@ -35,6 +35,7 @@ struct hb200_gemma {
   int32_t *pos, *len, *tok, *log_index, *token_log;
   unsigned long long* keys;
   double* rope_tab;  // [B * chunk_T][D/2][2] the pass's RoPE angles, shared by all layers
+  void* frag;  // hb_kq_frag_bytes of the widest product
   void* attn_ws;
   size_t attn_ws_bytes;
   int log_stride;
@@ -152,17 +153,22 @@ int gemma_enqueue_step(hb200_gemma* m, const int32_t* d_tokens, bool lm_head, cu
   // launch (the o_proj / down_proj output stays in m->o until then): two launches fewer per
   // layer.  The last layer's post-FFN norm has no next matvec and runs on its own.
   const bool fold = m->tp == nullptr && getenv("HB200_NO_FOLD") == nullptr;
+  auto linear = [&](const void* w, int K, int N, const float* x, int M, const float* gamma, float eps, float* y) {
+    const hb200_kquant_seg s = {w, nullptr, y, N};
+    return hb_kquant_forward_multi(ctx, HB200_FMT_Q4_K, &s, 1, K, x, M, nullptr, nullptr, nullptr, gamma, eps,
+                                   m->frag, st);
+  };
   for (int l = 0; l < c.n_layers; ++l) {
     const hb200_gemma_layer& L = m->layers[l];
     hb200_kquant_seg segs[3] = {
         {L.wq, nullptr, m->q, qdim}, {L.wk, nullptr, m->k, kvdim}, {L.wv, nullptr, m->v, kvdim}};
     if (fold && l > 0)  // x = x1 + rmsnorm(o) * post_ffn_norm of the previous layer
-      rc = hb200_kquant_forward_multi_pre(ctx, HB200_FMT_Q4_K, segs, 3, Hd, m->o, B, m->x1,
-                                          m->layers[l - 1].post_ffn_norm, m->x, L.attn_norm,
-                                          c.rms_eps, st);
+      rc = hb_kquant_forward_multi(ctx, HB200_FMT_Q4_K, segs, 3, Hd, m->o, B, m->x1,
+                                   m->layers[l - 1].post_ffn_norm, m->x, L.attn_norm, c.rms_eps,
+                                   m->frag, st);
     else
-      rc = hb200_kquant_forward_multi(ctx, HB200_FMT_Q4_K, segs, 3, Hd, m->x, B, L.attn_norm,
-                                      c.rms_eps, st);
+      rc = hb_kquant_forward_multi(ctx, HB200_FMT_Q4_K, segs, 3, Hd, m->x, B, nullptr, nullptr,
+                                   nullptr, L.attn_norm, c.rms_eps, m->frag, st);
     if (rc) return rc;
     const bool ring = m->slots[l] < c.max_seq;
     rc = hb200_rope_kv_write_prefill_angles(ctx, m->q, m->k, m->v, m->kc[l], m->vc[l], m->pos,
@@ -178,23 +184,20 @@ int gemma_enqueue_step(hb200_gemma* m, const int32_t* d_tokens, bool lm_head, cu
                               c.local_kv_heads, D, m->slots[l], m->win[l], c.attn_scale,
                               m->attn_ws, m->attn_ws_bytes, m->att, st);
     if (rc) return rc;
-    rc = hb200_kquant_forward(ctx, HB200_FMT_Q4_K, L.wo, qdim, Hd, m->att, B, nullptr, 0.f, nullptr,
-                              m->o, st);
+    rc = linear(L.wo, qdim, Hd, m->att, B, nullptr, 0.f, m->o);
     if (rc) return rc;
     if (fold) {  // x1 = x + rmsnorm(o) * post_attn_norm, then the gated FFN on x1
-      rc = hb200_kquant_gateup_gelu_pre(ctx, HB200_FMT_Q4_K, L.wgate, L.wup, Hd, c.local_ffn, m->o,
-                                        B, m->x, L.post_attn_norm, m->x1, L.ffn_norm, c.rms_eps,
-                                        m->h, st);
+      rc = hb_kquant_gateup_gelu(ctx, HB200_FMT_Q4_K, L.wgate, L.wup, Hd, c.local_ffn, m->o, B, m->x,
+                                 L.post_attn_norm, m->x1, L.ffn_norm, c.rms_eps, m->h, m->frag, st);
     } else {
       rc = hb200_tp_allreduce_rmsnorm(m->tp, ctx, m->o, L.post_attn_norm, m->x, c.rms_eps, B, Hd,
                                       m->x1, st);
       if (rc) return rc;
-      rc = hb200_kquant_gateup_gelu(ctx, HB200_FMT_Q4_K, L.wgate, L.wup, Hd, c.local_ffn, m->x1, B,
-                                    L.ffn_norm, c.rms_eps, m->h, st);
+      rc = hb_kquant_gateup_gelu(ctx, HB200_FMT_Q4_K, L.wgate, L.wup, Hd, c.local_ffn, m->x1, B,
+                                 nullptr, nullptr, nullptr, L.ffn_norm, c.rms_eps, m->h, m->frag, st);
     }
     if (rc) return rc;
-    rc = hb200_kquant_forward(ctx, HB200_FMT_Q4_K, L.wdown, c.local_ffn, Hd, m->h, B, nullptr, 0.f,
-                              nullptr, m->o, st);
+    rc = linear(L.wdown, c.local_ffn, Hd, m->h, B, nullptr, 0.f, m->o);
     if (rc) return rc;
     if (!fold || l == c.n_layers - 1) {
       rc = hb200_tp_allreduce_rmsnorm(m->tp, ctx, m->o, L.post_ffn_norm, m->x1, c.rms_eps, B, Hd,
@@ -210,8 +213,7 @@ int gemma_enqueue_step(hb200_gemma* m, const int32_t* d_tokens, bool lm_head, cu
                                 cudaMemcpyDeviceToDevice, st));
       xl = m->x1;
     }
-    rc = hb200_kquant_forward(ctx, HB200_FMT_Q4_K, m->lm_head, Hd, c.local_vocab, xl, nseq,
-                              m->final_norm, c.rms_eps, nullptr, m->logits, st);
+    rc = linear(m->lm_head, Hd, c.local_vocab, xl, nseq, m->final_norm, c.rms_eps, m->logits);
     if (rc) return rc;
     // enough CTAs to spread a single token's logits over the SMs, few atomics at large batch
     const int chunk = nseq <= 8 ? 2048 : 8192;
@@ -307,6 +309,10 @@ extern "C" int hb200_gemma_create(hb200_ctx* ctx, hb200_tp* tp, const hb200_gemm
   A(cudaMalloc(reinterpret_cast<void**>(&m->keys), sizeof(unsigned long long) * batch));
   A(cudaMemset(m->keys, 0, sizeof(unsigned long long) * batch));
   A(cudaMalloc(reinterpret_cast<void**>(&m->rope_tab), sizeof(double) * (size_t)B * D));
+  // staged activations of the products of 2 to 15 rows: the model's own, as its graphs replay beside
+  // whatever else uses the context
+  const int widest = std::max(cfg->hidden, std::max(qdim, cfg->local_ffn));
+  A(cudaMalloc(&m->frag, hb_kq_frag_bytes(widest)));
   m->attn_ws_bytes = hb200_attn_workspace_bytes(ctx, batch, cfg->local_q_heads,
                                                 cfg->local_kv_heads, D, max_slots);
   // the split count, hence the partials, depend on the number of query tokens in a pass, and
@@ -334,6 +340,7 @@ extern "C" int hb200_gemma_destroy(hb200_gemma* m) {
   for (auto p : m->vc) cudaFree(p);
   cudaFree(m->pos); cudaFree(m->tok); cudaFree(m->log_index); cudaFree(m->token_log);
   cudaFree(m->keys); cudaFree(m->attn_ws);
+  cudaFree(m->frag);
   delete m;
   return HB200_OK;
 }

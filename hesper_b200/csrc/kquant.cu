@@ -716,7 +716,8 @@ static int kq_pre_check(const KQPre& pre, const float* d_x) {
 
 static int kq_forward_multi_impl(hb200_ctx* ctx, int fmt, const hb200_kquant_seg* segs, int nseg,
                                  int K, const float* d_x, int M, const KQPre& pre,
-                                 const float* d_rms_gamma, float rms_eps, hb200_stream stream) {
+                                 const float* d_rms_gamma, float rms_eps, hb200_stream stream,
+                                 void* frag = nullptr) {
   int rc = kq_check(ctx, fmt, K, M, d_x);
   if (rc) return rc;
   rc = kq_pre_check(pre, d_x);
@@ -745,7 +746,8 @@ static int kq_forward_multi_impl(hb200_ctx* ctx, int fmt, const hb200_kquant_seg
                       rms_eps, st);
     if (rc <= 0) return rc;
   } else if (kq_few_tokens(ctx, fmt, rows, K, M)) {
-    rc = hb_kq_sb_run(ctx, fmt, segs, nseg, K, 0, d_x, M, pre.base, pre.gamma, pre.out, d_rms_gamma, rms_eps, st);
+    rc = hb_kq_sb_run(ctx, fmt, segs, nseg, K, 0, d_x, M, pre.base, pre.gamma, pre.out, d_rms_gamma, rms_eps,
+                      static_cast<uint8_t*>(frag), st);
     if (rc <= 0) return rc;
   }
   const int rowbytes = kq_rowbytes(fmt, K);
@@ -809,7 +811,7 @@ extern "C" int hb200_kquant_forward(hb200_ctx* ctx, int fmt, const void* d_block
 static int kq_gateup_impl(hb200_ctx* ctx, int fmt, const void* d_blocks_gate,
                           const void* d_blocks_up, int K, int N, const float* d_x, int M,
                           const KQPre& pre, const float* d_rms_gamma, float rms_eps, float* d_y,
-                          hb200_stream stream) {
+                          hb200_stream stream, void* frag = nullptr) {
   int rc = kq_check(ctx, fmt, K, M, d_x);
   if (rc) return rc;
   rc = kq_pre_check(pre, d_x);
@@ -832,7 +834,8 @@ static int kq_gateup_impl(hb200_ctx* ctx, int fmt, const void* d_blocks_gate,
                       rms_eps, st);
     if (rc <= 0) return rc;
   } else if (kq_few_tokens(ctx, fmt, 2L * N, K, M)) {
-    rc = hb_kq_sb_run(ctx, fmt, gs, 2, K, 1, d_x, M, pre.base, pre.gamma, pre.out, d_rms_gamma, rms_eps, st);
+    rc = hb_kq_sb_run(ctx, fmt, gs, 2, K, 1, d_x, M, pre.base, pre.gamma, pre.out, d_rms_gamma, rms_eps,
+                      static_cast<uint8_t*>(frag), st);
     if (rc <= 0) return rc;
   }
   const int rowbytes = kq_rowbytes(fmt, K);
@@ -878,4 +881,19 @@ extern "C" int hb200_kquant_gateup_gelu_pre(hb200_ctx* ctx, int fmt, const void*
   HB_REQUIRE(d_pre_gamma != nullptr, "kquant (pre-step): null gamma");
   return kq_gateup_impl(ctx, fmt, d_blocks_gate, d_blocks_up, K, N, d_o, M,
                         KQPre{d_pre_base, d_pre_gamma, d_x_out}, d_rms_gamma, rms_eps, d_y, stream);
+}
+
+int hb_kquant_forward_multi(hb200_ctx* ctx, int fmt, const hb200_kquant_seg* segs, int nseg, int K,
+                            const float* d_x, int M, const float* pre_base, const float* pre_gamma,
+                            float* pre_out, const float* gamma, float eps, void* frag, cudaStream_t st) {
+  return kq_forward_multi_impl(ctx, fmt, segs, nseg, K, d_x, M, KQPre{pre_base, pre_gamma, pre_out}, gamma, eps,
+                               st, frag);
+}
+
+int hb_kquant_gateup_gelu(hb200_ctx* ctx, int fmt, const void* d_gate, const void* d_up, int K, int N,
+                          const float* d_x, int M, const float* pre_base, const float* pre_gamma,
+                          float* pre_out, const float* gamma, float eps, float* d_y, void* frag,
+                          cudaStream_t st) {
+  return kq_gateup_impl(ctx, fmt, d_gate, d_up, K, N, d_x, M, KQPre{pre_base, pre_gamma, pre_out}, gamma, eps, d_y,
+                        st, frag);
 }

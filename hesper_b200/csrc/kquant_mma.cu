@@ -956,15 +956,14 @@ int hb_kq_stage(hb200_ctx* ctx, int fmt, int K, int NT, const float* d_x, int M,
   return qm_stage_launch<false>(ctx, p, M, st);
 }
 
-// The same for the few-token kernel (kquant_sb.cu): ntl * 8 token columns, M of them real.
+// The same for the few-token kernel (kquant_sb.cu), into `frag`: ntl * 8 token columns, M of them real.
 int hb_kq_stage_i8(hb200_ctx* ctx, int fmt, int K, int ntl, const float* d_x, int M, const float* d_pre_base,
                    const float* d_pre_gamma, float* d_pre_out, const float* d_rms_gamma, float rms_eps,
-                   cudaStream_t st) {
+                   uint8_t* frag, cudaStream_t st) {
   QmStage p = {};
   p.sb_bytes = (size_t)ntl * 4608;
   p.sums_off = fmt == HB200_FMT_Q4_K;
-  HB_REQUIRE(p.sb_bytes * (size_t)(K / 256) <= kScratchRowScale - kScratchLmSplit && K <= 65536,
-             "kquant (few tokens): K=%d does not fit the activation scratch", K);
+  HB_REQUIRE(K <= 65536, "kquant (few tokens): K=%d", K);
   p.x = d_x;
   p.gamma = d_rms_gamma;
   p.pre_base = d_pre_base;
@@ -974,6 +973,6 @@ int hb_kq_stage_i8(hb200_ctx* ctx, int fmt, int K, int ntl, const float* d_x, in
   p.K = K;
   p.M = M;
   p.ntl = ntl;
-  p.xb = static_cast<uint8_t*>(ctx->d_scratch) + kScratchLmSplit;
+  p.xb = frag;
   return qm_stage_launch<true>(ctx, p, ntl * 8, st);
 }

@@ -26,6 +26,7 @@
 // What bounds it: instruction issue -- about 330 instructions per 16 rows x 256 weights at up to
 // 8 tokens, 520 at up to 15 (products, int -> float, scales) -- 2 to 3.5 us at K=2560 N=10240 --
 // next to 2.2 (Q4_K) or 4.2 us (Q8_0) of weight stream.
+#include <optional>
 #include <type_traits>
 
 #include "tcgen05.cuh"
@@ -417,10 +418,12 @@ static int sb_launch(hb200_ctx* ctx, const SbParams& p, const SbPlan& plan, cuda
 }
 
 // 2 to 15 tokens; gu: two tensors of equal shape, gate and up, into segs[0].d_y.  HB200_OK when the
-// launches were made, 1 when the shape is outside what this path covers, < 0 on error.
+// launches were made, 1 when the call is outside what this path covers, < 0 on error.
+// Captured calls without memory of their own are outside: the streaming kernel of kquant.cu keeps
+// nothing in the context, so captured branches, and a replay beside an eager stream, may share one.
 int hb_kq_sb_run(hb200_ctx* ctx, int fmt, const hb200_kquant_seg* segs, int nseg, int K, int gu, const float* d_x,
                  int M, const float* pre_base, const float* pre_gamma, float* pre_out, const float* gamma, float eps,
-                 cudaStream_t st) {
+                 uint8_t* frag, cudaStream_t st) {
   const int NTL = M <= 8 ? 1 : 2, nsb = K / 256;
   int N[kSbMaxSeg] = {};
   for (int s = 0; s < nseg && s < kSbMaxSeg; ++s) N[s] = segs[s].N;
@@ -428,6 +431,17 @@ int hb_kq_sb_run(hb200_ctx* ctx, int fmt, const hb200_kquant_seg* segs, int nseg
   if (!sb_plan(fmt, K, N, nseg, gu, M, ctx->sm_count, ctx->smem_optin, &plan)) return 1;
   TcEncodeTiledFn encode = tc_tensor_map_encoder();
   if (encode == nullptr) return 1;
+  std::optional<ScratchUse> use;
+  if (frag == nullptr) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+      cudaGetLastError();
+      return 1;
+    }
+    if (cs != cudaStreamCaptureStatusNone) return 1;
+    use.emplace(ctx, st);
+    frag = static_cast<uint8_t*>(ctx->d_scratch) + kScratchLmSplit;
+  }
   const int unit = fmt == HB200_FMT_Q4_K ? 144 : 272;
   SbParams p = {};
   int cta0 = 0;
@@ -454,10 +468,10 @@ int hb_kq_sb_run(hb200_ctx* ctx, int fmt, const hb200_kquant_seg* segs, int nseg
   p.nsb = nsb;
   p.M = M;
   p.wbytes = plan.wbytes;
-  p.xb = static_cast<const uint8_t*>(ctx->d_scratch) + kScratchLmSplit;
+  p.xb = frag;
   p.status = ctx->d_status;
-  ScratchUse use(ctx, st);  // the staged fragments
-  const int rc = hb_kq_stage_i8(ctx, fmt, K, NTL, d_x, M, pre_base, pre_gamma, pre_out, gamma, eps, st);
+  static_assert(hb_kq_frag_bytes(65536) <= kScratchRowScale - kScratchLmSplit, "fragments in the scratch");
+  const int rc = hb_kq_stage_i8(ctx, fmt, K, NTL, d_x, M, pre_base, pre_gamma, pre_out, gamma, eps, frag, st);
   if (rc != HB200_OK) return rc;
   if (fmt == HB200_FMT_Q4_K) return NTL == 1 ? sb_launch<12, 1>(ctx, p, plan, st) : sb_launch<12, 2>(ctx, p, plan, st);
   return NTL == 1 ? sb_launch<8, 1>(ctx, p, plan, st) : sb_launch<8, 2>(ctx, p, plan, st);

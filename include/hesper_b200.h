@@ -210,8 +210,9 @@ typedef struct hb200_kquant_seg {
  * binds to: (inputF32Ptr, weightPtr, outputF32Ptr, inDim, outDim, quantTag).
  *   fmt  HB200_FMT_Q4_K or HB200_FMT_Q8_0; K a multiple of 256; 1 <= M <= 4096
  *   d_rms_gamma nullable: RMSNorm prologue as forwardFusedRMSNormLinear (:7897 region)
- * Up to 15 tokens stream the weights once per token through the dp4a kernel (activations
- * block-quantised to 16 bits, error ~2e-5).  From 16 tokens on the product runs on the
+ * Up to 15 tokens: activations block-quantised to 16 bits, integer products, error ~2e-5.  2 to 15
+ * tokens read the weights once (csrc/kquant_sb.cu), except in a stream capture, where they stream
+ * them once per token and use nothing of the context.  From 16 tokens on the product runs on the
  * tensor cores, up to 256 tokens per pass: both formats are dequantised to f16 inside the
  * tcgen05 kernel; weights and activations rounded to f16 (every staged activation row
  * scaled by its own power of two), error ~4e-4 of max|y| (the bar of this path is 1e-3). */
@@ -238,9 +239,8 @@ int hb200_kquant_gateup_gelu(hb200_ctx *ctx, int fmt, const void *d_blocks_gate,
  * Hesper/Models/Gemma4.lean:904-925 followed by the next block's fused norm + matvec):
  *   x' = d_pre_base + rmsnorm(d_o) * d_pre_gamma      (also written to d_x_out, [M][K])
  *   then hb200_kquant_forward_multi / hb200_kquant_gateup_gelu on x'.
- * The step has no launch of its own: up to 15 tokens it runs inside the matvec kernel's
- * prologue, from 16 tokens inside the kernel that stages the activations for the tensor-core
- * product (Q8_0 from 16 tokens: one hb200_rmsnorm launch).  d_x_out may alias neither input; all
+ * The step has no launch of its own: it runs inside the matvec kernel's prologue or inside the
+ * kernel that stages the activations of several tokens.  d_x_out may alias neither input; all
  * arrays 16-byte aligned; rms_eps serves both norms. */
 int hb200_kquant_forward_multi_pre(hb200_ctx *ctx, int fmt, const hb200_kquant_seg *segs,
                                    int nseg, int K, const float *d_o, int M,

@@ -1,4 +1,5 @@
-"""GPU: a context's scratch serves one stream at a time, and the library enforces it.
+"""GPU: a context's scratch serves one stream at a time, and the library enforces it; what may be
+captured and replayed beside other work does not use it.
 
 The batched products stage their activations in the context's scratch; two calls issued back
 to back on two different streams would otherwise overlap on the device and the second staging
@@ -9,7 +10,8 @@ import numpy as np
 import pytest
 import torch
 
-from hesper_b200 import LinearLayer, BitLinear, formats
+from hesper_b200 import BitLinear, Context, GemmaModel, LinearLayer, formats, tp
+from tp_common import SMALL_GEMMA
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +41,67 @@ def test_batched_calls_on_two_streams_do_not_share_scratch_in_time(ctx):
             assert torch.equal(outs_q[i], ref_q[i]), f"Q4_K call {i}"
             assert torch.equal(outs_t[i], ref_t[i]), f"ternary call {i}"
     ctx.check()
+
+
+@pytest.mark.parametrize("fmt,M", [(12, 7), (8, 2), (8, 15)])
+def test_captured_calls_of_a_few_tokens_share_nothing(ctx, monkeypatch, fmt, M):
+    """2 to 15 tokens in a stream capture use no memory of the context: two branches of one graph,
+    and its replays beside calls on another stream, do not disturb each other.  That they run on the
+    streaming kernel shows in the bits, which are those of a context kept on it."""
+    rng = np.random.default_rng(M)
+    K, N = 2560, 4096
+    blocks = [formats.random_kquant(rng, fmt, N, K) for _ in range(2)]
+    layers = [LinearLayer.create_from_bytes(ctx, b, fmt, K, N) for b in blocks]
+    x = torch.randn(M, K, device="cuda")
+    eager = layers[0].forward(x)
+    monkeypatch.setenv("HB200_NO_MMA", "1")
+    plain = Context(0)
+    monkeypatch.delenv("HB200_NO_MMA")
+    want = [LinearLayer.create_from_bytes(plain, b, fmt, K, N).forward(x) for b in blocks]
+    torch.cuda.synchronize()
+    ys = [torch.empty(M, N, device="cuda") for _ in range(2)]
+    g, side, other = torch.cuda.CUDAGraph(), torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.graph(g):
+        main = torch.cuda.current_stream()
+        side.wait_stream(main)
+        layers[1].forward(x, out=ys[1], stream=side)
+        layers[0].forward(x, out=ys[0])
+        main.wait_stream(side)
+    for _ in range(20):
+        for y in ys:
+            y.zero_()
+        beside = [layers[0].forward(x, stream=other) for _ in range(4)]
+        g.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, w) for y, w in zip(ys, want))
+        assert all(torch.equal(b, eager) for b in beside)
+    ctx.check()
+    plain.close()
+
+
+def test_decode_graph_of_a_few_sequences_beside_another_stream(ctx):
+    """The engine's graph replays on memory of the engine's own: tokens and products are the same
+    with calls of 7 tokens queued on another stream of the same context."""
+    w = tp.random_gemma_weights(SMALL_GEMMA, seed=5)
+    p = tp.plan(SMALL_GEMMA, 0, 1)
+    model = GemmaModel(ctx, SMALL_GEMMA, tp.shard_weights(SMALL_GEMMA, w, p), p, None, batch=4, max_new_tokens=40)
+    prompt = np.arange(12, dtype=np.int32).reshape(4, 3)
+    model.generate(prompt, 2)
+    model.set_position(3)
+    want, _, _ = model.generate(None, 30)
+    rng = np.random.default_rng(0)
+    layer = LinearLayer.create_from_bytes(ctx, formats.random_kquant(rng, 12, 4096, 2560), 12, 2560, 4096)
+    x = torch.randn(7, 2560, device="cuda")
+    ref = layer.forward(x)
+    other = torch.cuda.Stream()
+    for _ in range(5):
+        model.generate(prompt, 2)
+        model.set_position(3)
+        torch.cuda.synchronize()
+        outs = [layer.forward(x, stream=other) for _ in range(400)]
+        got, _, _ = model.generate(None, 30)
+        torch.cuda.synchronize()
+        assert np.array_equal(got, want)
+        assert all(torch.equal(o, ref) for o in outs)
+    ctx.check()
+    model.close()
