@@ -231,7 +231,9 @@ int hb_lmhead_mma_run(struct hb200_ctx* ctx, const void* d_table, int dtype, lon
 // never overlap in time may overlap in space):
 constexpr size_t kScratchBytes = (size_t)56 << 20;
 constexpr size_t kScratchActs = 0;                     // batched ternary: d[512], sumq[512], int8 tiles
-constexpr size_t kScratchLmSplit = (size_t)8 << 20;   // 16-bit products: hi/lo activation tiles
+constexpr size_t kScratchLmSplit = (size_t)8 << 20;   // LM head: hi/lo activation tiles; k-quants of
+                                                       // 2 to 15 tokens: their fragments
+constexpr size_t kScratchKqActs = (size_t)7 << 20;    // batched k-quants: f16 activation tiles and sums
 constexpr size_t kScratchRowScale = ((size_t)16 << 20) - 4096;  // f16 products: one power-of-two
                                                        // scale per staged activation row
 constexpr size_t kScratchSplitK = (size_t)16 << 20;   // batched paths: split-K partials

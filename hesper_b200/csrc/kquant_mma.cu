@@ -893,7 +893,7 @@ int hb_kq_mma_run_multi(hb200_ctx* ctx, const HbKqSeg* segs, int nseg, int K, in
   if (glu) tiles = (int)((segs[0].N + kQmRows / 2 - 1) / (kQmRows / 2));
   p.nseg = nseg;
   p.glu = glu;
-  p.xb = static_cast<const uint8_t*>(ctx->d_scratch) + kScratchLmSplit;
+  p.xb = static_cast<const uint8_t*>(ctx->d_scratch) + kScratchKqActs;
   p.rowscale = reinterpret_cast<const float*>(static_cast<const uint8_t*>(ctx->d_scratch) +
                                               kScratchRowScale);
   p.M = M;
@@ -917,10 +917,14 @@ int hb_kq_mma_run_multi(hb200_ctx* ctx, const HbKqSeg* segs, int nseg, int K, in
 // Bytes of staged activations per super-block of 256 weights.
 static size_t qm_sb_bytes(int fmt, int NT) { return (size_t)NT * (fmt == HB200_FMT_Q4_K ? 544 : 512); }
 
+constexpr size_t kQmActBytes = kScratchRowScale - kScratchKqActs;
+constexpr int kQmMaxK = 65280;
+static_assert((size_t)64 * 544 * (kQmMaxK / 256) <= kQmActBytes, "a pass of 64 tokens fits at every K");
+
 // Most tokens (64, 128 or 256) one pass can stage at this K.
 int hb_kq_mma_max_tokens(int fmt, int K) {
   for (int NT = 256; NT > 64; NT >>= 1)
-    if (qm_sb_bytes(fmt, NT) * (size_t)(K / 256) <= kScratchRowScale - kScratchLmSplit) return NT;
+    if (qm_sb_bytes(fmt, NT) * (size_t)(K / 256) <= kQmActBytes) return NT;
   return 64;
 }
 
@@ -942,7 +946,7 @@ int hb_kq_stage(hb200_ctx* ctx, int fmt, int K, int NT, const float* d_x, int M,
   QmStage p = {};
   p.sb_bytes = qm_sb_bytes(fmt, NT);
   p.sums_off = fmt == HB200_FMT_Q4_K ? NT * 512 : 0;
-  HB_REQUIRE(p.sb_bytes * (size_t)(K / 256) <= kScratchRowScale - kScratchLmSplit && K <= 65536,
+  HB_REQUIRE(p.sb_bytes * (size_t)(K / 256) <= kQmActBytes && K <= kQmMaxK,
              "kquant (fused batched): K=%d does not fit the activation scratch", K);
   p.x = d_x;
   p.gamma = d_rms_gamma;
@@ -951,7 +955,7 @@ int hb_kq_stage(hb200_ctx* ctx, int fmt, int K, int NT, const float* d_x, int M,
   p.pre_out = d_pre_out;
   p.eps = rms_eps;
   p.K = K;
-  p.xb = static_cast<uint8_t*>(ctx->d_scratch) + kScratchLmSplit;
+  p.xb = static_cast<uint8_t*>(ctx->d_scratch) + kScratchKqActs;
   p.rowscale = reinterpret_cast<float*>(static_cast<uint8_t*>(ctx->d_scratch) + kScratchRowScale);
   return qm_stage_launch<false>(ctx, p, M, st);
 }

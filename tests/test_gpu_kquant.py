@@ -141,6 +141,23 @@ def test_few_tokens(ctx, oracle, fmt, K, Ns, M, gate_up):
         assert _check(y, oracle.kquant_matvec(fmt, b, K, n, xn)) < 2e-4
 
 
+@pytest.mark.parametrize("fmt", [12, 8])
+@pytest.mark.parametrize("M", [16, 64])
+def test_longest_rows_of_the_batched_product(ctx, oracle, fmt, M):
+    """K = 65280 is the longest row 16 tokens or more take, in both formats; 65536 is refused."""
+    K, N = 65280, 70
+    rng = np.random.default_rng(fmt + M)
+    blocks = formats.random_kquant(rng, fmt, N, K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    y = LinearLayer.create_from_bytes(ctx, blocks, fmt, K, N).forward(_dev(x))
+    ctx.check()
+    rows = [0, 9, M - 1]
+    assert _check(y[rows], oracle.kquant_matvec(fmt, blocks, K, N, x[rows])) < 1e-3
+    long = LinearLayer.create_from_bytes(ctx, formats.random_kquant(rng, fmt, 8, 65536), fmt, 65536, 8)
+    with pytest.raises(hb.HesperB200Error):
+        long.forward(torch.zeros(M, 65536, device="cuda"))
+
+
 def test_fused_qkv_multi(ctx, oracle):
     K = 2560
     rng = np.random.default_rng(8)
