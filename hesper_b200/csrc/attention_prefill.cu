@@ -13,18 +13,20 @@
 //     scale * log2 e, f16) and K as the K-major operand; O += P V with P in tensor memory (it
 //     replaces the S it came from) and V, as it lies in the cache, as the MN-major operand.
 //     S has two buffers: S(j+1) runs while the softmax works on S(j).
-//   * warps 0-3: one thread per row.  Online softmax in the exp2 domain with P rounded to f16
-//     (same rounding as the decode kernel's FAST mode: bar 2e-3 against an f64 evaluation).  The
-//     reference maximum of a row moves only when a tile exceeds it by more than 2^8 (P then stays
-//     below 2^8, far inside f16): O is rescaled in tensor memory a few times per row instead
-//     of once per tile, and the quotient O / l is the same.
+//   * warps 0-3: one thread per row.  Online softmax in the exp2 domain.  The reference maximum of a
+//     row moves only when a tile exceeds it by more than 2^8 (P then stays below 2^8, far inside
+//     f16): O is rescaled in tensor memory a few times per row instead of once per tile, and the
+//     quotient O / l is the same.  P is two f16 terms, what was rounded and what that lost: the
+//     maximum of a tile no longer weighs exactly 1, which with one term raised the error against an
+//     f64 evaluation by 5 % on average (10 % at most); with two it is 0.77 of what it was, the query's
+//     f16 rounding alone, for 14 % more time (256-token chunk at 8192 positions 31 -> 35.6 us).
 //   * a row's visible positions are [max(0, pos - window + 1), pos] with pos the token's own
 //     position: causal inside the chunk, sliding window if asked.
 //
 // Tensor memory at D = 256: O 256 columns, Q 128, S 2 x 64 = all 512.  What bounds it: a tile is
-// 16 MMAs of N=64 plus 4 of N=256, 1024 cycles of the tensor pipe, against ~700 of softmax (64
-// exponentials per row are 512 cycles of the special-function unit) that overlap all but the part
-// between S(j) and P(j); K and V come from L2 at 64 KB per tile.  When the query tiles leave SMs
+// 16 MMAs of N=64 plus 8 of N=256, 1536 cycles of the tensor pipe (the four for P's second term
+// show in full), with the softmax's 64 exponentials per row (512 cycles of the special-function
+// unit) beside it; K and V come from L2 at 64 KB per tile.  When the query tiles leave SMs
 // idle the positions are dealt to several CTAs and a second kernel merges their partials.
 #include <math_constants.h>
 
@@ -221,10 +223,10 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       tc_after_sync();
       const uint32_t vd = vdesc0 + vi * (Cfg::kSlotBytes >> 4);
 #pragma unroll
-      for (int m = 0; m < kPfTile / 16; ++m)
+      for (int m = 0; m < kPfTile / 8; ++m)  // the weights' f16 terms, then what they lost
         tc_mma_f16_ta_w<tc_desc_hi(1024) | kSw, Cfg::kIdescO>(
-            tmem + Cfg::kO0, tmem + Cfg::kS0 + (j & 1) * kPfTile + m * 8, vd + ((m * 2048) >> 4),
-            (j > 0 || m > 0) ? 1u : 0u);
+            tmem + Cfg::kO0, tmem + Cfg::kS0 + (j & 1) * kPfTile + m * 8,
+            vd + (((m % (kPfTile / 16)) * 2048) >> 4), (j > 0 || m > 0) ? 1u : 0u);
       tc_commit_w(&kv_free[vi]);
       tc_commit_w(&o_done[j & 1]);
       vi += 2;
@@ -334,7 +336,12 @@ __global__ void __launch_bounds__(kPfThreads, 1)
       if (grow) m = mt;
       const float base = m == -CUDART_INF_F ? 0.f : m;  // nothing visible yet: avoid inf - inf
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
-      uint32_t pk[32];
+      uint32_t pk[32], lo16[32];
+      auto two_terms = [&](int i, float x, float y) {
+        pk[i] = pf_pack(x, y);
+        const float2 r = __half22float2(*reinterpret_cast<const __half2*>(&pk[i]));
+        lo16[i] = pf_pack(x - r.x, y - r.y);
+      };
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float e0 = pf_exp2(__uint_as_float(v0[2 * i]) - base), e1 = pf_exp2(__uint_as_float(v0[2 * i + 1]) - base);
@@ -343,11 +350,12 @@ __global__ void __launch_bounds__(kPfThreads, 1)
         sum[1] += e1;
         sum[2] += e2;
         sum[3] += e3;
-        pk[i] = pf_pack(e0, e1);
-        pk[16 + i] = pf_pack(e2, e3);
+        two_terms(i, e0, e1);
+        two_terms(16 + i, e2, e3);
       }
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       HB_TMEM_ST32(s_addr, pk);
+      HB_TMEM_ST32(s_addr + 32, lo16);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_before_sync();
       __syncwarp();

@@ -167,6 +167,28 @@ def test_prefill_walks_of_one_to_nine_tiles(ctx, oracle, D, ramp):
     assert np.abs(outs[0].cpu().numpy() - ref).max() / np.abs(ref).max() <= (1e-2 if ramp else TOL)
 
 
+@pytest.mark.parametrize("H,Hkv,D,slots,T", [(8, 2, 64, 2000, 40), (4, 1, 128, 1500, 33), (8, 2, 256, 2100, 64)])
+def test_prefill_weights_are_not_rounded_to_f16(ctx, H, Hkv, D, slots, T):
+    """A query and a scale whose product is exact in f16: what is left are the softmax weights, in two
+    f16 terms, and f32 sums.  One f16 term each would show as 2^-11 / sqrt(3) / 1.4 = 2e-4; two leave
+    2^-22, and up to 132 sums of 16 positions in f32 lose at most 2^-23 of the result each: 1.6e-5."""
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    scale = float(np.float32(2.0 ** -4) / np.float32(1.4426950408889634))
+    q = torch.randn(1, T, H, D, device="cuda", generator=gen).half()
+    k, v = (torch.randn(1, Hkv, slots, D, device="cuda", generator=gen).half() for _ in "kv")
+    sl = torch.tensor([slots], dtype=torch.int32, device="cuda")
+    out = flash_attention_prefill(ctx, q, k, v, sl, num_heads=H, num_kv_heads=Hkv, head_dim=D, max_seq_len=slots,
+                                  scale=scale)
+    ctx.check()
+    kd, vd = (x[0].double().repeat_interleave(H // Hkv, 0) for x in (k, v))
+    s = torch.einsum("thd,hnd->htn", q[0].double(), kd) * scale
+    seen = torch.arange(slots, device="cuda") <= slots - T + torch.arange(T, device="cuda")[:, None]
+    ref = torch.einsum("htn,hnd->thd", torch.softmax(s.masked_fill(~seen, float("-inf")), -1), vd)
+    err = float((out[0].double() - ref).norm() / ref.norm())
+    print(f"PREFILL_WEIGHTS D={D} {err:.2e}")
+    assert err <= 3e-5
+
+
 def test_prefill_kv_writer_equals_single_token_calls(ctx):
     lib = _lib.load()
     B, T, H, Hkv, D, slots, base = 2, 7, 8, 2, 64, 40, 500000.0
