@@ -28,6 +28,7 @@
 #include <math_constants.h>
 
 #include <optional>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -152,16 +153,21 @@ struct AttnCfg {
   static constexpr int kSmem = kQBytes + kAttnWarps * kStages * kStageBytes;
 };
 
-// PRECISE: the scaled query and the softmax weights are each split into two f16 terms
-// (hi + lo), doubling the tensor-core work and removing their rounding from the result;
-// K and V are f16 in the cache, so what remains is f32 accumulation error (~1e-6).
-template <int D, bool PRECISE, int NSTAGES>
+// TERMS: which operands are split into two f16 terms (hi + lo), so that their rounding leaves the
+// result; K and V are f16 in the cache.
+//   0  none;
+//   1  the softmax weights, where a call runs with fewer splits than its positions would fill: a
+//      running maximum's weight is exactly 1, fewer of them raised the error by 2 % on average and
+//      up to 6 %; two terms take it to 0.8 of what it was with all splits;
+//   2  the scaled query too (the PRECISE mode): what remains is f32 accumulation error (~1e-6).
+template <int D, int TERMS, int NSTAGES>
 __global__ void __launch_bounds__(kAttnThreads, D >= 256 ? 1 : 2) attn_decode_kernel(const __grid_constant__ AttnParams p) {
   using Cfg = AttnCfg<D, NSTAGES>;
   constexpr int QS = Cfg::kQStride;
   constexpr int NS = Cfg::kStages;
   constexpr int CPR = D / 8;   // 16-byte chunks per row
   constexpr int KS = D / 16;   // k-steps of the score product = m-tiles of the output
+  constexpr bool PRECISE = TERMS == 2;
   extern __shared__ __align__(128) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -353,7 +359,7 @@ __global__ void __launch_bounds__(kAttnThreads, D >= 256 ? 1 : 2) attn_decode_ke
     const uint32_t pb0 = movmatrix_t(ph0);
     const uint32_t pb1 = movmatrix_t(ph1);
     uint32_t pl0 = 0, pl1 = 0;
-    if (PRECISE) {  // what f16 rounding dropped from the softmax weights
+    if (TERMS > 0) {  // what f16 rounding dropped from the softmax weights
       const float2 r0 = __half22float2(*reinterpret_cast<const __half2*>(&ph0));
       const float2 r1 = __half22float2(*reinterpret_cast<const __half2*>(&ph1));
       pl0 = movmatrix_t(pack_h2(p00 - r0.x, p01 - r0.y));
@@ -374,7 +380,7 @@ __global__ void __launch_bounds__(kAttnThreads, D >= 256 ? 1 : 2) attn_decode_ke
         o[s][2] *= al0;
         o[s][3] *= al1;
         mma16816(o[s], a, pb0, pb1);
-        if (PRECISE) mma16816(o[s], a, pl0, pl1);
+        if (TERMS > 0) mma16816(o[s], a, pl0, pl1);
       }
     }
     __syncwarp();  // the stage may be refilled by the next iteration's copies
@@ -676,29 +682,29 @@ static int attn_pick_splits(const hb200_ctx* ctx, int B, int Hkv, int D, int max
   return (int)want;
 }
 
-template <int D, bool PRECISE, int NSTAGES>
+template <int D, int TERMS, int NSTAGES>
 static int attn_launch_ns(hb200_ctx* ctx, const AttnParams& p, cudaStream_t st);
 
-template <int D, bool PRECISE>
+template <int D, int TERMS>
 static int attn_launch(hb200_ctx* ctx, const AttnParams& p, cudaStream_t st) {
   // a grid of more than two waves of single CTAs: share the SMs (3 stages); else 4 stages
   const int grid = p.B * p.Hkv * p.nsplit;
   if constexpr (D >= 256) {
-    return attn_launch_ns<D, PRECISE, 3>(ctx, p, st);  // 4 stages would not fit at this size
+    return attn_launch_ns<D, TERMS, 3>(ctx, p, st);  // 4 stages would not fit at this size
   } else {
-    if (grid > 2 * ctx->sm_count) return attn_launch_ns<D, PRECISE, 3>(ctx, p, st);
-    return attn_launch_ns<D, PRECISE, 4>(ctx, p, st);
+    if (grid > 2 * ctx->sm_count) return attn_launch_ns<D, TERMS, 3>(ctx, p, st);
+    return attn_launch_ns<D, TERMS, 4>(ctx, p, st);
   }
 }
 
 // Clusters of ns CTAs of the decode kernel that the GPU holds at once (a cluster lives in one GPC,
 // whose SMs bound it), asked for once per context.  0: unknown.
-template <int D, bool PRECISE>
+template <int D, int TERMS>
 static int attn_clusters_at_once(hb200_ctx* ctx, int ns) {
   constexpr int kStages = D >= 256 ? 3 : 4;  // as attn_launch picks them for a grid of one wave
   using Cfg = AttnCfg<D, kStages>;
-  const void* kern = reinterpret_cast<const void*>(attn_decode_kernel<D, PRECISE, kStages>);
-  int16_t& known = ctx->attn_clusters[PRECISE][D >= 256 ? 2 : (D >= 128 ? 1 : 0)][ns];
+  const void* kern = reinterpret_cast<const void*>(attn_decode_kernel<D, TERMS, kStages>);
+  int16_t& known = ctx->attn_clusters[TERMS == 2][D >= 256 ? 2 : (D >= 128 ? 1 : 0)][ns];
   if (known == 0) {
     const size_t smem = (size_t)Cfg::kSmem + (D <= 128 ? (size_t)ns * 8 * (D + 2) * sizeof(float) : 0);
     int n = 0;
@@ -734,18 +740,18 @@ static int attn_clusters_at_once(hb200_ctx* ctx, int ns) {
 static int attn_one_wave_splits(hb200_ctx* ctx, int D, bool precise, long pairs, int most) {
   for (int ns = most; ns >= 2; --ns) {
     if (pairs * ns > ctx->sm_count || (ctx->attn_cluster_refused >> ns & 1u)) continue;
-    const int n = D == 64    ? (precise ? attn_clusters_at_once<64, true>(ctx, ns) : attn_clusters_at_once<64, false>(ctx, ns))
-                  : D == 128 ? (precise ? attn_clusters_at_once<128, true>(ctx, ns) : attn_clusters_at_once<128, false>(ctx, ns))
-                             : (precise ? attn_clusters_at_once<256, true>(ctx, ns) : attn_clusters_at_once<256, false>(ctx, ns));
+    const int n = D == 64    ? (precise ? attn_clusters_at_once<64, 2>(ctx, ns) : attn_clusters_at_once<64, 1>(ctx, ns))
+                  : D == 128 ? (precise ? attn_clusters_at_once<128, 2>(ctx, ns) : attn_clusters_at_once<128, 1>(ctx, ns))
+                             : (precise ? attn_clusters_at_once<256, 2>(ctx, ns) : attn_clusters_at_once<256, 1>(ctx, ns));
     if (n >= pairs) return ns;
   }
   return 0;
 }
 
-template <int D, bool PRECISE, int NSTAGES>
+template <int D, int TERMS, int NSTAGES>
 static int attn_launch_ns(hb200_ctx* ctx, const AttnParams& p, cudaStream_t st) {
   using Cfg = AttnCfg<D, NSTAGES>;
-  auto kern = attn_decode_kernel<D, PRECISE, NSTAGES>;
+  auto kern = attn_decode_kernel<D, TERMS, NSTAGES>;
   {
     const int rc = hb_func_smem(ctx, reinterpret_cast<const void*>(kern), (size_t)Cfg::kSmem);
     if (rc != HB200_OK) return rc;
@@ -790,7 +796,7 @@ static int attn_launch_ns(hb200_ctx* ctx, const AttnParams& p, cudaStream_t st) 
     }
     AttnParams q = p;  // ticket path
     q.cluster = 0;
-    return attn_launch_ns<D, PRECISE, NSTAGES>(ctx, q, st);
+    return attn_launch_ns<D, TERMS, NSTAGES>(ctx, q, st);
   }
   HB_CUDA(launch_pdl(kern, dim3(grid), dim3(kAttnThreads), (size_t)Cfg::kSmem, st, ctx->pdl, p));
   if (p.nsplit > 1 && p.tickets == nullptr) {
@@ -865,6 +871,7 @@ static int attn_run(hb200_ctx* ctx, const void* d_q, int q_is_f16, const void* d
   // Beyond 16 splits the cluster would have to shorten the split list; that still wins while a
   // split stays short (<= 48 chunks of 16 positions), measured: 8000 positions in 16 splits +
   // cluster 12.9 us against 62 splits + ticket 17.6 us, 32768 positions 30.8 against 20.0 us.
+  bool fewer = false;  // splits than the positions would fill
   const bool short_splits = p.nsplit <= 16 || (eff_len + kChunk - 1) / kChunk <= 16 * 48;
   if (p.nsplit > 1 && ctx->attn_mode != HB200_ATTN_EXACT) {
     const long pairs = (long)B * Hkv;
@@ -878,6 +885,7 @@ static int attn_run(hb200_ctx* ctx, const void* d_q, int q_is_f16, const void* d
     const int one = attn_one_wave_splits(ctx, D, ctx->attn_mode == HB200_ATTN_PRECISE, pairs, most);
     const bool wave = one > 1 && (small || pairs * one * 10 >= 6L * ctx->sm_count);
     if (wave || small) {
+      fewer = wave && one < (small ? most : p.nsplit);
       p.nsplit = wave ? one : most;
       p.cluster = D <= 128 ? 1 : 2;  // D = 256: the partials reuse the stage region (2 barriers)
     }
@@ -911,17 +919,17 @@ static int attn_run(hb200_ctx* ctx, const void* d_q, int q_is_f16, const void* d
     }
     return HB200_OK;
   }
-  if (ctx->attn_mode == HB200_ATTN_PRECISE) {
-    switch (D) {
-      case 64: return attn_launch<64, true>(ctx, p, st);
-      case 128: return attn_launch<128, true>(ctx, p, st);
-      default: return attn_launch<256, true>(ctx, p, st);
-    }
-  }
+  const int terms = ctx->attn_mode == HB200_ATTN_PRECISE ? 2 : (fewer ? 1 : 0);
+  auto launch = [&](auto d) {
+    constexpr int kD = decltype(d)::value;
+    return terms == 0   ? attn_launch<kD, 0>(ctx, p, st)
+           : terms == 1 ? attn_launch<kD, 1>(ctx, p, st)
+                        : attn_launch<kD, 2>(ctx, p, st);
+  };
   switch (D) {
-    case 64: return attn_launch<64, false>(ctx, p, st);
-    case 128: return attn_launch<128, false>(ctx, p, st);
-    default: return attn_launch<256, false>(ctx, p, st);
+    case 64: return launch(std::integral_constant<int, 64>{});
+    case 128: return launch(std::integral_constant<int, 128>{});
+    default: return launch(std::integral_constant<int, 256>{});
   }
 }
 

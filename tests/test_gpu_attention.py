@@ -167,3 +167,25 @@ def test_exact_mode_is_bit_reproducible(ctx, oracle, B, H, Hkv, D, L, window):
     ctx.check()
     assert np.array_equal(out, mirror)
     _check(out, ref, tol=2e-5)
+
+
+@pytest.mark.parametrize("B,H,Hkv,D,L", [(16, 4, 1, 256, 4096), (32, 2, 2, 128, 3950), (40, 4, 1, 64, 1300)])
+def test_weights_of_fewer_splits_are_not_rounded_to_f16(ctx, B, H, Hkv, D, L):
+    """Calls that run with fewer splits than their positions would fill (so that all run at once) keep
+    the softmax weights in two f16 terms.  A query and a scale whose product is exact in f16 leave
+    only the weights and f32 sums: one f16 term would show as about 2e-4, two leave 2^-22, and at
+    most 256 sums of 16 positions lose up to 2^-23 of the result each: 3e-5."""
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    scale = float(np.float32(2.0 ** -4) / np.float32(1.4426950408889634))
+    q = torch.randn(B, H, D, device="cuda", generator=gen).half()
+    k, v = (torch.randn(B, Hkv, L, D, device="cuda", generator=gen).half() for _ in "kv")
+    sl = torch.full((B,), L, dtype=torch.int32, device="cuda")
+    out = execute_flash_attention_v11(ctx, q, k, v, sl, num_heads=H, num_kv_heads=Hkv, head_dim=D, max_seq_len=L,
+                                      scale=scale)
+    ctx.check()
+    kd, vd = (x.double().repeat_interleave(H // Hkv, 1) for x in (k, v))
+    w = torch.softmax(torch.einsum("bhd,bhnd->bhn", q.double(), kd) * scale, -1)
+    ref = torch.einsum("bhn,bhnd->bhd", w, vd)
+    err = float((out.double() - ref).norm() / ref.norm())
+    print(f"DECODE_WEIGHTS D={D} {err:.2e}")
+    assert err <= 5e-5
