@@ -142,6 +142,18 @@ __device__ __forceinline__ void q4k_expand(const uint32_t (&q)[8], __half2 d, __
   }
 }
 
+// The same by the f32 formula: dmin * m may lie outside f16 although the weight does not.
+template <bool HI>
+__device__ __forceinline__ void q4k_expand_f32(const uint32_t (&q)[8], float d, float c, uint32_t (&o)[16]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t t = HI ? q[i] >> 4 : q[i];
+    auto w = [&](int sh) { return fmaf(d, (float)(t >> sh & 15u), c); };
+    o[2 * i] = as_u32(__floats2half2_rn(w(0), w(16)));
+    o[2 * i + 1] = as_u32(__floats2half2_rn(w(8), w(24)));
+  }
+}
+
 // Four int8 times d, rounded once to f16: bytes biased to 1024 + (q + 128), the bias taken off
 // exactly, then an f16 product (d is an f16, q an integer: the exact product is rounded once).
 // Pairs {0, 2}, {1, 3} as in q4k_expand.
@@ -660,7 +672,11 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
               : "memory");
         };
         uint4 hdr;
-        if constexpr (FMT == 12) hdr = *reinterpret_cast<const uint4*>(blk);
+        bool wide = false;  // a row of this warp whose dmin * 63 f16 does not hold
+        if constexpr (FMT == 12) {
+          hdr = *reinterpret_cast<const uint4*>(blk);
+          wide = __any_sync(0xffffffffu, (hdr.x & 0x7FFF0000u) > 0x640F0000u);  // |dmin| > 1039
+        }
 #pragma unroll
         for (int hh = 0; hh < 2 / kAParts; ++hh) {
           const int half = kAParts == 1 ? hh : (s & 1);
@@ -691,11 +707,16 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
             // exactly up to its own rounding)
             const __half2 dm = __high2half2(as_h2(hdr.x));
             const __half2 cc = __hneg2(__hmul2(dm, mn));
-            const __half2 lost = __hmul2(__hfma2(dm, mn, cc), __floats2half2_rn(-32.f, -32.f));
+            __half2 lost = __hmul2(__hfma2(dm, mn, cc), __floats2half2_rn(-32.f, -32.f));
             const uint32_t qq[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
             const __half2 d = __low2half2(as_h2(hdr.x));
             uint32_t o[16];
             q4k_expand<false>(qq, d, __low2half2(mul), __low2half2(add), __low2half2(cc), o);
+            if (wide) {
+              const float dm32 = -__high2float(as_h2(hdr.x));
+              q4k_expand_f32<false>(qq, __low2float(d) * (float)(sc2 & 63u), dm32 * (float)(m2 & 63u), o);
+              lost = __floats2half2_rn(0.f, 0.f);
+            }
             if (hh == 0) stage_free();
             store16(col0, o);
             asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(
@@ -703,6 +724,10 @@ __global__ void __launch_bounds__(QmCfg<NT, FMT>::kThreads, 1) kq_mma_kernel(con
                          "r"(as_u32(lost))
                          : "memory");
             q4k_expand<true>(qq, d, __high2half2(mul), __high2half2(add), __high2half2(cc), o);
+            if (wide) {
+              const float dm32 = -__high2float(as_h2(hdr.x));
+              q4k_expand_f32<true>(qq, __low2float(d) * (float)(sc2 >> 8), dm32 * (float)(m2 >> 8), o);
+            }
             store16(col0 + 16, o);
           } else {
             // Q8_0 (Hesper/Layers/Linear.lean:6207-6223): blocks 2c and 2c+1 of the row's eight, 34

@@ -141,6 +141,30 @@ def test_few_tokens(ctx, oracle, fmt, K, Ns, M, gate_up):
         assert _check(y, oracle.kquant_matvec(fmt, b, K, n, xn)) < 2e-4
 
 
+@pytest.mark.parametrize("M", [16, 100, 200])
+def test_minima_beyond_f16(ctx, oracle, M):
+    """dmin * m far above f16's largest value, next to weights that f16 holds (d * sc * q cancels it):
+    every third row has such blocks, from the smallest dmin whose product with 63 is out of range."""
+    K, N = 512, 200
+    rng = np.random.default_rng(M)
+    nb = N * (K // 256)
+    d, dmin = np.full(nb, 0.01), np.full(nb, 0.02)
+    sc, m = rng.integers(0, 64, (nb, 8)), rng.integers(0, 64, (nb, 8))
+    q = rng.integers(0, 16, (nb, 256))
+    for i in range(0, nb, 3):
+        if i % 2:  # 60 * 1100 * {14, 15} - 63 * 15000 = -21000, 45000
+            d[i], dmin[i], sc[i], m[i] = 1100.0, 15000.0, 60, 63
+            q[i] = rng.integers(14, 16, 256)
+        else:      # 62 * 75 * {13 .. 15} - 63 * 1040: 65520 rounds to infinity in f16
+            d[i], dmin[i], sc[i], m[i] = 75.0, 1040.0, 62, 63
+            q[i] = rng.integers(13, 16, 256)
+    blocks = formats.q4k_build(d, dmin, sc, m, q).reshape(-1)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    y = LinearLayer.create_from_bytes(ctx, blocks, 12, K, N).forward(_dev(x))
+    ctx.check()
+    assert _check(y, oracle.kquant_matvec(12, blocks, K, N, x)) < 1e-3
+
+
 @pytest.mark.parametrize("fmt", [12, 8])
 @pytest.mark.parametrize("M", [16, 64])
 def test_longest_rows_of_the_batched_product(ctx, oracle, fmt, M):
