@@ -22,6 +22,8 @@ namespace {
 
 PyObject* g_error = nullptr;  // hesper_b200._lib.HesperB200Error
 
+PyObject* g_empty = nullptr;  // ()
+
 struct Fail {};  // a Python error is set
 
 [[noreturn]] void fail(PyObject* type, const std::string& msg) {
@@ -274,42 +276,52 @@ PyObject* kquant_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// (ctx, fmt, gate_blocks, up_blocks, K, N, x, rms_gamma, eps, pre_base, pre_gamma, out, stream);
-// pre_gamma not None: returns (y, x')
+struct Pre {  // pre=(base, gamma) of a call, or None; what is missing in the pair the library refuses
+  bool given;
+  Ref hold;
+  const float *base = nullptr, *gamma = nullptr;
+  explicit Pre(PyObject* o) : given(o != Py_None), hold(PySequence_Fast(given ? o : g_empty, "pre must be a pair")) {
+    if (!given) return;
+    if (PySequence_Fast_GET_SIZE(hold.o) != 2) fail(PyExc_ValueError, "pre must be a pair (base, gamma)");
+    base = fptr(PySequence_Fast_GET_ITEM(hold.o, 0), "pre base");
+    gamma = fptr(PySequence_Fast_GET_ITEM(hold.o, 1), "pre gamma");
+  }
+};
+
+// (ctx, fmt, gate_blocks, up_blocks, K, N, x, rms_gamma, eps, pre, out, stream); pre not None: returns (y, x')
 PyObject* kquant_gateup(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return guarded(n, 13, [&]() -> PyObject* {
+  return guarded(n, 12, [&]() -> PyObject* {
     const long K = as_long(a[4]), N = as_long(a[5]);
     const at::Tensor& x = need(a[6], at::kFloat, "input");
     const long M = rows(x, K);
     float* y;
-    Ref out(output(a[11], x, M, N, &y));
+    const Pre pre(a[9]);
+    Ref out(output(a[10], x, M, N, &y));
     const int fmt = (int)as_long(a[1]);
     const void *wg = ptr(a[2], "blocks"), *wu = ptr(a[3], "blocks");
     const float* gam = fptr(a[7], "rms_gamma");
     const float eps = as_float(a[8]);
     hb200_ctx* ctx = as_ctx(a[0]);
-    hb200_stream st = as_stream(a[12]);
-    if (a[10] == Py_None) {
+    hb200_stream st = as_stream(a[11]);
+    if (!pre.given) {
       call([&] {
         return hb200_kquant_gateup_gelu(ctx, fmt, wg, wu, (int)K, (int)N, x.data_ptr<float>(), (int)M, gam, eps, y, st);
       });
       return out.release();
     }
-    const float *base = fptr(a[9], "pre base"), *pg = fptr(a[10], "pre gamma");
     at::Tensor xo = at::empty_like(x);
     call([&] {
-      return hb200_kquant_gateup_gelu_pre(ctx, fmt, wg, wu, (int)K, (int)N, x.data_ptr<float>(), (int)M, base, pg,
-                                          xo.data_ptr<float>(), gam, eps, y, st);
+      return hb200_kquant_gateup_gelu_pre(ctx, fmt, wg, wu, (int)K, (int)N, x.data_ptr<float>(), (int)M, pre.base,
+                                          pre.gamma, xo.data_ptr<float>(), gam, eps, y, st);
     });
     Ref o2(THPVariable_Wrap(std::move(xo)));
     return PyTuple_Pack(2, out.o, o2.o);
   });
 }
 
-// (ctx, fmt, [(blocks, N)], K, x, rms_gamma, eps, residuals, pre_base, pre_gamma, stream);
-// pre_gamma not None: returns (ys, x')
+// (ctx, fmt, [(blocks, N)], K, x, rms_gamma, eps, residuals, pre, stream); pre not None: returns (ys, x')
 PyObject* kquant_multi(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return guarded(n, 11, [&]() -> PyObject* {
+  return guarded(n, 10, [&]() -> PyObject* {
     const long K = as_long(a[3]);
     const at::Tensor& x = need(a[4], at::kFloat, "input");
     const long M = rows(x, K);
@@ -333,19 +345,19 @@ PyObject* kquant_multi(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const float* gam = fptr(a[5], "rms_gamma");
     const float eps = as_float(a[6]);
     hb200_ctx* ctx = as_ctx(a[0]);
-    hb200_stream st = as_stream(a[10]);
-    if (a[9] == Py_None) {
+    hb200_stream st = as_stream(a[9]);
+    const Pre pre(a[8]);
+    if (!pre.given) {
       call([&] {
         return hb200_kquant_forward_multi(ctx, fmt, segs.data(), (int)nl, (int)K, x.data_ptr<float>(), (int)M, gam,
                                           eps, st);
       });
       return ys.release();
     }
-    const float *base = fptr(a[8], "pre base"), *pg = fptr(a[9], "pre gamma");
     at::Tensor xo = at::empty_like(x);
     call([&] {
       return hb200_kquant_forward_multi_pre(ctx, fmt, segs.data(), (int)nl, (int)K, x.data_ptr<float>(), (int)M,
-                                            base, pg, xo.data_ptr<float>(), gam, eps, st);
+                                            pre.base, pre.gamma, xo.data_ptr<float>(), gam, eps, st);
     });
     Ref o2(THPVariable_Wrap(std::move(xo)));
     return PyTuple_Pack(2, ys.o, o2.o);
@@ -443,4 +455,7 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_binding", "Layer API calls over t
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__binding() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__binding() {
+  g_empty = PyTuple_New(0);
+  return g_empty ? PyModule_Create(&module) : nullptr;
+}

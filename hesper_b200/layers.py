@@ -203,10 +203,9 @@ class LinearLayer:
 
         pre=(base, gamma): the layer input becomes x' = base + rmsnorm(x) * gamma first
         (a post-norm with its residual add); returns (y, x') in that case."""
-        base, pg = pre if pre is not None else (None, None)
         c = gate.ctx
         return c._b.kquant_gateup(c._addr, gate.fmt, gate.blocks, up.blocks, gate.in_dim, gate.out_dim, x,
-                                  rms_gamma, eps, base, pg, out, stream)
+                                  rms_gamma, eps, pre, out, stream)
 
     @staticmethod
     def forward_multi(layers: Sequence["LinearLayer"], x, *, rms_gamma=None, eps: float = 1e-6,
@@ -215,11 +214,10 @@ class LinearLayer:
 
         pre=(base, gamma): the layers' input becomes x' = base + rmsnorm(x) * gamma first;
         returns (ys, x') in that case."""
-        base, pg = pre if pre is not None else (None, None)
         l0 = layers[0]
         c = l0.ctx
         return c._b.kquant_multi(c._addr, l0.fmt, [(l.blocks, l.out_dim) for l in layers], l0.in_dim, x,
-                                 rms_gamma, eps, residuals, base, pg, stream)
+                                 rms_gamma, eps, residuals, pre, stream)
 
 
 def flash_attention_workspace(ctx: Context, B: int, H: int, Hkv: int, D: int, max_seq: int,

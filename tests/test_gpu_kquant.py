@@ -141,6 +141,25 @@ def test_few_tokens(ctx, oracle, fmt, K, Ns, M, gate_up):
         assert _check(y, oracle.kquant_matvec(fmt, b, K, n, xn)) < 2e-4
 
 
+@pytest.mark.parametrize("M", [1, 5, 20])
+def test_half_a_pre_step_is_refused(ctx, M):
+    K, N = 256, 64
+    rng = np.random.default_rng(0)
+    a, b = (LinearLayer.create_from_bytes(ctx, formats.random_kquant(rng, 12, N, K), 12, K, N) for _ in "ab")
+    x, base, gamma = (torch.randn(n, K, device="cuda") for n in (M, M, 1))
+    for pre in ((base, None), (None, gamma), (None, None)):
+        with pytest.raises(hb.HesperB200Error, match="null"):
+            LinearLayer.forward_multi([a, b], x, pre=pre)
+        with pytest.raises(hb.HesperB200Error, match="null"):
+            LinearLayer.forward_fused_gate_up(a, b, x, pre=pre)
+    with pytest.raises(ValueError):
+        LinearLayer.forward_fused_gate_up(a, b, x, pre=(base,))
+    y, xo = LinearLayer.forward_fused_gate_up(a, b, x, pre=(base, gamma))
+    ys, xo2 = LinearLayer.forward_multi([a, b], x, pre=[base, gamma])
+    assert torch.equal(xo, xo2) and y.shape == ys[1].shape == (M, N)
+    ctx.check()
+
+
 @pytest.mark.parametrize("M", [16, 100, 200])
 def test_minima_beyond_f16(ctx, oracle, M):
     """dmin * m far above f16's largest value, next to weights that f16 holds (d * sc * q cancels it):
