@@ -146,6 +146,12 @@ PyObject* guarded(Py_ssize_t n, Py_ssize_t want, F&& f) {
   try {
     return f();
   } catch (const Fail&) {
+  } catch (const c10::OutOfMemoryError& e) {  // as torch.empty raises it
+    PyObject* torch = PyImport_ImportModule("torch");
+    PyObject* type = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
+    if (type) PyErr_SetString(type, e.what_without_backtrace());
+    Py_XDECREF(type);
+    Py_XDECREF(torch);
   } catch (const std::exception& e) {
     PyErr_SetString(PyExc_RuntimeError, e.what());
   }

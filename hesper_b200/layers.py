@@ -237,7 +237,7 @@ def flash_attention_prefill(ctx: Context, q: torch.Tensor, k_cache: torch.Tensor
     seqlens[b]-T .. seqlens[b]-1 of the f16 caches [B, Hkv, max_seq_len, D]; returns [B, T, H, D].
     """
     return ctx._b.attn_prefill(ctx._addr, q, k_cache, v_cache, seqlens, num_heads, num_kv_heads, head_dim,
-                               max_seq_len, scale, window, stream)
+                               max_seq_len, scale, int(window), stream)
 
 
 def execute_flash_attention_v11(ctx: Context, q: torch.Tensor, k_cache: torch.Tensor,
@@ -251,4 +251,4 @@ def execute_flash_attention_v11(ctx: Context, q: torch.Tensor, k_cache: torch.Te
     seqlens [B] int32 (the reference's params[1] = cacheLen, one per sequence).
     """
     return ctx._b.attn_decode(ctx._addr, q, k_cache, v_cache, seqlens, num_heads, num_kv_heads, head_dim,
-                              max_seq_len, scale, window, workspace, out, stream)
+                              max_seq_len, scale, int(window), workspace, out, stream)

@@ -169,6 +169,14 @@ def test_exact_mode_is_bit_reproducible(ctx, oracle, B, H, Hkv, D, L, window):
     _check(out, ref, tol=2e-5)
 
 
+def test_window_takes_what_int_takes(ctx):
+    q, kv = torch.randn(1, 2, 64, device="cuda"), torch.randn(1, 1, 40, 64, device="cuda").half()
+    sl = torch.tensor([40], dtype=torch.int32, device="cuda")
+    outs = [execute_flash_attention_v11(ctx, q, kv, kv, sl, num_heads=2, num_kv_heads=1, head_dim=64, max_seq_len=40,
+                                        scale=0.125, window=w) for w in (16, 16.0, np.int64(16))]
+    assert all(torch.equal(o, outs[0]) for o in outs)
+
+
 @pytest.mark.parametrize("B,H,Hkv,D,L", [(16, 4, 1, 256, 4096), (32, 2, 2, 128, 3950), (40, 4, 1, 64, 1300)])
 def test_weights_of_fewer_splits_are_not_rounded_to_f16(ctx, B, H, Hkv, D, L):
     """Calls that run with fewer splits than their positions would fill (so that all run at once) keep

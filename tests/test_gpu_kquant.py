@@ -160,6 +160,14 @@ def test_half_a_pre_step_is_refused(ctx, M):
     ctx.check()
 
 
+def test_an_output_that_does_not_fit_is_an_out_of_memory_error(ctx):
+    rng = np.random.default_rng(0)
+    layer = LinearLayer.create_from_bytes(ctx, formats.random_kquant(rng, 12, 8, 256), 12, 256, 8)
+    layer.out_dim = 2 ** 31 - 1  # 35 TB of output for 4096 tokens; nothing is launched
+    with pytest.raises(torch.OutOfMemoryError):
+        layer.forward(torch.zeros(4096, 256, device="cuda"))
+
+
 @pytest.mark.parametrize("M", [16, 100, 200])
 def test_minima_beyond_f16(ctx, oracle, M):
     """dmin * m far above f16's largest value, next to weights that f16 holds (d * sc * q cancels it):
