@@ -17,6 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libhesper_b200.so")
 BINDING = os.path.join(HERE, "_binding.so")
+BINDING_TAG = os.path.join(OBJ, "_binding.tag")  # the Python and torch it was built against
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -36,12 +37,28 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _binding_tag() -> str:
+    import torch
+    return f"{sys.version} | torch {torch.__version__} in {os.path.dirname(torch.__file__)}"
+
+
+def binding_stale() -> bool:
+    """Whether _binding.so is missing, older than its sources or built against another Python or torch
+    than those that would load it."""
+    if _stale(BINDING, [os.path.join(CSRC, "py_binding.cpp"), os.path.join(HERE, "..", "include", "hesper_b200.h")]):
+        return True
+    try:
+        with open(BINDING_TAG) as f:
+            return f.read() != _binding_tag()
+    except OSError:
+        return True
+
+
 def build_binding(force: bool = False) -> str:
     """_binding.so, linked against the library beside it and the torch that is installed."""
-    src = os.path.join(CSRC, "py_binding.cpp")
-    header = os.path.join(HERE, "..", "include", "hesper_b200.h")
-    if not (force or _stale(BINDING, [src, header])):
+    if not (force or binding_stale()):
         return BINDING
+    src = os.path.join(CSRC, "py_binding.cpp")
     import sysconfig
 
     import torch
@@ -58,6 +75,8 @@ def build_binding(force: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed: " + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+    with open(BINDING_TAG, "w") as f:
+        f.write(_binding_tag())
     return BINDING
 
 
