@@ -46,6 +46,7 @@ struct PfParams {
   float* out;              // [nseq][T][H][D]
   int q_is_f16;
   int nseq, T, H, Hkv, G, slots, window, ring;
+  int out_bulk;            // out is 16-byte aligned: rows leave by bulk copies, else by float2 stores
   float scale_log2;
   // nsplit > 1: the K/V tiles of a query tile are dealt to nsplit CTAs; each writes its
   // unnormalised partial and its (max, sum), attn_prefill_merge_kernel combines them
@@ -388,9 +389,14 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     if (live) {
       const size_t ri = ((size_t)b * p.T + t) * p.H + h;
       float* dst = p.nsplit > 1 ? p.part_o + (ri * p.nsplit + split) * D : p.out + ri * D;
-      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(orow)),
-                   "n"(D * 4)
-                   : "memory");
+      if (p.nsplit > 1 || p.out_bulk) {
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(orow)),
+                     "n"(D * 4)
+                     : "memory");
+      } else {
+        for (int c = 0; c < D; c += 2)
+          *reinterpret_cast<float2*>(dst + c) = *reinterpret_cast<const float2*>(orow + c);
+      }
       if (p.nsplit > 1)
         *reinterpret_cast<float2*>(p.part_ml + (ri * p.nsplit + split) * 2) = make_float2(m, l);
     }
@@ -491,7 +497,7 @@ int hb_attn_prefill_tiled(hb200_ctx* ctx, const void* d_q, int q_is_f16, const v
   if (!(D == 64 || D == 128 || D == 256)) return 1;
   if (nseq > 65535 || Hkv > 65535 || (long)nseq * Hkv * slots >= (1l << 31)) return 1;
   if (q_is_f16 ? (reinterpret_cast<uintptr_t>(d_q) & 3) : (reinterpret_cast<uintptr_t>(d_q) & 15)) return 1;
-  if (reinterpret_cast<uintptr_t>(d_out) & 15) return 1;  // rows leave by bulk copies
+  if (reinterpret_cast<uintptr_t>(d_out) & 7) return 1;
   TcEncodeTiledFn encode = tc_tensor_map_encoder();
   if (encode == nullptr) return 1;
   PfParams p = {};
@@ -518,6 +524,7 @@ int hb_attn_prefill_tiled(hb200_ctx* ctx, const void* d_q, int q_is_f16, const v
   p.slots = slots;
   p.window = window;
   p.ring = ring;
+  p.out_bulk = (reinterpret_cast<uintptr_t>(d_out) & 15) == 0;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = ctx->d_status;
   const int TQ = kPfRows / G;

@@ -189,6 +189,32 @@ def test_prefill_weights_are_not_rounded_to_f16(ctx, H, Hkv, D, slots, T):
     assert err <= 3e-5
 
 
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("workspace", [False, True])
+def test_prefill_output_aligned_to_eight_bytes(ctx, D, workspace):
+    """An output on an 8-byte boundary takes the same kernel, also without a workspace (the route of one
+    decode query per token could not do without one)."""
+    lib = _lib.load()
+    H, Hkv, T, slots = 4, 2, 37, 700
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    q = torch.randn(1, T, H, D, device="cuda", generator=gen)
+    k, v = (torch.randn(1, Hkv, slots, D, device="cuda", generator=gen).half() for _ in "kv")
+    sl = torch.tensor([slots - 5], dtype=torch.int32, device="cuda")
+    n = int(lib.hb200_attn_prefill_workspace_bytes(ctx.handle, 1, T, H, Hkv, D, slots)) if workspace else 0
+    ws = torch.empty(max(n, 16), dtype=torch.uint8, device="cuda")
+    outs = []
+    for shift in (0, 2):
+        buf = torch.full((T * H * D + 8,), 7.0, device="cuda")
+        rc = lib.hb200_attn_prefill(ctx.handle, q.data_ptr(), 0, k.data_ptr(), v.data_ptr(), sl.data_ptr(), 1, T, H,
+                                    Hkv, D, slots, 0, C.c_float(D ** -0.5), ws.data_ptr() if n else None,
+                                    C.c_size_t(n), buf.data_ptr() + 4 * shift, None)
+        assert rc == 0, lib.hb200_last_error()
+        ctx.check()
+        assert bool((buf[:shift] == 7).all()) and bool((buf[shift + T * H * D:] == 7).all())
+        outs.append(buf[shift:shift + T * H * D])
+    assert torch.equal(*outs)
+
+
 def test_prefill_kv_writer_equals_single_token_calls(ctx):
     lib = _lib.load()
     B, T, H, Hkv, D, slots, base = 2, 7, 8, 2, 64, 40, 500000.0
