@@ -753,6 +753,12 @@ static int kq_forward_multi_impl(hb200_ctx* ctx, int fmt, const hb200_kquant_seg
   const int rowbytes = kq_rowbytes(fmt, K);
   KQPlan plan;
   if (!kq_plan(ctx, rows, K, M, rowbytes, false, pre.gamma != nullptr, &plan)) {
+    if (M > 1 && M < kKQBatchedFrom && !ctx->no_mma) {  // captured: only that kernel takes the row
+      ScratchUse use(ctx, st);
+      rc = hb_kq_sb_run(ctx, fmt, segs, nseg, K, 0, d_x, M, pre.base, pre.gamma, pre.out, d_rms_gamma, rms_eps,
+                        static_cast<uint8_t*>(ctx->d_scratch) + kScratchLmSplit, st);
+      if (rc <= 0) return rc;
+    }
     set_error("kquant: K=%d does not fit the shared-memory budget", K);
     return HB200_ERR_UNSUPPORTED;
   }
@@ -841,6 +847,12 @@ static int kq_gateup_impl(hb200_ctx* ctx, int fmt, const void* d_blocks_gate,
   const int rowbytes = kq_rowbytes(fmt, K);
   KQPlan plan;
   if (!kq_plan(ctx, N, K, M, rowbytes, true, pre.gamma != nullptr, &plan)) {
+    if (M > 1 && M < kKQBatchedFrom && !ctx->no_mma) {
+      ScratchUse use(ctx, st);
+      rc = hb_kq_sb_run(ctx, fmt, gs, 2, K, 1, d_x, M, pre.base, pre.gamma, pre.out, d_rms_gamma, rms_eps,
+                        static_cast<uint8_t*>(ctx->d_scratch) + kScratchLmSplit, st);
+      if (rc <= 0) return rc;
+    }
     set_error("kquant gate/up: K=%d does not fit the shared-memory budget", K);
     return HB200_ERR_UNSUPPORTED;
   }

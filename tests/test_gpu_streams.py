@@ -105,3 +105,23 @@ def test_decode_graph_of_a_few_sequences_beside_another_stream(ctx):
         assert all(torch.equal(o, ref) for o in outs)
     ctx.check()
     model.close()
+
+
+@pytest.mark.parametrize("gate_up", [False, True])
+def test_captured_rows_too_long_for_the_streaming_kernel(ctx, gate_up):
+    """Rows that only the kernel for a few tokens takes are captured on it, with the context's scratch
+    as the batched products are."""
+    rng = np.random.default_rng(3)
+    K, N, M = 16384, 40, 5
+    a, b = (LinearLayer.create_from_bytes(ctx, formats.random_kquant(rng, 8, N, K), 8, K, N) for _ in "ab")
+    x = torch.randn(M, K, device="cuda")
+
+    def call():
+        return LinearLayer.forward_fused_gate_up(a, b, x) if gate_up else a.forward(x)
+    want, g = call(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        got = call()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    ctx.check()
