@@ -286,7 +286,7 @@ struct hb200_ctx {
   bool no_mma;         // HB200_NO_MMA=1: keep batched ternary products on the dp4a kernel
   int mv_mode;         // HB200_MV: 0 never the tensor-core matvec, 1 where it measured faster, 2 wherever it fits
   size_t smem_per_sm;  // shared memory of one SM (two co-resident launches must fit in it)
-  // dynamic shared memory already granted to each kernel in this context's CUDA context
+  // most dynamic shared memory of each kernel, granted in this context's CUDA context
   // (the attribute is per device and per context, so it cannot live in a process-wide static)
   struct FuncSmem {
     const void* func;
@@ -306,7 +306,7 @@ struct hb200_ctx {
   bool adopted;                   // lives in the caller's own CUDA context: never switch devices
 };
 
-// Raises cudaFuncAttributeMaxDynamicSharedMemorySize of `func` to `bytes` once per context.
+// Raises cudaFuncAttributeMaxDynamicSharedMemorySize of `func`, once per context, and checks `bytes`.
 int hb_func_smem(struct hb200_ctx* ctx, const void* func, size_t bytes);
 bool hb_func_flag(struct hb200_ctx* ctx, const void* func);
 void hb_func_set_flag(struct hb200_ctx* ctx, const void* func);

@@ -26,17 +26,20 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 }  // namespace hb
 
+// The attribute belongs to the CUDA context, which several hb200 contexts may share: whoever sets it
+// sets it to the most a block can have, so that none takes back what another relies on.
 int hb_func_smem(hb200_ctx* ctx, const void* func, size_t bytes) {
-  for (int i = 0; i < ctx->n_func_smem; ++i) {
-    if (ctx->func_smem[i].func == func) {
-      if (ctx->func_smem[i].bytes >= bytes) return HB200_OK;
-      HB_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-      ctx->func_smem[i].bytes = bytes;
-      return HB200_OK;
-    }
+  size_t most = 0;
+  for (int i = 0; i < ctx->n_func_smem && most == 0; ++i)
+    if (ctx->func_smem[i].func == func) most = ctx->func_smem[i].bytes;
+  if (most == 0) {
+    cudaFuncAttributes a;
+    HB_CUDA(cudaFuncGetAttributes(&a, func));
+    most = (size_t)ctx->smem_optin - a.sharedSizeBytes;
+    HB_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    if (ctx->n_func_smem < 96) ctx->func_smem[ctx->n_func_smem++] = {func, most, false};
   }
-  HB_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  if (ctx->n_func_smem < 96) ctx->func_smem[ctx->n_func_smem++] = {func, bytes, false};
+  HB_REQUIRE(bytes <= most, "a kernel needs %zu bytes of shared memory, a block has %zu", bytes, most);
   return HB200_OK;
 }
 

@@ -141,6 +141,24 @@ def test_few_tokens(ctx, oracle, fmt, K, Ns, M, gate_up):
         assert _check(y, oracle.kquant_matvec(fmt, b, K, n, xn)) < 2e-4
 
 
+def test_two_contexts_share_a_kernel_of_different_shared_memory(oracle, monkeypatch):
+    """Two contexts of one GPU, the same kernel with much and with little shared memory: neither's call
+    takes the other's back."""
+    monkeypatch.setenv("HB200_NO_MMA", "1")
+    rng = np.random.default_rng(8)
+    big, small = hb.Context(0), hb.Context(0)
+    wb, ws = formats.random_kquant(rng, 12, 10240, 2560), formats.random_kquant(rng, 12, 8, 256)
+    lb, ls = LinearLayer.create_from_bytes(big, wb, 12, 2560, 10240), LinearLayer.create_from_bytes(small, ws, 12, 256, 8)
+    x = rng.standard_normal((2, 2560)).astype(np.float32)
+    ref = oracle.kquant_matvec(12, wb, 2560, 10240, x)
+    _check(lb.forward(_dev(x)), ref)
+    ls.forward(torch.zeros(2, 256, device="cuda"))
+    _check(lb.forward(_dev(x)), ref)
+    for c in (big, small):
+        c.check()
+        c.close()
+
+
 @pytest.mark.parametrize("M", [1, 5, 20])
 def test_half_a_pre_step_is_refused(ctx, M):
     K, N = 256, 64
