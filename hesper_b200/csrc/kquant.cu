@@ -595,12 +595,21 @@ static int kq_batched_fused(hb200_ctx* ctx, int fmt, const KQBatchSeg* segs, int
 }
 
 // Whether 2 to 15 tokens take the kernel of kquant_sb.cu rather than this one, whose time grows by
-// a whole product per token.  Measured, us (this / that kernel): Q4_K K=2560 N=10240 at 2, 7, 15
-// tokens 10.1 / 9.2, 28.9 / 9.3, 58.7 / 11.8; Q8_0 12.8 / 10.6, 36.9 / 11.7, 74.7 / 12.2; Q4_K
-// K=10240 N=2560 14.2 / 15.7, 45.5 / 15.7, 95.6 / 17.8; K=2560 N=512 4.8 / 5.0, 13.9 / 5.0, 28.5 / 5.6.
-// So only two tokens on Q4_K with fewer rows than K stay.
+// a whole product per token.  Measured, us (this / that kernel, weights from memory): Q4_K K=2560 N=10240
+// at 2, 3, 7, 15 tokens 10.6 / 9.9, 14.5 / 10.0, 28.9 / 9.3, 58.7 / 11.8; Q8_0 13.5 / 11.8, 18.4 / 11.8,
+// 36.9 / 11.7, 74.7 / 12.2; the smallest, K=2560 N=512, at 3: Q4_K 6.8 / 5.7, Q8_0 6.7 / 5.5.  Two tokens
+// repeat the product once only, which the other kernel's staging launch has to earn back:
+//   Q8_0  from 10 M weights on: K x N = 2560 x 2048 5.5 / 6.3, 4096 x 1024 6.8 / 7.4, 5120 x 1024 8.0 /
+//         8.4, but 2560 x 4096 7.0 / 7.2, 5120 x 2048 9.7 / 8.6, 10240 x 1024 13.0 / 13.3, 1024 x 10240
+//         7.9 / 6.8, 10240 x 2560 19.3 / 15.7;
+//   Q4_K  (half the bytes) many rows, or rows at least as many as K from 16 M weights on: 2560 x 2560 5.9
+//         / 6.9, 2560 x 4096 6.1 / 6.9, 2560 x 6144 7.3 / 7.5, 10240 x 2560 14.2 / 15.7, but 4096 x 4096
+//         8.8 / 8.7, 1024 x 4096 4.8 / 4.7, 1024 x 10240 7.2 / 6.0.
 static bool kq_few_tokens(const hb200_ctx* ctx, int fmt, long rows, int K, int M) {
-  return M >= 2 && M < kKQBatchedFrom && !ctx->no_mma && (M > 2 || fmt == HB200_FMT_Q8_0 || rows >= K);
+  if (M < 2 || M >= kKQBatchedFrom || ctx->no_mma) return false;
+  if (M > 2) return true;
+  if (fmt == HB200_FMT_Q8_0) return rows * K >= 10000000L;
+  return rows >= 4L * K || (rows >= K && rows * K >= 16000000L);
 }
 
 // ---- host side --------------------------------------------------------------------

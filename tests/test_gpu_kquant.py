@@ -110,6 +110,9 @@ def test_gate_up_gelu(ctx, oracle, fmt, K, N, M):
     (512, [148 * 128 + 37], 15, False),  # two passes per CTA, the second one ragged
     (1024, [148 * 64 + 11], 3, True),    # gate/up, two passes
     (2560, [333], 12, True), (2560, [2600], 2, False),
+    # two tokens on either side of the rule: Q8_0 10 M weights; Q4_K rows >= 4 K, 16 M weights
+    (1024, [9765], 2, False), (1024, [9766], 2, False), (768, [3071], 2, False), (768, [3072], 2, False),
+    (3840, [4166], 2, False), (3840, [4167], 2, False), (1024, [2047], 2, True), (1024, [2048], 2, True),
     # the ring of weights wraps (tests/test_kquant_few_tokens_plan.py): one tile per CTA and fewer
     # stages than warps; unequal tensors; several laps; two passes
     (4096, [2304], 15, False), (9216, [2304], 9, False), (4096, [1152], 12, True),
