@@ -25,6 +25,7 @@
 //     to the workspace and a small combine kernel merges the splits (today: the last split to
 //     arrive merges them, or, for small grids, a thread-block cluster merges through the
 //     leader's shared memory).
+#include <limits.h>
 #include <math_constants.h>
 
 #include <optional>
@@ -881,9 +882,16 @@ static int attn_run(hb200_ctx* ctx, const void* d_q, int q_is_f16, const void* d
     // once per wave, and a second wave of clusters holds few.  Measured, us, splits chosen so against
     // before, D = 256: 8 pairs x 8192 positions 10 splits 17.9, 16 24.3; 16 x 4096 6 16.4, 16 27.8; 32 x
     // 2048 4 15.1, 8 26.5; 64 x 8192 2 72.9, 5 82.7 (30 positions 6.3, 7.3); D = 128: 20 x 2100 6 8.5,
-    // 16 11.3.  Long splits need most of the SMs at work: the line is 60 %.
+    // 16 11.3.  But a CTA by itself does not get an SM's bandwidth out of narrow rows: splits longer than
+    // the lines below stay as they were.  D = 64: 16 pairs x 8000 11.8, 14.8, 37 x 2000 9.0, 10.8, 37 x 4000
+    // 13.7, 11.0, 49 x 14000 44.7, 29.8; D = 128: 27 x 8000 23.3, 26.2, 37 x 4000 17.2, 19.8, 37 x 8000
+    // 29.1, 25.7; D = 256: 49 x 8000 62, 64, 49 x 14000 102, 97, 64 x 14000 (more SMs at work) 101, 125.
+    // D = 64 also has several CTAs of a short cluster on an SM: 27 x 1000 in 7 splits 6.1, 5 6.4.
     const int one = attn_one_wave_splits(ctx, D, ctx->attn_mode == HB200_ATTN_PRECISE, pairs, most);
-    const bool wave = one > 1 && (small || pairs * one * 10 >= 6L * ctx->sm_count);
+    const long busy = pairs * one, each = one > 1 ? eff_len / one : 0;
+    const long longest = D == 64 ? 1200 : (D == 128 ? 2100 : (busy * 10 >= 8L * ctx->sm_count ? LONG_MAX : 4000));
+    const bool fits = D == 64 && small && (most <= 4 || pairs * most * 2 <= 3L * ctx->sm_count);
+    const bool wave = one > 1 && !fits && each <= longest && (small || busy * 10 >= 6L * ctx->sm_count);
     if (wave || small) {
       fewer = wave && one < (small ? most : p.nsplit);
       p.nsplit = wave ? one : most;

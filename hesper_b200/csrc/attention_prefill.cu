@@ -1,4 +1,5 @@
-// attention_prefill.cu -- causal GQA attention of a prompt chunk on the 5th-generation tensor cores.
+// attention_prefill.cu -- causal GQA attention of a prompt chunk on the 5th-generation tensor cores;
+// chunks too small for it go to attention_prefill_mma.cu (pf_use_mma).
 //
 // T new query tokens per sequence against the f16 KV cache that already holds them (the role
 // of the reference's batched prefill kernels, flashAttentionBatchKernelF16 and its SWA variant,
@@ -30,6 +31,7 @@
 // idle the positions are dealt to several CTAs and a second kernel merges their partials.
 #include <math_constants.h>
 
+#include "attention_prefill.cuh"
 #include "tcgen05.cuh"
 
 namespace hb {
@@ -464,10 +466,47 @@ static int pf_pick_splits(const hb200_ctx* ctx, int nseq, int T, int H, int Hkv,
   return ns < 1 ? 1 : (int)ns;
 }
 
+// Positions of a cache that the tokens of a chunk see between them, at most.
+static long pf_span(int T, int slots, int window) {
+  return window > 0 && (long)window + T < slots ? (long)window + T : slots;
+}
+
+// Whether the mma.sync kernel (attention_prefill_mma.cu) takes a chunk.  The kernel here costs more to
+// start, holds an SM by itself and, at 128 rows a CTA, has half as many of them to deal; its tiles
+// are the cheaper the wider the head.  Device times over 223 shapes (1 to 20 KV heads x sequences of 4
+// query heads, 8 to 400 tokens, 16 to 8000 positions) give, in us,
+//   here  5.8 + 1.15 t w    D = 128: 7.8 + 1.2 t w     t tiles of a CTA, w waves of CTAs
+//   mma   3.8 + (0.47 + 0.72 c) t    5.8 + (0.62 + 1.05 c) t    c CTAs per SM, at least 1
+// and for the merge of splits 1.8 + 0.8 and 1.4 + 2.6 (1.5 + 1.0 and 0.8 + 1.75) per MB of partials,
+// within 10 %.  Measured, mma / here: D = 64 8 tokens x 16 positions 4.8 / 6.7, 40 x 300 9.3 / 11.0,
+// 20 pairs 100 x 8000 109 / 154, but 400 x 8000 40.5 / 22.1; D = 128 40 x 80 9.6 / 12.1, 400 x 1000 17.3 /
+// 16.0.  D = 256: only where a tile or two are all there is, 40 x 80 14.8 / 18.3, 16 x 300 21.7 / 16.5.
+static bool pf_use_mma(const hb200_ctx* ctx, int nseq, int T, int H, int Hkv, int D, int slots, int window) {
+  const long span = pf_span(T, slots, window);
+  if (D == 256) return span <= 128;
+  const int G = H / Hkv, sms = ctx->sm_count;
+  const float mb = (float)nseq * T * H * D * 4e-6f;
+  auto qtiles = [&](int rows) { return (long)((T + rows / G - 1) / (rows / G)) * Hkv * nseq; };
+  const long tiles = (span + 63) / 64, cn = qtiles(kPfRows), co = qtiles(kPmRows);
+  const int nn = pf_pick_splits(ctx, nseq, T, H, Hkv, slots, window);
+  const int no = hb_attn_prefill_mma_splits(ctx, nseq, T, G, Hkv, D, span);
+  const float tn = (float)((tiles + nn - 1) / nn * ((cn * nn + sms - 1) / sms));
+  const float to = (float)((tiles + no - 1) / no), c = fmaxf(1.f, (float)(co * no) / sms);
+  const bool d64 = D == 64;
+  const float here = (d64 ? 5.8f + 1.15f * tn : 7.8f + 1.2f * tn) +
+                     (nn > 1 ? (d64 ? 1.8f + 0.8f * nn * mb : 1.5f + 1.0f * nn * mb) : 0.f);
+  const float mma = (d64 ? 3.8f + (0.47f + 0.72f * c) * to : 5.8f + (0.62f + 1.05f * c) * to) +
+                    (no > 1 ? (d64 ? 1.4f + 2.6f * no * mb : 0.8f + 1.75f * no * mb) : 0.f);
+  return mma < here;
+}
+
 size_t hb_attn_prefill_tiled_ws(const hb200_ctx* ctx, int nseq, int T, int H, int Hkv, int D,
                                 int slots) {
   if (H % Hkv || H / Hkv > 8) return 0;
-  const int ns = pf_pick_splits(ctx, nseq, T, H, Hkv, slots, 0);
+  // of the kernels' split counts the larger one: a window may change which of them runs
+  int ns = pf_pick_splits(ctx, nseq, T, H, Hkv, slots, 0);
+  const int no = hb_attn_prefill_mma_splits(ctx, nseq, T, H / Hkv, Hkv, D, slots);
+  if (no > ns) ns = no;
   return ns > 1 ? (size_t)nseq * T * H * ns * ((size_t)D + 2) * sizeof(float) + 256 : 0;
 }
 
@@ -477,15 +516,19 @@ static int pf_launch(hb200_ctx* ctx, const PfParams& p, dim3 grid, cudaStream_t 
   if (rc) return rc;
   HB_CUDA(launch_pdl(attn_prefill_tiled_kernel<D>, grid, dim3(kPfThreads), (size_t)PfCfg<D>::kSmem, st,
                      ctx->pdl, p));
-  if (p.nsplit > 1) {
-    const long rows = (long)p.nseq * p.T * p.H;
-    HB_CUDA(launch_pdl(attn_prefill_merge_kernel<D>, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, st,
-                       ctx->pdl, (const float*)p.part_o, (const float*)p.part_ml, p.nsplit, rows, p.out));
-  }
   return HB200_OK;
 }
 
-// Causal attention of T query tokens per sequence on the tiled kernel.  HB200_OK when the
+static int pf_merge(hb200_ctx* ctx, const float* part_o, const float* part_ml, int nsplit, long rows, int D,
+                    float* out, cudaStream_t st) {
+  auto kern = D == 64 ? attn_prefill_merge_kernel<64> : (D == 128 ? attn_prefill_merge_kernel<128>
+                                                                  : attn_prefill_merge_kernel<256>);
+  HB_CUDA(launch_pdl(kern, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, st, ctx->pdl, part_o, part_ml, nsplit,
+                     rows, out));
+  return HB200_OK;
+}
+
+// Causal attention of T query tokens per sequence on a tiled kernel.  HB200_OK when the
 // launch was made, 1 when the shape is outside what it covers (the caller runs every token as a
 // decode query instead), < 0 on error.
 int hb_attn_prefill_tiled(hb200_ctx* ctx, const void* d_q, int q_is_f16, const void* d_k,
@@ -495,22 +538,42 @@ int hb_attn_prefill_tiled(hb200_ctx* ctx, const void* d_q, int q_is_f16, const v
   const int G = H / Hkv;
   if (!(G == 1 || G == 2 || G == 4 || G == 8)) return 1;
   if (!(D == 64 || D == 128 || D == 256)) return 1;
-  if (nseq > 65535 || Hkv > 65535 || (long)nseq * Hkv * slots >= (1l << 31)) return 1;
+  if (nseq > 65535 || Hkv > 65535) return 1;
   if (q_is_f16 ? (reinterpret_cast<uintptr_t>(d_q) & 3) : (reinterpret_cast<uintptr_t>(d_q) & 15)) return 1;
   if (reinterpret_cast<uintptr_t>(d_out) & 7) return 1;
   TcEncodeTiledFn encode = tc_tensor_map_encoder();
-  if (encode == nullptr) return 1;
+  const bool mma = encode == nullptr || (long)nseq * Hkv * slots >= (1l << 31) ||  // rows of a tensor map
+                   pf_use_mma(ctx, nseq, T, H, Hkv, D, slots, window);
+  int nsplit = mma ? hb_attn_prefill_mma_splits(ctx, nseq, T, G, Hkv, D, pf_span(T, slots, window))
+                   : pf_pick_splits(ctx, nseq, T, H, Hkv, slots, window);
+  if (nsplit > 1) {
+    // never more than the workspace holds (a caller may have sized it for another T)
+    const size_t per = (size_t)nseq * T * H * ((size_t)D + 2) * sizeof(float);
+    if (d_ws == nullptr || (reinterpret_cast<uintptr_t>(d_ws) & 15)) nsplit = 1;
+    else if ((size_t)nsplit * per > ws_bytes) nsplit = ws_bytes / per < 1 ? 1 : (int)(ws_bytes / per);
+  }
+  const long rows = (long)nseq * T * H;
+  float* const part_o = nsplit > 1 ? static_cast<float*>(d_ws) : nullptr;
+  float* const part_ml = nsplit > 1 ? part_o + (size_t)rows * nsplit * D : nullptr;
+  const float scale_log2 = scale * 1.4426950408889634f;
+  int rc;
+  if (mma) {
+    const PmParams p = {d_q, static_cast<const __half*>(d_k), static_cast<const __half*>(d_v), d_seqlens, d_out,
+                        q_is_f16, nseq, T, H, Hkv, G, slots, window, ring, scale_log2, nsplit, part_o, part_ml};
+    rc = hb_attn_prefill_mma(ctx, p, D, st);
+    return rc || nsplit == 1 ? rc : pf_merge(ctx, part_o, part_ml, nsplit, rows, D, d_out, st);
+  }
   PfParams p = {};
   const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)nseq * Hkv * slots};
   const cuuint64_t strides[1] = {(cuuint64_t)D * 2};
   const cuuint32_t box[2] = {64, kPfTile};
   const cuuint32_t estr[2] = {1, 1};
   for (int i = 0; i < 2; ++i) {
-    const CUresult rc = encode(i ? &p.tmv : &p.tmk, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
-                               const_cast<void*>(i ? d_v : d_k), dims, strides, box, estr,
-                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    HB_REQUIRE(rc == CUDA_SUCCESS, "attn (prefill): cuTensorMapEncodeTiled failed (%d)", (int)rc);
+    const CUresult erc = encode(i ? &p.tmv : &p.tmk, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
+                                const_cast<void*>(i ? d_v : d_k), dims, strides, box, estr,
+                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    HB_REQUIRE(erc == CUDA_SUCCESS, "attn (prefill): cuTensorMapEncodeTiled failed (%d)", (int)erc);
   }
   p.q = d_q;
   p.seqlens = d_seqlens;
@@ -525,24 +588,15 @@ int hb_attn_prefill_tiled(hb200_ctx* ctx, const void* d_q, int q_is_f16, const v
   p.window = window;
   p.ring = ring;
   p.out_bulk = (reinterpret_cast<uintptr_t>(d_out) & 15) == 0;
-  p.scale_log2 = scale * 1.4426950408889634f;
+  p.scale_log2 = scale_log2;
   p.status = ctx->d_status;
+  p.nsplit = nsplit;
+  p.part_o = part_o;
+  p.part_ml = part_ml;
   const int TQ = kPfRows / G;
-  p.nsplit = pf_pick_splits(ctx, nseq, T, H, Hkv, slots, window);
-  if (p.nsplit > 1) {
-    // never more than the workspace holds (a caller may have sized it for another T)
-    const size_t per = (size_t)nseq * T * H * ((size_t)D + 2) * sizeof(float);
-    if (d_ws == nullptr || (reinterpret_cast<uintptr_t>(d_ws) & 15)) p.nsplit = 1;
-    else if ((size_t)p.nsplit * per > ws_bytes) p.nsplit = ws_bytes / per < 1 ? 1 : (int)(ws_bytes / per);
-  }
-  if (p.nsplit > 1) {
-    p.part_o = static_cast<float*>(d_ws);
-    p.part_ml = p.part_o + (size_t)nseq * T * H * p.nsplit * (size_t)D;
-  }
   const dim3 grid((unsigned)((T + TQ - 1) / TQ) * p.nsplit, (unsigned)Hkv, (unsigned)nseq);
-  switch (D) {
-    case 64: return pf_launch<64>(ctx, p, grid, st);
-    case 128: return pf_launch<128>(ctx, p, grid, st);
-    default: return pf_launch<256>(ctx, p, grid, st);
-  }
+  rc = D == 64 ? pf_launch<64>(ctx, p, grid, st)
+       : D == 128 ? pf_launch<128>(ctx, p, grid, st)
+                  : pf_launch<256>(ctx, p, grid, st);
+  return rc || nsplit == 1 ? rc : pf_merge(ctx, part_o, part_ml, nsplit, rows, D, d_out, st);
 }
