@@ -68,7 +68,10 @@ struct PfCfg {
   static constexpr int kOutStride = D * 4 + 16;             // padded f32 row of the epilogue
   static constexpr int kRing = kSlots * kSlotBytes;
   static constexpr int kData = kRing > kPfRows * kOutStride ? kRing : kPfRows * kOutStride;
-  static constexpr int kSmem = 1024 + kData;
+  // D = 128 takes all of tensor memory: a second CTA of an SM, placed there early beside the kernel
+  // before, would only wait for the first.  More than half of the shared memory keeps it off.
+  static constexpr int kSmem = D == 128 ? 118784 : 1024 + kData;
+  static_assert(1024 + kData <= kSmem, "shared memory of a CTA");
   static constexpr uint32_t kIdescS = (1u << 4) | ((uint32_t)(kPfTile >> 3) << 17) | ((uint32_t)(kPfRows >> 4) << 24);
   // B (= V) is MN-major
   static constexpr uint32_t kIdescO =
