@@ -889,7 +889,7 @@ static int attn_run(hb200_ctx* ctx, const void* d_q, int q_is_f16, const void* d
     // D = 64 also has several CTAs of a short cluster on an SM: 27 x 1000 in 7 splits 6.1, 5 6.4.
     const int one = attn_one_wave_splits(ctx, D, ctx->attn_mode == HB200_ATTN_PRECISE, pairs, most);
     const long busy = pairs * one, each = one > 1 ? eff_len / one : 0;
-    const long longest = D == 64 ? 1200 : (D == 128 ? 2100 : (busy * 10 >= 8L * ctx->sm_count ? LONG_MAX : 4000));
+    const long longest = D == 64 ? 950 : (D == 128 ? 2100 : (busy * 10 >= 8L * ctx->sm_count ? LONG_MAX : 4000));
     const bool fits = D == 64 && small && (most <= 4 || pairs * most * 2 <= 3L * ctx->sm_count);
     const bool wave = one > 1 && !fits && each <= longest && (small || busy * 10 >= 6L * ctx->sm_count);
     if (wave || small) {
