@@ -602,6 +602,7 @@ few GB, so that a full-metric capture of one to three launches ends in a minute.
   i2s_mma  64-token ternary product on the tensor cores, ring of 40 matrices (177 MB), 2 passes
   lmhead64 64-token LM head on the tensor cores, one bf16 table V=128256 K=2560 (657 MB), 3 calls
   q4k_b32  32-token Q4_K product on the tensor cores, ring of 12 matrices, 2 passes
+  q80_m7   7-token Q8_0 product (the kernel for a few tokens), ring of 8 matrices (223 MB), 2 passes
   bitnet1 / bitnet64   BitNet-2B-shaped decode loop at batch 1 / 64: 2 prompt positions and
            3 new tokens, launched one by one (no graph) so that a launch list sees each kernel
   gemma1 / gemma32 / gemma256   Gemma-4-E4B-shaped Q4_K decode loop (one rank): 3 tokens at
@@ -640,11 +641,12 @@ def run_case(name: str) -> int:
         for _ in range(3):
             for l in layers:
                 l.forward(x, out=y)
-    elif name == "q4k_b32":
-        K, N, R, M = 2560, 10240, 12, 32
-        base = torch.from_numpy(formats.random_kquant(rng, 12, N, K)).cuda()
-        rb = formats.kquant_row_bytes(12, K)
-        layers = [hb.LinearLayer(ctx, torch.roll(base, r * rb), 12, K, N) for r in range(R)]
+    elif name in ("q4k_b32", "q80_m7"):
+        fmt, R, M = (12, 12, 32) if name == "q4k_b32" else (8, 8, 7)
+        K, N = 2560, 10240
+        base = torch.from_numpy(formats.random_kquant(rng, fmt, N, K)).cuda()
+        rb = formats.kquant_row_bytes(fmt, K)
+        layers = [hb.LinearLayer(ctx, torch.roll(base, r * rb), fmt, K, N) for r in range(R)]
         x = torch.randn(M, K, device="cuda")
         y = torch.empty(M, N, device="cuda")
         torch.cuda.synchronize()

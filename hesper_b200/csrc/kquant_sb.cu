@@ -23,9 +23,10 @@
 //     know that the one before has landed: every slot belongs to one K group (the ring's stages are
 //     a multiple of KG, the position decides the group), or the ring never wraps (sb_plan).
 //
-// What bounds it: instruction issue -- about 330 instructions per 16 rows x 256 weights at up to
-// 8 tokens, 520 at up to 15 (products, int -> float, scales) -- 2 to 3.5 us at K=2560 N=10240 --
-// next to 2.2 (Q4_K) or 4.2 us (Q8_0) of weight stream.
+// What bounds it is latency, not a rate: at K=2560 N=10240 instruction issue takes 2 to 3.5 us (about 330
+// instructions per 16 rows x 256 weights at up to 8 tokens, 520 at up to 15) and the weight stream
+// 2.3 (Q4_K) or 4.3 us (Q8_0), the call 9 to 12: the staging launch (2 to 3), a CTA's fill and, per pass,
+// the chain from a stage's arrival through two dependent products per 32 weights and token column.
 #include <optional>
 #include <type_traits>
 

@@ -27,8 +27,9 @@
 //     warps 4-19  epilogue: warp w reads lane quarter w & 3 of the accumulators (w >> 2) - 1, + 4, ...:
 //                 hi + lo, optional logits store, argmax over the tile's rows (redux + ballot); one
 //                 atomicMax of the ordered (value,row) key per token and CTA.
-// HBM-bound.  Measured, V=128256 K=2560, whole call: 32 tokens 149 -> 106 us (6.2 TB/s of table
-// bytes), 64 tokens 149 -> 117; with one box per step 124 and 131 (half a DRAM burst per row).
+// HBM-bound.  Measured, V=128256 K=2560, whole call (split, product, argmax): 32 tokens 143 to 149 ->
+// 113 to 117 us (5.6 to 5.8 TB/s of table bytes, by the box), of which the product is 106; 64 tokens
+// 149 -> 117 in the product; with one box per step 124 and 131 there (half a DRAM burst per row).
 // Every mbarrier wait is bounded; on expiry the kernel still releases its tensor memory.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

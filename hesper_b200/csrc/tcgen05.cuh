@@ -37,16 +37,6 @@ __device__ __forceinline__ bool tc_elect() {
   return p != 0;
 }
 
-// kind::f16 with the A operand in tensor memory (lane = row, two 16-bit K elements per
-// 32-bit column) and B through a shared-memory descriptor.
-__device__ __forceinline__ void tc_mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
-                                              uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                    smem_u32(bar))
@@ -59,7 +49,9 @@ __device__ __forceinline__ void tc_before_sync() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
 
-// The same two for a converged warp: every lane calls, one issues.  The MMA warp shares its
+// kind::f16 with the A operand in tensor memory (lane = row, two 16-bit K elements per 32-bit
+// column) and B through a shared-memory descriptor, and the commit, for a converged warp: every lane
+// calls, one issues.  The MMA warp shares its
 // scheduler with compute warps, so what an MMA costs is its instruction count: the descriptor's
 // high word (no swizzle, LBO, SBO) and the instruction descriptor are immediates, and the low
 // word -- smem address / 16 with LBO above it, tc_desc_lo -- is one addition per MMA.
