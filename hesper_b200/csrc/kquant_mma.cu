@@ -8,9 +8,10 @@
 // Hesper/Layers/Linear.lean:1152-1760,5973-6177).  Weights AND activations are rounded to f16
 // (2^-11 each): measured error ~4e-4 of max|y|, bar 1e-3.
 //
-// What bounds it: at 64 tokens the dequantiser (about 2 instructions per weight) and HBM, at
-// 256 tokens the tensor pipe (M=128, N=256, K=16 in 138 cycles).  Either way only when every SM
-// works, so the work is dealt in units of (row tile of 128, super-block of 256 weights):
+// What bounds it: at 64 tokens instruction issue of the SMs at work (81 % of the slots; 4.9 instructions
+// per weight, two of them the dequantiser's arithmetic, the rest loads, scales, tensor-memory stores,
+// barriers and polling), at 256 tokens the tensor pipe (M=128, N=256, K=16 in 138 cycles).  Either
+// way only when every SM works, so the work is dealt in units of (row tile of 128, super-block of 256 weights):
 //   * whole waves of row tiles go one tile to a CTA (W per CTA, results stored directly);
 //   * the R row tiles left over are cut along K into runs of `upc` consecutive units, one run
 //     per CTA.  A run that does not cover its tile leaves an f32 partial in the context's
