@@ -886,11 +886,12 @@ static int attn_run(hb200_ctx* ctx, const void* d_q, int q_is_f16, const void* d
     // the lines below stay as they were.  D = 64: 16 pairs x 8000 11.8, 14.8, 37 x 2000 9.0, 10.8, 37 x 4000
     // 13.7, 11.0, 49 x 14000 44.7, 29.8; D = 128: 27 x 8000 23.3, 26.2, 37 x 4000 17.2, 19.8, 37 x 8000
     // 29.1, 25.7; D = 256: 49 x 8000 62, 64, 49 x 14000 102, 97, 64 x 14000 (more SMs at work) 101, 125.
-    // D = 64 also has several CTAs of a short cluster on an SM: 27 x 1000 in 7 splits 6.1, 5 6.4.
+    // D = 64 also has several CTAs of a cluster on an SM, up to 1.55 per SM in all: 27 x 1000 in 7 splits
+    // 6.1, 5 6.4, 14 x 6816 in 16 9.7, 10 10.2, but 16 x 2000 in 15 9.7, 9 6.9.
     const int one = attn_one_wave_splits(ctx, D, ctx->attn_mode == HB200_ATTN_PRECISE, pairs, most);
     const long busy = pairs * one, each = one > 1 ? eff_len / one : 0;
     const long longest = D == 64 ? 950 : (D == 128 ? 2100 : (busy * 10 >= 8L * ctx->sm_count ? LONG_MAX : 4000));
-    const bool fits = D == 64 && small && (most <= 4 || pairs * most * 2 <= 3L * ctx->sm_count);
+    const bool fits = D == 64 && small && (most <= 4 || pairs * most * 16 <= 25L * ctx->sm_count);
     const bool wave = one > 1 && !fits && each <= longest && (small || busy * 10 >= 6L * ctx->sm_count);
     if (wave || small) {
       fewer = wave && one < (small ? most : p.nsplit);
